@@ -34,8 +34,29 @@ template <typename T> using cplx_t = typename cplx<T>::type;
 template <typename C> __host__ __device__ __forceinline__ C cmake(double re, double im) {
     C r; r.x = (decltype(r.x))re; r.y = (decltype(r.y))im; return r;
 }
-__device__ __forceinline__ float2 operator+(float2 a, float2 b) { return make_float2(a.x + b.x, a.y + b.y); }
-__device__ __forceinline__ float2 operator-(float2 a, float2 b) { return make_float2(a.x - b.x, a.y - b.y); }
+// FP32 complex sums, differences and real scalings as one packed instruction
+// (two IEEE round-to-nearest operations; the same values as two scalar ones):
+// the transforms are bound by instruction issue, not by the FP32 lanes
+__device__ __forceinline__ uint64_t f2_bits(float2 a) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a.x), "f"(a.y));
+    return r;
+}
+__device__ __forceinline__ float2 bits_f2(uint64_t v) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+__device__ __forceinline__ float2 operator+(float2 a, float2 b) {
+    uint64_t r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(f2_bits(a)), "l"(f2_bits(b)));
+    return bits_f2(r);
+}
+__device__ __forceinline__ float2 operator-(float2 a, float2 b) {
+    uint64_t r;
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(f2_bits(a)), "l"(f2_bits(b)));
+    return bits_f2(r);
+}
 __device__ __forceinline__ double2 operator+(double2 a, double2 b) { return make_double2(a.x + b.x, a.y + b.y); }
 __device__ __forceinline__ double2 operator-(double2 a, double2 b) { return make_double2(a.x - b.x, a.y - b.y); }
 
@@ -59,6 +80,18 @@ template <int SIGN, typename C> __device__ __forceinline__ C mul_isign(C a) {
 }
 template <typename C, typename S> __device__ __forceinline__ C cscale(C a, S s) {
     C r; r.x = a.x * s; r.y = a.y * s; return r;
+}
+// acc + a s for a real s
+template <typename C, typename S> __device__ __forceinline__ C cmadd(C acc, C a, S s) {
+    if constexpr (sizeof(C) == sizeof(float2)) {
+        uint64_t r;
+        asm("fma.rn.f32x2 %0, %1, %2, %3;"
+            : "=l"(r)
+            : "l"(f2_bits(a)), "l"(f2_bits(make_float2((float)s, (float)s))), "l"(f2_bits(acc)));
+        return bits_f2(r);
+    } else {
+        C r; r.x = acc.x + a.x * s; r.y = acc.y + a.y * s; return r;
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -122,7 +155,7 @@ template <int SIGN, int OFF, int STRIDE> struct Dft<3, SIGN, OFF, STRIDE> {
         constexpr double s = 0.86602540378443864676372317075293618;  // sin(2 pi / 3)
         C x0 = v[OFF], x1 = v[OFF + STRIDE], x2 = v[OFF + 2 * STRIDE];
         C t = x1 + x2, u = x1 - x2;
-        C m = x0 + cscale(t, (T)c);
+        C m = cmadd(x0, t, (T)c);
         C is = mul_isign<SIGN>(cscale(u, (T)s));
         v[OFF] = x0 + t;
         v[OFF + STRIDE] = m + is;
@@ -196,8 +229,8 @@ template <int R, int SIGN, int OFF, int STRIDE> struct DftPrime {
         C re = x0, im;
         im.x = 0;
         im.y = 0;
-        ((re = re + cscale(sp[Ns + 1], (T)TwC<((Ns + 1) * K) % R, R>::c)), ...);
-        ((im = im + cscale(sm[Ns + 1], (T)TwC<((Ns + 1) * K) % R, R>::s)), ...);
+        ((re = cmadd(re, sp[Ns + 1], (T)TwC<((Ns + 1) * K) % R, R>::c)), ...);
+        ((im = cmadd(im, sm[Ns + 1], (T)TwC<((Ns + 1) * K) % R, R>::s)), ...);
         const C ji = mul_isign<SIGN>(im);
         out[K] = re + ji;
         out[R - K] = re - ji;
