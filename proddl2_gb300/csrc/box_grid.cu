@@ -69,9 +69,8 @@ template <typename T2, int SIGN> __device__ __forceinline__ T2 tw_at(const T2* t
 // and writes its R-point DFT to dst[(j / Ns) Ns R + j mod Ns + k Ns].  The
 // twiddle index (j mod Ns) r n/(Ns R) stays below n; the R-th roots of unity
 // are held in registers for the whole stage, radices 2 and 4 need none, 6
-// is two 3-point DFTs joined by W6 twiddles.  LS lanes share one line
-// (butterflies j = lane, lane + LS, ..).
-template <typename T2, int SIGN, int R, int LS = 32>
+// is two 3-point DFTs joined by W6 twiddles.
+template <typename T2, int SIGN, int R>
 __device__ __forceinline__ void stockham_stage(const T2* src, T2* dst, const T2* tw, int n, int ns, int lane) {
     using S = decltype(T2::x);
     const int nb = n / R;
@@ -84,7 +83,7 @@ __device__ __forceinline__ void stockham_stage(const T2* src, T2* dst, const T2*
     root[0].y = 0;
 #pragma unroll
     for (int m = 1; m < R; ++m) root[m] = tw_at<T2, SIGN>(tw, m * nb);
-    for (int j = lane; j < nb; j += LS) {
+    for (int j = lane; j < nb; j += 32) {
         T2 v[R];
 #pragma unroll
         for (int r = 0; r < R; ++r) v[r] = src[j + r * nb];
@@ -180,11 +179,8 @@ __device__ __forceinline__ void stockham_stage(const T2* src, T2* dst, const T2*
 
 // Unnormalised DFT of the warp's line in a (n points), b a second buffer of
 // n points; returns the buffer that holds the result.  SIGN -1: forward
-// e^{-2 pi i jk/n}; +1: inverse.  Ends with __syncwarp.  MAXR < 11: the plan
-// has no factor 11 or 13 (those stages are not compiled: fewer registers).
-// LS = 16: two lines per warp, lane = the thread's index within its half
-// (each half passes its own line's buffers).
-template <typename T2, int SIGN, int MAXR = 13, int LS = 32>
+// e^{-2 pi i jk/n}; +1: inverse.  Ends with __syncwarp..
+template <typename T2, int SIGN>
 __device__ T2* warp_fft(T2* a, T2* b, const T2* tw, const BoxPlan& pl, int lane) {
     T2* src = a;
     T2* dst = b;
@@ -193,19 +189,15 @@ __device__ T2* warp_fft(T2* a, T2* b, const T2* tw, const BoxPlan& pl, int lane)
     for (int s = 0; s < pl.nf; ++s) {
         const int R = pl.f[s];
         switch (R) {
-            case 4: stockham_stage<T2, SIGN, 4, LS>(src, dst, tw, pl.n, ns, lane); break;
-            case 6: stockham_stage<T2, SIGN, 6, LS>(src, dst, tw, pl.n, ns, lane); break;
-            case 2: stockham_stage<T2, SIGN, 2, LS>(src, dst, tw, pl.n, ns, lane); break;
-            case 3: stockham_stage<T2, SIGN, 3, LS>(src, dst, tw, pl.n, ns, lane); break;
-            case 5: stockham_stage<T2, SIGN, 5, LS>(src, dst, tw, pl.n, ns, lane); break;
-            case 7: stockham_stage<T2, SIGN, 7, LS>(src, dst, tw, pl.n, ns, lane); break;
-            case 9: stockham_stage<T2, SIGN, 9, LS>(src, dst, tw, pl.n, ns, lane); break;
-            default:
-                if constexpr (MAXR >= 11) {
-                    if (R == 11) stockham_stage<T2, SIGN, 11, LS>(src, dst, tw, pl.n, ns, lane);
-                    else stockham_stage<T2, SIGN, 13, LS>(src, dst, tw, pl.n, ns, lane);
-                }
-                break;
+            case 4: stockham_stage<T2, SIGN, 4>(src, dst, tw, pl.n, ns, lane); break;
+            case 6: stockham_stage<T2, SIGN, 6>(src, dst, tw, pl.n, ns, lane); break;
+            case 2: stockham_stage<T2, SIGN, 2>(src, dst, tw, pl.n, ns, lane); break;
+            case 3: stockham_stage<T2, SIGN, 3>(src, dst, tw, pl.n, ns, lane); break;
+            case 5: stockham_stage<T2, SIGN, 5>(src, dst, tw, pl.n, ns, lane); break;
+            case 7: stockham_stage<T2, SIGN, 7>(src, dst, tw, pl.n, ns, lane); break;
+            case 9: stockham_stage<T2, SIGN, 9>(src, dst, tw, pl.n, ns, lane); break;
+            case 11: stockham_stage<T2, SIGN, 11>(src, dst, tw, pl.n, ns, lane); break;
+            default: stockham_stage<T2, SIGN, 13>(src, dst, tw, pl.n, ns, lane); break;
         }
         __syncwarp();
         T2* t = src;
@@ -495,169 +487,6 @@ __global__ void __launch_bounds__(32 * kBoxWarps, 2) box_pencil_kernel(
 }
 
 // ---------------------------------------------------------------------------
-// plane stage: CTA = one (rotation, x) plane.  Inverse y transform of every
-// kz column, then each row's real inverse z transform (the half spectrum
-// extended by Hermitian symmetry, a complex inverse transform, the real
-// part); every warp keeps the KC smallest (value, offset) of its rows, and
-// warp 0 merges them into the plane's pool.
-// ---------------------------------------------------------------------------
-// QUAD: input = the tensor pencil stage's x-quads [B][nxp / 4][nh][4]
-// plh (plh.n = nz / 2 for even nz, else 0): each row's real inverse
-// transform as one nz/2-point complex transform of the Hermitian-folded half
-// spectrum, Y[k] = A + i w^k B with A = X[k] + conj(X[nz/2 - k]),
-// B = X[k] - conj(X[nz/2 - k]), w = e^{2 pi i / nz}: output m holds the real
-// values of z = 2m and 2m + 1.
-// PW warps; MAXR: the largest radix of the y and z plans (9: none of 11, 13)
-template <bool DBG, bool QUAD, int PW, int MAXR>
-__global__ void __launch_bounds__(32 * PW, 2) box_plane_kernel(const float2* __restrict__ g2,
-                                                                  const float2* __restrict__ twy_g,
-                                                                  const float2* __restrict__ twz_g, BoxPlan ply,
-                                                                  BoxPlan plz, BoxPlan plh, int nx, int pp,
-                                                                  float* __restrict__ cand_v,
-                                                                  int32_t* __restrict__ cand_i,
-                                                                  float* __restrict__ dbg, int nxp) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    const int ny = ply.n, nz = plz.n, hz = nz / 2 + 1;
-    const int lmax = ny > nz ? ny : nz;
-    const int ns = plh.n;
-    // rows of an odd pitch: a half-warp reading a column hits 16 bank pairs
-    const int pitch = hz | 1;
-    float2* plane = reinterpret_cast<float2*>(smem_raw);  // [Ny][pitch]
-    float2* twy = plane + (size_t)ny * pitch;             // [ny]
-    float2* twz = twy + ny;                               // [nz]
-    float2* twh = twz + nz;                               // [nz / 2]: e^{-2 pi i m / (nz / 2)}
-    float2* wbuf = twh + nz / 2;                          // [8][2][lmax]
-    __shared__ float lv_s[PW * KC];
-    __shared__ int li_s[PW * KC];
-
-    const int x = blockIdx.x, q = blockIdx.y;
-    const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
-    for (int i = tid; i < ny; i += blockDim.x) twy[i] = twy_g[i];
-    for (int i = tid; i < nz; i += blockDim.x) twz[i] = twz_g[i];
-    for (int i = tid; i < ns; i += blockDim.x) twh[i] = twz_g[2 * i];
-    {
-        // the plane's values, 8 loads in flight per thread before their stores
-        const size_t nh = (size_t)ny * hz;
-        const float2* src = QUAD ? g2 + (size_t)q * nxp * nh + (size_t)(x >> 2) * nh * 4 + (x & 3)
-                                 : g2 + ((size_t)q * nx + x) * pp;
-        const int step = QUAD ? 4 : 1;
-        const int tot = ny * hz;
-        // i / hz as a multiply-high by ceil(2^32 / hz): exact for i < 2^32 / hz
-        const unsigned mhz = 0xffffffffu / (unsigned)hz + 1u;
-        for (int i0 = tid; i0 < tot; i0 += 8 * blockDim.x) {
-            float2 v[8];
-#pragma unroll
-            for (int k = 0; k < 8; ++k) {
-                const int i = i0 + k * blockDim.x;
-                if (i < tot) v[k] = src[(size_t)i * step];
-            }
-#pragma unroll
-            for (int k = 0; k < 8; ++k) {
-                const int i = i0 + k * blockDim.x;
-                if (i < tot) {
-                    const int yq = (int)__umulhi((unsigned)i, mhz);
-                    plane[yq * pitch + (i - yq * hz)] = v[k];
-                }
-            }
-        }
-    }
-    __syncthreads();
-    float2* a = wbuf + (size_t)w * 2 * lmax;
-    float2* b = a + lmax;
-    // columns kz: inverse transform along ky
-    for (int kz = w; kz < hz; kz += PW) {
-        __syncwarp();
-        for (int k = lane; k < ny; k += 32) a[k] = plane[k * pitch + kz];
-        const float2* o = warp_fft<float2, +1, MAXR>(a, b, twy, ply, lane);
-        for (int y = lane; y < ny; y += 32) plane[y * pitch + kz] = o[y];
-    }
-    __syncthreads();
-    // rows y: real inverse transform along kz, and the warp's top KC.  Even
-    // nz: two rows per warp, 16 lanes each (the short nz/2-point transforms
-    // leave most of a warp idle in their larger-radix stages); each half's
-    // line sits at offset line * ns of the warp's two buffers.
-    WarpTopK tk;
-    tk.init();
-    const size_t row0 = (size_t)x * ny;
-    const int line = lane >> 4, li = lane & 15;
-    for (int y0 = 2 * w; y0 < ny && ns > 0; y0 += 2 * PW) {
-        __syncwarp();
-        const int y = y0 + line < ny ? y0 + line : y0;  // an odd last row: both halves take it
-        const float2* row = plane + (size_t)y * pitch;
-        float2* al = a + line * ns;
-        for (int k = li; k < ns; k += 16) {
-            const float2 X = row[k], Xm = row[ns - k];
-            const float2 A = make_float2(X.x + Xm.x, X.y - Xm.y);
-            const float2 B = make_float2(X.x - Xm.x, X.y + Xm.y);
-            const float2 wk = twz[k];  // conj(w^k)
-            const float2 cb = make_float2(B.x * wk.x + B.y * wk.y, B.y * wk.x - B.x * wk.y);  // B w^k
-            al[k] = make_float2(A.x - cb.y, A.y + cb.x);
-        }
-        const float2* o = warp_fft<float2, +1, MAXR, 16>(al, b + line * ns, twh, plh, li);
-        // the same plan in both halves: both results in a, or both in b
-        const float2* res = (o == al ? a : b);
-#pragma unroll 1
-        for (int hl = 0; hl < 2 && y0 + hl < ny; ++hl) {
-            const float2* ol = res + hl * ns;
-            const int yy = y0 + hl;
-            for (int z0 = 0; z0 < nz; z0 += 32) {
-                const int z = z0 + lane;
-                const bool ok = z < nz;
-                const float2 c = ol[ok ? z >> 1 : 0];
-                const float v = ok ? ((z & 1) ? c.y : c.x) : INFINITY;
-                const int idx = ok ? (int)((row0 + yy) * nz + z) : 0x7fffffff;
-                if (DBG && ok) dbg[(size_t)q * nx * ny * nz + (size_t)idx] = v;
-                tk.offer(v, idx, lane);
-            }
-        }
-    }
-    for (int y = w; y < ny && ns == 0; y += PW) {
-        __syncwarp();
-        const float2* row = plane + (size_t)y * pitch;
-        for (int k = lane; k < nz; k += 32) {
-            if (k < hz) {
-                a[k] = row[k];
-            } else {
-                const float2 c = row[nz - k];
-                a[k] = make_float2(c.x, -c.y);
-            }
-        }
-        const float2* o = warp_fft<float2, +1, MAXR>(a, b, twz, plz, lane);
-        for (int z0 = 0; z0 < nz; z0 += 32) {
-            const int z = z0 + lane;
-            const bool ok = z < nz;
-            const float v = ok ? o[z].x : INFINITY;
-            const int idx = ok ? (int)((row0 + y) * nz + z) : 0x7fffffff;
-            if (DBG && ok) dbg[(size_t)q * nx * ny * nz + (size_t)idx] = v;
-            tk.offer(v, idx, lane);
-        }
-    }
-    if (lane < KC) {
-        lv_s[w * KC + lane] = tk.lv;
-        li_s[w * KC + lane] = tk.li;
-    }
-    // the warps' sorted lists merged pairwise over log2(PW) levels into
-    // list 0 (warp w merges list w + step into list w)
-    for (int step = 1; step < PW; step <<= 1) {
-        __syncthreads();
-        if ((w & (2 * step - 1)) == 0 && w + step < PW) {
-            float sv = lane < KC ? lv_s[w * KC + lane] : lv_s[(w + step) * KC + 31 - lane];
-            int si = lane < KC ? li_s[w * KC + lane] : li_s[(w + step) * KC + 31 - lane];
-            warp_merge32(sv, si, lane);
-            if (lane < KC) {
-                lv_s[w * KC + lane] = sv;
-                li_s[w * KC + lane] = si;
-            }
-        }
-    }
-    __syncthreads();
-    if (w == 0 && lane < KC) {
-        cand_v[((size_t)q * nx + x) * KC + lane] = lv_s[lane];
-        cand_i[((size_t)q * nx + x) * KC + lane] = li_s[lane];
-    }
-}
-
-// ---------------------------------------------------------------------------
 // finalize: merge the Nx x KC pools, FP64 direct-space rescoring of the KC
 // best cells (mod each axis' size), sort by (energy, offset), maxValCorr,
 // translation = h unwrap(cell) per axis.  One CTA per rotation.
@@ -771,9 +600,10 @@ size_t pencil_smem_bytes(int nx, int ny, int nz, int K, int n_ent, bool weighted
            (size_t)kBoxWarps * nx * sizeof(float2) + (size_t)n_ent * sizeof(uint32_t) * (weighted ? 2 : 1) +
            ((size_t)K + 1) * sizeof(int32_t);
 }
-size_t plane_smem_bytes(int ny, int nz) {
+// the plane's share of the size limit a ligand is accepted under (plane,
+// twiddles and 16 line buffers; plane_lines_kernel needs less)
+size_t plane_limit_bytes(int ny, int nz) {
     const int hz = nz / 2 + 1, lmax = std::max(ny, nz);
-    // up to 16 warps (plans without factors 11 and 13)
     return ((size_t)ny * (hz | 1) + ny + nz + nz / 2 + (size_t)16 * 2 * lmax) * sizeof(float2);
 }
 size_t prep_smem_bytes(int nx, int K, int n_ent) {
@@ -797,42 +627,12 @@ cudaError_t box_prep(const BatchArgs& a, cudaStream_t s) {
     return cudaGetLastError();
 }
 
-bool big_radix(const BoxPlan& pl) {
-    for (int i = 0; i < pl.nf; ++i)
-        if (pl.f[i] > 9) return true;
-    return false;
-}
-
-template <bool DBG, bool QUAD, int PW, int MAXR>
-cudaError_t box_plane_launch(dim3 grid, size_t sm, const float2* src, const float2* twy, const float2* twz,
-                             const BoxPlan& py, const BoxPlan& pz, const BoxPlan& ph, int nx, const BatchArgs& a,
-                             float* dbg, int nxp, cudaStream_t s) {
-    cudaError_t e = set_smem((const void*)box_plane_kernel<DBG, QUAD, PW, MAXR>, sm);
-    if (e != cudaSuccess) return e;
-    box_plane_kernel<DBG, QUAD, PW, MAXR><<<grid, 32 * PW, sm, s>>>(src, twy, twz, py, pz, ph, nx, a.PP, a.cand_v,
-                                                                    a.cand_i, dbg, nxp);
-    return cudaGetLastError();
-}
-
-// plans without factors 11 and 13 run 16 warps per CTA (the smaller
-// stages fit 64 registers), others 8
-template <bool DBG, bool QUAD>
-cudaError_t box_plane(dim3 grid, size_t sm, const float2* src, const float2* twy, const float2* twz, const BoxPlan& py,
-                      const BoxPlan& pz, int nx, const BatchArgs& a, float* dbg, int nxp, cudaStream_t s) {
-    // even nz: rows through the half-length transform
-    BoxPlan ph{};
-    if (pz.n % 2 == 0 && !factor_plan(pz.n / 2, ph)) ph = BoxPlan{};
-    if (big_radix(py) || big_radix(pz))
-        return box_plane_launch<DBG, QUAD, 8, 13>(grid, sm, src, twy, twz, py, pz, ph, nx, a, dbg, nxp, s);
-    return box_plane_launch<DBG, QUAD, 16, 9>(grid, sm, src, twy, twz, py, pz, ph, nx, a, dbg, nxp, s);
-}
-
 cudaError_t box_middle(const BatchArgs& a, cudaStream_t s) {
     const int nb = a.n_rot;
     if (nb <= 0) return cudaSuccess;
     const int nx = a.box.n[0], ny = a.box.n[1], nz = a.box.n[2];
-    BoxPlan px, py, pz;
-    if (!factor_plan(nx, px) || !factor_plan(ny, py) || !factor_plan(nz, pz)) return cudaErrorInvalidValue;
+    BoxPlan px;
+    if (!factor_plan(nx, px)) return cudaErrorInvalidValue;
     const float2* twx = a.box_tw32;
     const float2* twy = twx + nx;
     const float2* twz = twy + ny;
@@ -841,8 +641,6 @@ cudaError_t box_middle(const BatchArgs& a, cudaStream_t s) {
     const bool weighted = a.lig_w32 != nullptr;
     const size_t sm2 = pencil_smem_bytes(nx, ny, nz, a.K, a.n_ent, weighted);
     const int np = ny * (nz / 2 + 1);
-    const size_t sm3 = plane_smem_bytes(ny, nz);
-    dim3 grid3(nx, nb);
     if (a.use_tc) {
         // tensor form: the x stage as split-FP16 tcgen05 GEMMs over 128
         // rotations per CTA, then the plane stage from its x-quads
@@ -864,8 +662,7 @@ cudaError_t box_middle(const BatchArgs& a, cudaStream_t s) {
         }
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
         if (a.ev && (e = cudaEventRecord(a.ev[1], s)) != cudaSuccess) return e;
-        e = a.dbg_corr ? box_plane<true, true>(grid3, sm3, a.g2t, twy, twz, py, pz, nx, a, a.dbg_corr, nxp, s)
-                       : box_plane<false, true>(grid3, sm3, a.g2t, twy, twz, py, pz, nx, a, nullptr, nxp, s);
+        e = box_plane(a, twy, twz, true, s);
         if (e != cudaSuccess) return e;
         if (a.ev && (e = cudaEventRecord(a.ev[2], s)) != cudaSuccess) return e;
         return cudaSuccess;
@@ -884,8 +681,7 @@ cudaError_t box_middle(const BatchArgs& a, cudaStream_t s) {
     }
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     if (a.ev && (e = cudaEventRecord(a.ev[1], s)) != cudaSuccess) return e;
-    e = a.dbg_corr ? box_plane<true, false>(grid3, sm3, a.g2, twy, twz, py, pz, nx, a, a.dbg_corr, nx, s)
-                   : box_plane<false, false>(grid3, sm3, a.g2, twy, twz, py, pz, nx, a, nullptr, nx, s);
+    e = box_plane(a, twy, twz, false, s);
     if (e != cudaSuccess) return e;
     if (a.ev && (e = cudaEventRecord(a.ev[2], s)) != cudaSuccess) return e;
     return cudaSuccess;
@@ -916,7 +712,7 @@ cudaError_t box_load_kernels(int) {
     cudaFuncAttributes fa;
     cudaError_t e = cudaFuncGetAttributes(&fa, (const void*)box_prep_kernel);
     if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, (const void*)box_pencil_kernel<false>);
-    if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, (const void*)box_plane_kernel<false, false, 16, 9>);
+    if (e == cudaSuccess) e = box_plane_load();
     if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, (const void*)box_finalize_kernel);
     return e;
 }
@@ -927,7 +723,7 @@ bool box_plan(int n, BoxPlan* pl) { return factor_plan(n, *pl); }
 
 size_t box_pencil_smem(int nx, int ny, int nz, int K, int n_ent, bool weighted) {
     return std::max(pencil_smem_bytes(nx, ny, nz, K, n_ent, weighted),
-                    std::max(plane_smem_bytes(ny, nz), prep_smem_bytes(nx, K, n_ent)));
+                    std::max(plane_limit_bytes(ny, nz), prep_smem_bytes(nx, K, n_ent)));
 }
 
 // Forward transform of one real FP64 term grid [Nx][Ny][Nz] into spec_t

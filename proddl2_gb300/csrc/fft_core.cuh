@@ -259,6 +259,8 @@ template <int R, int SIGN, int OFF, int STRIDE> struct DftPrime {
 };
 template <int SIGN, int OFF, int STRIDE> struct Dft<5, SIGN, OFF, STRIDE> : DftPrime<5, SIGN, OFF, STRIDE> {};
 template <int SIGN, int OFF, int STRIDE> struct Dft<7, SIGN, OFF, STRIDE> : DftPrime<7, SIGN, OFF, STRIDE> {};
+template <int SIGN, int OFF, int STRIDE> struct Dft<11, SIGN, OFF, STRIDE> : DftPrime<11, SIGN, OFF, STRIDE> {};
+template <int SIGN, int OFF, int STRIDE> struct Dft<13, SIGN, OFF, STRIDE> : DftPrime<13, SIGN, OFF, STRIDE> {};
 
 // composite radix: R = A * B, decimation in time.
 //   sub-DFTs of length B over v[OFF + STRIDE*(A*n2 + n1)] for each n1 < A,
@@ -267,7 +269,7 @@ template <int SIGN, int OFF, int STRIDE> struct Dft<7, SIGN, OFF, STRIDE> : DftP
 template <int R, int SIGN, int OFF, int STRIDE> struct DftComposite {
     static constexpr int A = smallest_factor(R);
     static constexpr int B = R / A;
-    static_assert(A < R, "radix must factor over 2, 3, 4, 5, 7");
+    static_assert(A < R, "radix must factor over 2, 3, 4, 5, 7, 11, 13");
     template <int N1> struct Sub {
         template <typename C> __device__ __forceinline__ static void run(C* v) {
             Dft<B, SIGN, OFF + STRIDE * N1, STRIDE * A>::run(v);

@@ -291,6 +291,10 @@ cudaError_t box_circ_scales(const float2* circ, int K, int nh, int nx, int8_t* c
 size_t box_tc_smem(const int dims[3], int n_chunks, int n_terms);
 size_t cubic_tc_smem(int n, int n_chunks, int n_terms);
 
+// plane stage of a batch on a box grid (quad: from the tensor stage's x-quads)
+cudaError_t box_plane(const BatchArgs& a, const float2* twy, const float2* twz, bool quad, cudaStream_t s);
+cudaError_t box_plane_load();
+
 // Read-only view of a ready context's scan inputs (receptor spectra and
 // grids, ligand, geometry); the work pointers of `args` are the context's own.
 struct ScanInputs {
