@@ -5,8 +5,15 @@
 #include "internal.h"
 #include "scan_kernels.cuh"
 #include "pencil_tc.cuh"
+#include "plane_lines.cuh"
 
 namespace fftdock {
+
+// threads of a cubic edge's plane CTA: about one first-pass butterfly each at
+// the small edges.  Measured against 256 threads, ms per 1000 rotations:
+// 24^3 0.21 -> 0.14, 32^3 0.26 -> 0.16, 48^3 0.40 -> 0.31, 64^3 planes 0.61 -> 0.51
+// (its x-quads: 0.56 -> 0.69, so 256 there).
+constexpr int plane_threads(int n, bool quad) { return n <= 16 ? 32 : n <= 32 ? 64 : n <= (quad ? 48 : 64) ? 128 : 256; }
 
 template <int N> struct SizeOpsImpl {
     static constexpr int G = SizeTraits<N>::G;
@@ -20,7 +27,6 @@ template <int N> struct SizeOpsImpl {
                ((size_t)K * N + 1) * sizeof(int32_t) +
                (size_t)n_ent * sizeof(uint32_t);
     }
-    static size_t plane_smem() { return (size_t)N * H * sizeof(float2) + N * sizeof(float2) + (size_t)G * KC * 8; }
     template <typename T> static size_t line_smem() { return (size_t)(N * 32 + N) * sizeof(cplx_t<T>); }
 
     static cudaError_t set_smem(const void* fn, size_t bytes) {
@@ -99,37 +105,12 @@ template <int N> struct SizeOpsImpl {
         return cudaGetLastError();
     }
 
-    template <bool DBG, bool QUAD>
-    static cudaError_t launch_plane(dim3 grid, size_t sm, const float2* src, const BatchArgs& a, float* corr,
-                                    cudaStream_t s) {
-        cudaError_t e = set_smem((const void*)plane_kernel<N, DBG, QUAD>, sm);
-        if (e != cudaSuccess) return e;
-        if constexpr (QUAD) {
-            // clusters of 4 CTAs along x (the planes of one x-quad)
-            cudaLaunchConfig_t cfg = {};
-            cfg.gridDim = grid;
-            cfg.blockDim = dim3(32 * G);
-            cfg.dynamicSmemBytes = sm;
-            cfg.stream = s;
-            cudaLaunchAttribute at[1];
-            at[0].id = cudaLaunchAttributeClusterDimension;
-            at[0].val.clusterDim.x = 4;
-            at[0].val.clusterDim.y = 1;
-            at[0].val.clusterDim.z = 1;
-            cfg.attrs = at;
-            cfg.numAttrs = 1;
-            return cudaLaunchKernelEx(&cfg, plane_kernel<N, DBG, QUAD>, src, (const float2*)a.tw32, a.cand_v,
-                                      a.cand_i, corr);
-        } else {
-            plane_kernel<N, DBG, QUAD><<<grid, 32 * G, sm, s>>>(src, a.tw32, a.cand_v, a.cand_i, corr);
-            return cudaGetLastError();
-        }
-    }
     template <bool QUAD>
-    static cudaError_t plane(dim3 grid, size_t sm, const float2* src, const BatchArgs& a, float* corr,
-                             cudaStream_t s) {
-        return corr ? launch_plane<true, QUAD>(grid, sm, src, a, corr, s)
-                    : launch_plane<false, QUAD>(grid, sm, src, a, nullptr, s);
+    static cudaError_t plane(int nb, const float2* src, const BatchArgs& a, float* corr, cudaStream_t s) {
+        constexpr int MODE = QUAD ? plane_quad_mode(N, N) : kPlanePlanes;
+        constexpr int NT = plane_threads(N, QUAD);
+        return launch_planes<MODE>(&plane_lines_kernel<N, MODE, NT>, dim3(N, nb), NT, plane_lines_smem(N, N), s, src,
+                                   a.tw32, a.tw32, PlanePlan{}, N, N, a.PP, a.cand_v, a.cand_i, corr);
     }
 
     // K1 over a.n_rot rotations
@@ -182,13 +163,11 @@ template <int N> struct SizeOpsImpl {
         }
         if (a.ev && (e = cudaEventRecord(a.ev[1], s)) != cudaSuccess) return e;
         // K3 (the queue + clustering path also writes every correlation grid)
-        const size_t sm3 = plane_smem();
-        dim3 grid3(N, nb);
         float* corr = a.dbg_corr ? a.dbg_corr : a.wide.corr;
         if constexpr (kHasTc) {
-            if (tc) e = plane<true>(grid3, sm3, a.g2t, a, corr, s);  // the tensor stage's x-quads
+            if (tc) e = plane<true>(nb, a.g2t, a, corr, s);  // the tensor stage's x-quads
         }
-        if (!tc) e = plane<false>(grid3, sm3, a.g2, a, corr, s);
+        if (!tc) e = plane<false>(nb, a.g2, a, corr, s);
         if (e != cudaSuccess) return e;
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
         if (a.ev && (e = cudaEventRecord(a.ev[2], s)) != cudaSuccess) return e;
@@ -228,7 +207,7 @@ template <int N> struct SizeOpsImpl {
         if (e == cudaSuccess)
             e = spec_bf16 ? cudaFuncGetAttributes(&fa, (const void*)pencil_kernel<N, __nv_bfloat162, false>)
                           : cudaFuncGetAttributes(&fa, (const void*)pencil_kernel<N, float2, false>);
-        if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, (const void*)plane_kernel<N, false, false>);
+        if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, (const void*)plane_lines_kernel<N, kPlanePlanes, plane_threads(N, false)>);
         if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, (const void*)finalize_kernel<N>);
         return e;
     }

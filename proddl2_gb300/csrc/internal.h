@@ -198,7 +198,7 @@ struct BatchArgs {
     cudaEvent_t* ev;            // optional: events recorded by the middle stage (see SizeOps::middle)
     // tensor-core pencil stage (use_tc): it writes g2t as x-quads
     // [B][N/4][N*H][4] (four consecutive x per pencil), which the plane stage
-    // reads in clusters of 4 CTAs
+    // reads (plane_lines.cuh)
     float2* g2t;
     int use_tc;
     const float2* circ;         // [K][N*H][N] receptor circulant samples

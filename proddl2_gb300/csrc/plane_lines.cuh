@@ -21,21 +21,29 @@
 // Folded passes (even nz, ns = nz / 2):
 // * the real columns kz = 0 and ns travel as one complex column
 //   X0 + i Xns through the y passes (ns columns instead of ns + 1);
-// * the last y pass takes the columns kz and ns - kz together and writes the
-//   Hermitian-folded half spectrum Y[kz] = A + i w^kz B, A = X[kz] +
-//   conj(X[ns - kz]), B = X[kz] - conj(X[ns - kz]), w = e^{2 pi i / nz}: each
-//   row is then one ns-point complex transform whose output m holds the real
-//   values of z = 2 m and 2 m + 1;
-// * the first y pass reads the plane straight from global memory when it is
-//   stored plane by plane.
+// * the first z pass takes the butterflies j and m - j of a row together:
+//   their inputs hold every k with its mirror ns - k, so they are first folded
+//   to Y[k] = A + i w^k B, A = X[k] + conj(X[ns - k]), B = X[k] -
+//   conj(X[ns - k]), w = e^{2 pi i / nz}; the row is then one ns-point complex
+//   transform whose output m holds the real values of z = 2 m and 2 m + 1;
+// * the first y pass reads global memory.  From the tensor pencil stage's
+//   x-quads (four planes interleaved) every CTA reads its 8 of each 32 bytes,
+//   or, on larger planes, a cluster of 4 CTAs shares the pass: each CTA does a
+//   quarter of the butterflies for all four planes, two planes per thread from
+//   one 16-byte load, and stores the results into the planes' CTAs through
+//   distributed shared memory (kPlaneQuad, kPlaneQuadCluster).
 // Odd nz: two rows a, b travel as one complex line a + i b of nz points.
 //
-// Bound: the shared-memory passes (seven reads and writes of the plane) and
-// their barriers.  Measured on box grids against one warp per line through
-// two shared buffers (runtime Stockham stages, lanes idle in short rows,
-// per-lane twiddles, an insertion list per warp), per 1024 rotations: 112 x
-// 120 x 126 x-quads 20.5 -> 6.0 ms; per 1000 rotations: 90 x 96 x 100 planes
-// 14.9 -> 3.1 ms (1.1 TB/s of plane bytes).
+// Bound: instruction issue and the six shared-memory passes (the plane's
+// bytes move at 2.5 TB/s at 128^3).  Against the kernels it replaced -- on
+// cubic edges a two-pass transform with its lines spread over warps (exchange
+// barriers in every pass, (value, offset) minima, one re-read of all cells),
+// on box grids one warp per line through two buffers -- in ms per 1000
+// rotations, planes | x-quads (shape + 18 terms): 48^3 0.46 -> 0.31 | 0.82 ->
+// 0.31, 64^3 0.76 -> 0.51 | 0.99 -> 0.56, 80^3 3.21 -> 1.12 | 3.65 -> 1.01, 96^3
+// 3.47 -> 1.60 | 4.11 -> 1.58, 112^3 7.91 -> 2.35 | 8.57 -> 2.69, 128^3 4.80 ->
+// 3.42 | 5.73 -> 3.87, 144^3 11.6 -> 5.8 | 15.4 -> 6.4; 90 x 96 x 100 14.9 -> 2.9 |,
+// 112 x 120 x 126 | 20.0 -> 4.5.
 #pragma once
 
 #include <type_traits>
@@ -46,22 +54,23 @@
 
 namespace fftdock {
 
-// Radices of one axis, first pass first.  Two passes cover every size that is
-// a product of a radix up to 16 and one up to 13; the rest take three or
-// four (the last radix stays small: its pass holds two columns).
+// Radices of one axis, first pass first.  Two passes cover most sizes; the
+// rest take three or four.
 struct LineRadices {
     int n;
     int np;      // passes (>= 2; a radix of 1 pads a prime length)
     int r[4];
 };
 
-constexpr bool line_radices(int n, LineRadices& out) {
+// two passes: first radix up to amax, last up to 16, least wa a + wb b (the
+// first pass holds two planes or two butterflies per thread, so it weighs more)
+constexpr bool line_radices(int n, int amin, int amax, LineRadices& out) {
     out.n = n;
     out.np = 0;
     int best = 1 << 30;
-    for (int a = 2; a <= 16; ++a) {
-        if (n % a != 0 || n / a > 13) continue;
-        const int b = n / a, cost = 10 * a + 14 * b;
+    for (int a = amin; a <= amax; ++a) {
+        if (n % a != 0 || n / a > 16) continue;
+        const int b = n / a, cost = 13 * a + 10 * b;
         if (cost < best) {
             best = cost;
             out.np = 2;
@@ -70,7 +79,7 @@ constexpr bool line_radices(int n, LineRadices& out) {
         }
     }
     if (out.np) return true;
-    // three passes, then four: the least sum of radices
+    // three passes, then four: the least sum of radices, largest last
     for (int np = 3; np <= 4; ++np) {
         best = 1 << 30;
         for (int a = 2; a <= 13; ++a) {
@@ -83,9 +92,9 @@ constexpr bool line_radices(int n, LineRadices& out) {
                     if (a + b + c < best) {
                         best = a + b + c;
                         out.np = 3;
-                        out.r[0] = a;
+                        out.r[0] = c;
                         out.r[1] = b;
-                        out.r[2] = c;
+                        out.r[2] = a;
                     }
                 } else {
                     for (int d = 2; d <= b; ++d) {
@@ -93,10 +102,10 @@ constexpr bool line_radices(int n, LineRadices& out) {
                         if (a + b + d + c / d < best) {
                             best = a + b + d + c / d;
                             out.np = 4;
-                            out.r[0] = a;
-                            out.r[1] = b;
-                            out.r[2] = d;
-                            out.r[3] = c / d;
+                            out.r[0] = c / d;
+                            out.r[1] = d;
+                            out.r[2] = b;
+                            out.r[3] = a;
                         }
                     }
                 }
@@ -114,8 +123,7 @@ struct PlanePlan {
     int ncol;         // columns of the y passes: ns (even nz) or hz
     int pitch;        // row pitch in complex values, odd
     // ceil(2^32 / d) for the index divisions: exact while index * d < 2^32
-    unsigned m_hz, m_col, m_pair, m_row;
-    int npair;        // column pairs of the folded last y pass (even nz)
+    unsigned m_col, m_row;
     int nrow;         // lines of the z passes: ny (even nz) or ceil(ny / 2)
 };
 
@@ -128,13 +136,10 @@ constexpr bool plane_plan(int ny, int nz, PlanePlan& p) {
     p.pitch = p.hz | 1;
     const bool even = nz % 2 == 0;
     p.ncol = even ? nz / 2 : p.hz;
-    p.npair = even ? (nz / 2 + 1) / 2 : 0;
     p.nrow = even ? ny : (ny + 1) / 2;
-    p.m_hz = div_magic(p.hz);
     p.m_col = div_magic(p.ncol);
-    p.m_pair = div_magic(p.npair);
     p.m_row = div_magic(p.nrow);
-    return line_radices(ny, p.y) && line_radices(even ? nz / 2 : nz, p.z);
+    return line_radices(ny, 2, 13, p.y) && (even ? line_radices(nz / 2, 1, 11, p.z) : line_radices(nz, 2, 13, p.z));
 }
 template <int N> constexpr PlanePlan fixed_plane_plan() {
     PlanePlan p{};
@@ -142,15 +147,22 @@ template <int N> constexpr PlanePlan fixed_plane_plan() {
     return p;
 }
 
-constexpr int kPlaneThreads = 256;
 constexpr int kPlaneCand = 256;  // candidate list of the selection
+// input of plane_lines_kernel: [B][nx][pp] planes, or the tensor pencil
+// stage's x-quads [B][nxp / 4][ny hz][4], read by each CTA alone (8 of every
+// 32 bytes) or shared by clusters of 4 CTAs.  Measured per 1000 rotations
+// (shape + 18 terms), alone | cluster: 48^3 0.37 | 0.66 ms, 64^3 0.56 | 0.93,
+// 80^3 1.01 | 1.39, 96^3 1.58 | 1.95, 112^3 3.00 | 2.68, 128^3 4.50 | 3.86, 112 x
+// 120 x 126 4.71 | 4.48: alone while the four-fold reads stay cheap beside
+// the cluster's barriers, the line between the 96 and 112 edges.
+constexpr int kPlanePlanes = 0, kPlaneQuad = 1, kPlaneQuadCluster = 2;
+constexpr int plane_quad_mode(int ny, int nz) { return ny * (nz / 2 + 1) <= 5400 ? kPlaneQuad : kPlaneQuadCluster; }
 
 // dynamic shared memory: plane, twiddles of both axes, y of a row position,
 // the warps' top-KC lists
 constexpr size_t plane_lines_smem(int ny, int nz) {
     const size_t hz = nz / 2 + 1, rows = (size_t)ny + (ny & 1);  // a lone last row's line (odd nz) spans two
-    return (rows * (hz | 1) + ny + nz) * sizeof(float2) + ((size_t)ny + 2) * sizeof(int) +
-           (size_t)(kPlaneThreads / 32) * KC * 8;
+    return (rows * (hz | 1) + ny + nz) * sizeof(float2) + ((size_t)ny + 2) * sizeof(int) + (size_t)8 * KC * 8;
 }
 
 __device__ __forceinline__ int div_by(int i, int d, unsigned magic) {
@@ -198,15 +210,14 @@ __device__ __forceinline__ int line_digits(const LineRadices& l, int b) {
     return f;
 }
 
-// FIXED: N > 0 = the cubic edge N at compile time, 0 = the plan in `rp`.
-// QUAD: input = the tensor pencil stage's x-quads [B][nxp / 4][ny hz][4],
-// staged by clusters of 4 CTAs (see plane_kernel); else [B][nx][pp].
+// N > 0: the cubic edge N at compile time; 0: the plan in `rp`.  NT threads.
 // dbg (optional, [B][nx][ny][nz]): also write the plane's values.
-template <int N, bool QUAD>
-__global__ void __launch_bounds__(kPlaneThreads, 3) plane_lines_kernel(
+template <int N, int MODE, int NT>
+__global__ void __launch_bounds__(NT, 768 / NT) plane_lines_kernel(
     const float2* __restrict__ g2, const float2* __restrict__ twy_g, const float2* __restrict__ twz_g,
     const __grid_constant__ PlanePlan rp,
     int nx_rt, int nxp_rt, int pp, float* __restrict__ cand_v, int32_t* __restrict__ cand_i, float* __restrict__ dbg) {
+    constexpr bool QUAD = MODE != kPlanePlanes, CLUSTER = MODE == kPlaneQuadCluster;
     constexpr PlanePlan FP = fixed_plane_plan<(N > 0 ? N : 16)>();
     PlanePlan P;  // compile-time plans: every field is a constant
     if constexpr (N > 0) P = FP;
@@ -227,66 +238,40 @@ __global__ void __launch_bounds__(kPlaneThreads, 3) plane_lines_kernel(
     float2* twz = twy + ny;                               // [nz]
     int* ytab = reinterpret_cast<int*>(twz + nz);         // [ny] y of row position p
     float* lv_s = reinterpret_cast<float*>(ytab + ((ny + 1) & ~1));  // [8][KC]
-    int* li_s = reinterpret_cast<int*>(lv_s + (kPlaneThreads / 32) * KC);
+    int* li_s = reinterpret_cast<int*>(lv_s + 8 * KC);
     __shared__ float cand_sv[kPlaneCand];
     __shared__ int cand_si[kPlaneCand];
     __shared__ int n_cand;
+    __shared__ int nonzero;  // some input value of this plane is not zero
 
     const int x = blockIdx.x, q = blockIdx.y;
     const int tid = threadIdx.x, w = tid >> 5, l = tid & 31;
-    if constexpr (QUAD) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
-    for (int i = tid; i < ny; i += kPlaneThreads) twy[i] = twy_g[i];
-    for (int i = tid; i < nz; i += kPlaneThreads) twz[i] = twz_g[i];
+    if (tid == 0) nonzero = 0;
+    if constexpr (CLUSTER) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    for (int i = tid; i < ny; i += NT) twy[i] = twy_g[i];
+    for (int i = tid; i < nz; i += NT) twz[i] = twz_g[i];
     {
         const int rl = N > 0 ? RYL : rp.y.r[rp.y.np - 1];
-        for (int p = tid; p < ny; p += kPlaneThreads) {
+        for (int p = tid; p < ny; p += NT) {
             const int b = p / rl;
             ytab[p] = ydigits(b) + (p - b * rl) * (ny / rl);
         }
     }
-    const int nh = ny * hz;
-    if constexpr (QUAD) {
-        uint32_t rank;
-        asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
-        const int xb = x - (int)rank;  // the cluster's first plane
-        // this CTA's quarter of the pencils as 16-byte halves of their quads
-        // (planes xb, xb + 1 | xb + 2, xb + 3), coalesced, loads in batches
-        // ahead of their stores
-        const int q4 = (nh + 3) / 4, p0 = (int)rank * q4, n2 = 2 * max(0, min(q4, nh - p0));
-        const float4* gs = reinterpret_cast<const float4*>(g2 + (size_t)q * nh * nxp + (size_t)(xb >> 2) * nh * 4) +
-                           (size_t)2 * p0;
-        const uint32_t loc = static_cast<uint32_t>(__cvta_generic_to_shared(plane));
-        uint32_t rb[4];
-#pragma unroll
-        for (int j = 0; j < 4; ++j)
-            asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(rb[j]) : "r"(loc), "r"(j));
-        const uint32_t d0 = (tid & 1) ? rb[2] : rb[0], d1 = (tid & 1) ? rb[3] : rb[1];
-        asm volatile("barrier.cluster.wait.aligned;" ::: "memory");  // every CTA of the cluster runs
-        constexpr int BATCH = 8;
-        for (int e0 = tid; e0 < n2; e0 += BATCH * kPlaneThreads) {
-            float4 a[BATCH];
-#pragma unroll
-            for (int k = 0; k < BATCH; ++k) {
-                const int e = e0 + k * kPlaneThreads;
-                if (e < n2) a[k] = __ldg(gs + e);
-            }
-#pragma unroll
-            for (int k = 0; k < BATCH; ++k) {
-                const int e = e0 + k * kPlaneThreads;
-                if (e < n2) {
-                    const int p = p0 + (e >> 1);
-                    const int ky = div_by(p, hz, P.m_hz);
-                    const uint32_t off = (uint32_t)(p + ky * (pitch - hz)) * 8u;
-                    asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(d0 + off), "f"(a[k].x), "f"(a[k].y)
-                                 : "memory");
-                    asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(d1 + off), "f"(a[k].z), "f"(a[k].w)
-                                 : "memory");
-                }
-            }
+    const size_t nh = (size_t)ny * hz;
+    // A plane whose input is all zeros (the ligand reaches no receptor cell at
+    // this x: exact zeros from the tensor stage) transforms to all zeros; its
+    // KC best cells are its first KC.  A third of the planes at 128^3 with
+    // 4000 / 1500 atoms.
+    auto zero_plane = [&]() {
+        const int cells = ny * nz;
+        if (tid < KC) {
+            const size_t o = ((size_t)q * nx + x) * KC + tid;
+            cand_v[o] = tid < cells ? 0.f : INFINITY;
+            cand_i[o] = tid < cells ? x * cells + tid : 0x7fffffff;
         }
-        asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-        if (x >= nx) return;  // a padding plane of the last quad
-    }
+        if (dbg)
+            for (int i = tid; i < cells; i += NT) dbg[((size_t)q * nx + x) * cells + i] = 0.f;
+    };
     __syncthreads();
 
     // element (line, pos) of an in-place pass over sub-blocks of length len
@@ -294,7 +279,7 @@ __global__ void __launch_bounds__(kPlaneThreads, 3) plane_lines_kernel(
         with_radix<0, 13>(R_, [&](auto radix) {
             constexpr int R = decltype(radix)::value;
             const int m = len / R, items = n_lines * (n / R), tstep = tws * (n / len);
-            for (int it = tid; it < items; it += kPlaneThreads) {
+            for (int it = tid; it < items; it += NT) {
                 const int qb = div_by(it, n_lines, magic);
                 float2* p = plane + (it - qb * n_lines) * ls;
                 const int b = qb / m, j = qb - b * m;
@@ -312,25 +297,108 @@ __global__ void __launch_bounds__(kPlaneThreads, 3) plane_lines_kernel(
     };
 
     // ---- y, first pass: butterfly j of column kz reads ky = j + r ny / R ----
-    {
-        const float2* src = g2 + ((size_t)q * nx + x) * pp;
-        with_radix<RY0, 16>(P.y.r[0], [&](auto radix) {
+    if constexpr (CLUSTER) {
+        uint32_t rank;
+        asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+        const float4* src = reinterpret_cast<const float4*>(g2 + (size_t)q * nh * nxp + (size_t)((x - (int)rank) >> 2) * nh * 4);
+        // this thread's planes: 2 h and 2 h + 1 of the quad
+        const int h = tid & 1;
+        uint32_t d0, d1;
+        const uint32_t loc = static_cast<uint32_t>(__cvta_generic_to_shared(plane));
+        const uint32_t flag = static_cast<uint32_t>(__cvta_generic_to_shared(&nonzero));
+        {
+            asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(d0) : "r"(loc), "r"(2 * h));
+            asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(d1) : "r"(loc), "r"(2 * h + 1));
+        }
+        with_radix<RY0, 13>(N > 0 ? RY0 : rp.y.r[0], [&](auto radix) {
             constexpr int R = decltype(radix)::value;
-            const int m = ny / R, items = P.ncol * m;
+            const int m = ny / R, total = P.ncol * m, share = (total + 3) / 4;
+            const int i0 = (int)rank * share, i1 = min(i0 + share, total);
+            bool arrived = false;
+            unsigned any_a = 0, any_b = 0;
 #pragma unroll 1
-            for (int it = tid; it < items; it += kPlaneThreads) {
+            for (int it = i0 + (tid >> 1); it < i1; it += NT / 2) {
                 const int j = div_by(it, P.ncol, P.m_col);
                 const int kz = it - j * P.ncol;
-                float2 v[R];
+                float2 va[R], vb[R];
 #pragma unroll
-                for (int r = 0; r < R; ++r)
-                    v[r] = QUAD ? plane[(j + r * m) * pitch + kz] : __ldg(src + (j + r * m) * hz + kz);
+                for (int r = 0; r < R; ++r) {
+                    const float4 t = __ldg(src + (size_t)((j + r * m) * hz + kz) * 2 + h);
+                    va[r] = make_float2(t.x, t.y);
+                    vb[r] = make_float2(t.z, t.w);
+                    any_a |= __float_as_uint(t.x) | __float_as_uint(t.y);
+                    any_b |= __float_as_uint(t.z) | __float_as_uint(t.w);
+                }
                 if (even && kz == 0) {
                     // the real columns 0 and ns as one complex column
 #pragma unroll
                     for (int r = 0; r < R; ++r) {
-                        const float2 o = QUAD ? plane[(j + r * m) * pitch + ns] : __ldg(src + (j + r * m) * hz + ns);
+                        const float4 t = __ldg(src + (size_t)((j + r * m) * hz + ns) * 2 + h);
+                        va[r] = make_float2(va[r].x - t.y, va[r].y + t.x);
+                        vb[r] = make_float2(vb[r].x - t.w, vb[r].y + t.z);
+                        any_a |= __float_as_uint(t.x) | __float_as_uint(t.y);
+                        any_b |= __float_as_uint(t.z) | __float_as_uint(t.w);
+                    }
+                }
+                dft<R, +1>(va);
+                dft<R, +1>(vb);
+#pragma unroll
+                for (int r = 1; r < R; ++r) {
+                    const float2 t = twy[j * r];
+                    va[r] = ctwiddle<+1>(va[r], t);
+                    vb[r] = ctwiddle<+1>(vb[r], t);
+                }
+                if (!arrived) {
+                    asm volatile("barrier.cluster.wait;" ::: "memory");  // every CTA of the cluster runs
+                    arrived = true;
+                }
+                const uint32_t off = (uint32_t)(j * pitch + kz) * 8u, st = (uint32_t)(m * pitch) * 8u;
+#pragma unroll
+                for (int r = 0; r < R; ++r) {
+                    asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(d0 + off + r * st), "f"(va[r].x),
+                                 "f"(va[r].y)
+                                 : "memory");
+                    asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(d1 + off + r * st), "f"(vb[r].x),
+                                 "f"(vb[r].y)
+                                 : "memory");
+                }
+            }
+            if (!arrived) asm volatile("barrier.cluster.wait;" ::: "memory");
+            // (x & 0x7fffffff: -0 counts as zero)
+            if (any_a & 0x7fffffffu) asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(d0 - loc + flag), "r"(1) : "memory");
+            if (any_b & 0x7fffffffu) asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(d1 - loc + flag), "r"(1) : "memory");
+        });
+        asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+        if (x >= nx) return;  // a padding plane of the last quad
+        if (nonzero == 0) {
+            zero_plane();
+            return;
+        }
+    } else {
+        const float2* src = QUAD ? g2 + (size_t)q * nh * nxp + (size_t)(x >> 2) * nh * 4 + (x & 3)
+                                 : g2 + ((size_t)q * nx + x) * pp;
+        constexpr int SS = QUAD ? 4 : 1;
+        unsigned any = 0;
+        with_radix<RY0, 13>(N > 0 ? RY0 : rp.y.r[0], [&](auto radix) {
+            constexpr int R = decltype(radix)::value;
+            const int m = ny / R, items = P.ncol * m;
+#pragma unroll 1
+            for (int it = tid; it < items; it += NT) {
+                const int j = div_by(it, P.ncol, P.m_col);
+                const int kz = it - j * P.ncol;
+                float2 v[R];
+#pragma unroll
+                for (int r = 0; r < R; ++r) {
+                    v[r] = __ldg(src + SS * ((j + r * m) * hz + kz));
+                    if (QUAD) any |= __float_as_uint(v[r].x) | __float_as_uint(v[r].y);
+                }
+                if (even && kz == 0) {
+                    // the real columns 0 and ns as one complex column
+#pragma unroll
+                    for (int r = 0; r < R; ++r) {
+                        const float2 o = __ldg(src + SS * ((j + r * m) * hz + ns));
                         v[r] = make_float2(v[r].x - o.y, v[r].y + o.x);
+                        if (QUAD) any |= __float_as_uint(o.x) | __float_as_uint(o.y);
                     }
                 }
                 dft<R, +1>(v);
@@ -340,8 +408,16 @@ __global__ void __launch_bounds__(kPlaneThreads, 3) plane_lines_kernel(
                 for (int r = 0; r < R; ++r) plane[(j + r * m) * pitch + kz] = v[r];
             }
         });
+        if (QUAD) {
+            // (-0 counts as zero)
+            if (!__syncthreads_or((any & 0x7fffffffu) != 0u)) {
+                zero_plane();
+                return;
+            }
+        } else {
+            __syncthreads();
+        }
     }
-    __syncthreads();
     if constexpr (N == 0) {
         int len = ny / P.y.r[0];
         for (int s = 1; s + 1 < P.y.np; ++s) {
@@ -351,67 +427,25 @@ __global__ void __launch_bounds__(kPlaneThreads, 3) plane_lines_kernel(
         }
     }
     // ---- y, last pass ----
-    if (even) {
-        with_radix<RYL, 13>(N > 0 ? RYL : rp.y.r[rp.y.np - 1], [&](auto radix) {
-            constexpr int R = decltype(radix)::value;
-            const int items = P.npair * (ny / R);
+    with_radix<RYL, 16>(N > 0 ? RYL : rp.y.r[rp.y.np - 1], [&](auto radix) {
+        constexpr int R = decltype(radix)::value;
+        const int items = P.ncol * (ny / R);
 #pragma unroll 1
-            for (int it = tid; it < items; it += kPlaneThreads) {
-                const int b = div_by(it, P.npair, P.m_pair);
-                const int i = it - b * P.npair;
-                // column pair (i, ns - i); pair 0 = the packed columns 0 | ns
-                // and the self-paired column ns / 2 (even ns)
-                const bool two = i > 0 || (ns & 1) == 0;
-                const int c2 = i > 0 ? ns - i : (two ? ns >> 1 : 0);
-                float2* pa = plane + b * R * pitch + i;
-                float2* pc = plane + b * R * pitch + c2;
-                float2 va[R], vc[R];
+        for (int it = tid; it < items; it += NT) {
+            const int b = div_by(it, P.ncol, P.m_col);
+            float2* p = plane + b * R * pitch + (it - b * P.ncol);
+            float2 v[R];
 #pragma unroll
-                for (int r = 0; r < R; ++r) va[r] = pa[r * pitch];
+            for (int r = 0; r < R; ++r) v[r] = p[r * pitch];
+            dft<R, +1>(v);
 #pragma unroll
-                for (int r = 0; r < R; ++r) vc[r] = pc[r * pitch];
-                dft<R, +1>(va);
-                dft<R, +1>(vc);
-                if (i > 0) {
-                    const float2 wk = twz[i];  // conj(w^i)
-#pragma unroll
-                    for (int r = 0; r < R; ++r) {
-                        const float2 X = va[r], Xm = vc[r];
-                        const float2 A = make_float2(X.x + Xm.x, X.y - Xm.y);
-                        const float2 B = make_float2(X.x - Xm.x, X.y + Xm.y);
-                        const float2 C = cmul_conj(B, wk);
-                        pa[r * pitch] = make_float2(A.x - C.y, A.y + C.x);
-                        pc[r * pitch] = make_float2(A.x + C.y, C.x - A.y);
-                    }
-                } else {
-#pragma unroll
-                    for (int r = 0; r < R; ++r) {
-                        pa[r * pitch] = make_float2(va[r].x + va[r].y, va[r].x - va[r].y);
-                        if (two) pc[r * pitch] = make_float2(2.f * vc[r].x, -2.f * vc[r].y);
-                    }
-                }
-            }
-        });
-        __syncthreads();
-    } else {
-        with_radix<RYL, 13>(N > 0 ? RYL : rp.y.r[rp.y.np - 1], [&](auto radix) {
-            constexpr int R = decltype(radix)::value;
-            const int items = P.ncol * (ny / R);
-#pragma unroll 1
-            for (int it = tid; it < items; it += kPlaneThreads) {
-                const int b = div_by(it, P.ncol, P.m_col);
-                float2* p = plane + b * R * pitch + (it - b * P.ncol);
-                float2 v[R];
-#pragma unroll
-                for (int r = 0; r < R; ++r) v[r] = p[r * pitch];
-                dft<R, +1>(v);
-#pragma unroll
-                for (int r = 0; r < R; ++r) p[r * pitch] = v[r];
-            }
-        });
-        __syncthreads();
+            for (int r = 0; r < R; ++r) p[r * pitch] = v[r];
+        }
+    });
+    __syncthreads();
+    if (!even) {
         // rows at positions 2 t, 2 t + 1 -> one complex line a + i b of nz points
-        for (int t = w; t < P.nrow; t += kPlaneThreads / 32) {
+        for (int t = w; t < P.nrow; t += NT / 32) {
             float2* la = plane + 2 * t * pitch;
             const bool has_b = 2 * t + 1 < ny;
             float2 a[4], b[4];  // hz <= 128
@@ -438,23 +472,77 @@ __global__ void __launch_bounds__(kPlaneThreads, 3) plane_lines_kernel(
     const int nl = even ? ns : nz;                    // points per line
     const int lstride = even ? pitch : 2 * pitch;     // line stride
     const int nrow = P.nrow, tws = even ? 2 : 1;      // w_nl = w_nz^tws
-    with_radix<RZ0, 16>(P.z.r[0], [&](auto radix) {
+    if (even) {
+        with_radix<RZ0, 11>(N > 0 ? RZ0 : rp.z.r[0], [&](auto radix) {
             constexpr int R = decltype(radix)::value;
-        const int m = nl / R, items = nrow * m;
+            const int m = nl / R, items = nrow * ((m + 1) >> 1);
 #pragma unroll 1
-        for (int it = tid; it < items; it += kPlaneThreads) {
-            const int j = div_by(it, nrow, P.m_row);
-            float2* p = plane + (it - j * nrow) * lstride + j;
-            float2 v[R];
+            for (int it = tid; it < items; it += NT) {
+                // butterflies i and m - i of a row; i = 0: butterfly 0 and,
+                // for even m, m / 2 (each its own mirror)
+                const int i = div_by(it, nrow, P.m_row);
+                const bool two = i > 0 || (m & 1) == 0;
+                const int i2 = i > 0 ? m - i : (two ? m >> 1 : 0);
+                float2* row = plane + (it - i * nrow) * lstride;
+                float2 va[R], vb[R];
 #pragma unroll
-            for (int r = 0; r < R; ++r) v[r] = p[r * m];
-            dft<R, +1>(v);
+                for (int r = 0; r < R; ++r) va[r] = row[i + r * m];
 #pragma unroll
-            for (int r = 1; r < R; ++r) v[r] = ctwiddle<+1>(v[r], twz[tws * j * r]);
+                for (int r = 0; r < R; ++r) vb[r] = row[i2 + r * m];
+                // X = X[k], Xm = X[ns - k] -> Y[k], Y[ns - k]
+                auto fold = [&](float2& X, float2& Xm, int k) {
+                    const float2 A = make_float2(X.x + Xm.x, X.y - Xm.y);
+                    const float2 B = make_float2(X.x - Xm.x, X.y + Xm.y);
+                    const float2 C = cmul_conj(B, twz[k]);
+                    X = make_float2(A.x - C.y, A.y + C.x);
+                    Xm = make_float2(A.x + C.y, C.x - A.y);
+                };
+                auto fold_self = [&](float2& X) { X = make_float2(2.f * X.x, -2.f * X.y); };  // k = ns / 2
+                if (i > 0) {
 #pragma unroll
-            for (int r = 0; r < R; ++r) p[r * m] = v[r];
-        }
-    });
+                    for (int r = 0; r < R; ++r) fold(va[r], vb[R - 1 - r], i + r * m);
+                } else {
+                    va[0] = make_float2(va[0].x + va[0].y, va[0].x - va[0].y);  // the packed X0 + i Xns
+#pragma unroll
+                    for (int r = 1; 2 * r < R; ++r) fold(va[r], va[R - r], r * m);
+                    if (R % 2 == 0) fold_self(va[R / 2]);
+#pragma unroll
+                    for (int r = 0; 2 * r + 1 < R; ++r) fold(vb[r], vb[R - 1 - r], i2 + r * m);
+                    if (R % 2 == 1) fold_self(vb[R / 2]);
+                }
+                dft<R, +1>(va);
+                dft<R, +1>(vb);
+#pragma unroll
+                for (int r = 1; r < R; ++r) va[r] = ctwiddle<+1>(va[r], twz[2 * i * r]);
+#pragma unroll
+                for (int r = 0; r < R; ++r) row[i + r * m] = va[r];
+                if (two) {
+#pragma unroll
+                    for (int r = 1; r < R; ++r) vb[r] = ctwiddle<+1>(vb[r], twz[2 * i2 * r]);
+#pragma unroll
+                    for (int r = 0; r < R; ++r) row[i2 + r * m] = vb[r];
+                }
+            }
+        });
+    } else {
+        with_radix<RZ0, 13>(N > 0 ? RZ0 : rp.z.r[0], [&](auto radix) {
+            constexpr int R = decltype(radix)::value;
+            const int m = nl / R, items = nrow * m;
+#pragma unroll 1
+            for (int it = tid; it < items; it += NT) {
+                const int j = div_by(it, nrow, P.m_row);
+                float2* p = plane + (it - j * nrow) * lstride + j;
+                float2 v[R];
+#pragma unroll
+                for (int r = 0; r < R; ++r) v[r] = p[r * m];
+                dft<R, +1>(v);
+#pragma unroll
+                for (int r = 1; r < R; ++r) v[r] = ctwiddle<+1>(v[r], twz[j * r]);
+#pragma unroll
+                for (int r = 0; r < R; ++r) p[r * m] = v[r];
+            }
+        });
+    }
     __syncthreads();
     if constexpr (N == 0) {
         int len = nl / P.z.r[0];
@@ -464,16 +552,69 @@ __global__ void __launch_bounds__(kPlaneThreads, 3) plane_lines_kernel(
             __syncthreads();
         }
     }
-    // last pass: real values back into the rows, every thread keeps the
-    // smallest (value, offset) it produced.  each_own(f) calls
-    // f(value, offset) for this thread's values again.
+    // last pass: real values back into the rows; every thread keeps the
+    // smallest value it produced
     const int zl = N > 0 ? RZL : rp.z.r[rp.z.np - 1];
     const int zstep = nl / zl, zitems = nrow * zstep;
-    float bmin_v = INFINITY;
-    int bmin_i = 0x7fffffff;
-    const int xrow = x * ny;
-    // offsets of the two reals of line position (line, block frequency f):
-    // even nz: z = 2 f, 2 f + 1 of row `line`; odd: z = f of rows 2 line, 2 line + 1
+    float bmin = INFINITY;
+    with_radix<RZL, 16>(zl, [&](auto radix) {
+        constexpr int R = decltype(radix)::value;
+#pragma unroll 1
+        for (int it = tid; it < zitems; it += NT) {
+            const int b = div_by(it, nrow, P.m_row);
+            const int line = it - b * nrow;
+            float2* p = plane + line * lstride + b * R;
+            float2 v[R];
+#pragma unroll
+            for (int r = 0; r < R; ++r) v[r] = p[r];
+            dft<R, +1>(v);
+            // odd nz and ny: the lone last line carries no second row
+            const bool both = even || 2 * line + 1 < ny;
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+                p[r] = v[r];
+                bmin = fminf(bmin, v[r].x);
+                if (both) bmin = fminf(bmin, v[r].y);
+            }
+        }
+    });
+
+    // ---- selection: the KC-th smallest of the threads' minima bounds the
+    // plane's KC-th value from above (at least KC cells lie at or below it),
+    // so the plane's KC best by (value, offset) are among the cells at or
+    // below it (usually 16 to 30).  Bitonic warp sorts, lists merged as a
+    // tree over the warps. ----
+    static_assert(KC == 16, "the bitonic selection keeps 16 of 32 lanes");
+    constexpr int NW = NT / 32;
+    {
+        float v = bmin;
+#pragma unroll
+        for (int k = 2; k <= 32; k <<= 1)
+#pragma unroll
+            for (int j = k >> 1; j > 0; j >>= 1) {
+                const float o = __shfl_xor_sync(0xffffffffu, v, j);
+                v = ((l & k) == 0) == ((l & j) == 0) ? fminf(v, o) : fmaxf(v, o);
+            }
+        if (l < KC) lv_s[w * KC + l] = v;
+    }
+    if (tid == 0) n_cand = 0;
+    for (int step = 1; step < NW; step <<= 1) {
+        __syncthreads();
+        if ((w & (2 * step - 1)) == 0 && w + step < NW) {
+            float v = l < KC ? lv_s[w * KC + l] : lv_s[(w + step) * KC + 31 - l];
+#pragma unroll
+            for (int j = 16; j > 0; j >>= 1) {
+                const float o = __shfl_xor_sync(0xffffffffu, v, j);
+                v = (l & j) == 0 ? fminf(v, o) : fmaxf(v, o);
+            }
+            if (l < KC) lv_s[w * KC + l] = v;
+        }
+    }
+    __syncthreads();
+    const float bound = lv_s[KC - 1];
+    // offset of (line, frequency f): even nz: z = 2 f (+ 1: the imaginary
+    // part) of row `line`; odd nz: z = f of rows 2 line and 2 line + 1
+    const int xrow = x * ny, fmul = even ? 2 : 1;
     auto offs = [&](int line, int& o0, int& o1) {
         if (even) {
             o0 = (xrow + ytab[line]) * nz;
@@ -483,63 +624,6 @@ __global__ void __launch_bounds__(kPlaneThreads, 3) plane_lines_kernel(
             o1 = 2 * line + 1 < ny ? (xrow + ytab[2 * line + 1]) * nz : -1;
         }
     };
-    const int fmul = even ? 2 : 1;
-    with_radix<RZL, 13>(zl, [&](auto radix) {
-            constexpr int R = decltype(radix)::value;
-#pragma unroll 1
-        for (int it = tid; it < zitems; it += kPlaneThreads) {
-            const int b = div_by(it, nrow, P.m_row);
-            const int line = it - b * nrow;
-            float2* p = plane + line * lstride + b * R;
-            float2 v[R];
-#pragma unroll
-            for (int r = 0; r < R; ++r) v[r] = p[r];
-            dft<R, +1>(v);
-            int o0, o1;
-            offs(line, o0, o1);
-            const int f0 = zdigits(b) * fmul, fs = zstep * fmul;
-#pragma unroll
-            for (int r = 0; r < R; ++r) {
-                p[r] = v[r];
-                const int f = f0 + r * fs;
-                if (better(v[r].x, o0 + f, bmin_v, bmin_i)) { bmin_v = v[r].x; bmin_i = o0 + f; }
-                if ((even || o1 >= 0) && better(v[r].y, o1 + f, bmin_v, bmin_i)) { bmin_v = v[r].y; bmin_i = o1 + f; }
-            }
-        }
-    });
-
-    // ---- selection (as in plane_kernel): the KC-th best of the threads'
-    // minima bounds the plane's KC-th best from above ----
-    static_assert(KC == 16, "the bitonic selection keeps 16 of 32 lanes");
-    constexpr int NW = kPlaneThreads / 32;
-    auto tree_merge = [&](int n_lists) {
-        for (int step = 1; step < n_lists; step <<= 1) {
-            __syncthreads();
-            if ((w & (2 * step - 1)) == 0 && w + step < n_lists) {
-                float sv = l < KC ? lv_s[w * KC + l] : lv_s[(w + step) * KC + 31 - l];
-                int si = l < KC ? li_s[w * KC + l] : li_s[(w + step) * KC + 31 - l];
-                warp_merge32(sv, si, l);
-                if (l < KC) {
-                    lv_s[w * KC + l] = sv;
-                    li_s[w * KC + l] = si;
-                }
-            }
-        }
-        __syncthreads();
-    };
-    {
-        float sv = bmin_v;
-        int si = bmin_i;
-        warp_sort32(sv, si, l);
-        if (l < KC) {
-            lv_s[w * KC + l] = sv;
-            li_s[w * KC + l] = si;
-        }
-    }
-    if (tid == 0) n_cand = 0;
-    tree_merge(NW);
-    const float tv = lv_s[KC - 1];
-    const int ti = li_s[KC - 1];
     if (dbg) {
         // the plane's values, whole rows (the pass barriers above cover the writes)
         float* out = dbg + ((size_t)q * nx + x) * (size_t)ny * nz;
@@ -559,31 +643,50 @@ __global__ void __launch_bounds__(kPlaneThreads, 3) plane_lines_kernel(
         }
     }
     // only a thread whose own minimum is at or below the bound holds cells at
-    // or below it (a few per plane): it re-reads its own values
-    if (!better(tv, ti, bmin_v, bmin_i)) {
-        for (int it = tid; it < zitems; it += kPlaneThreads) {
+    // or below it (a few per plane): its warp re-reads that thread's values
+    // together, one per lane
+    auto offer = [&](float v, int off) {
+        if (v <= bound) {
+            const int at = atomicAdd(&n_cand, 1);
+            if (at < kPlaneCand) { cand_sv[at] = v; cand_si[at] = off; }
+        }
+    };
+    unsigned qual = __ballot_sync(0xffffffffu, bmin <= bound);
+    while (qual) {
+        const int it0 = w * 32 + __ffs(qual) - 1;
+        qual &= qual - 1u;
+        const int cells = it0 < zitems ? ((zitems - 1 - it0) / NT + 1) * zl : 0;
+        for (int c = l; c < cells; c += 32) {
+            const int k = c / zl, r = c - k * zl;
+            const int it = it0 + k * NT;
             const int b = div_by(it, nrow, P.m_row);
             const int line = it - b * nrow;
-            const float2* p = plane + line * lstride + b * zl;
+            const float2 o = plane[line * lstride + b * zl + r];
             int o0, o1;
             offs(line, o0, o1);
-            const int f0 = zdigits(b) * fmul, fs = zstep * fmul;
-            for (int r = 0; r < zl; ++r) {
-                const float2 o = p[r];
-                const int f = f0 + r * fs;
-                if (!better(tv, ti, o.x, o0 + f)) {
-                    const int at = atomicAdd(&n_cand, 1);
-                    if (at < kPlaneCand) { cand_sv[at] = o.x; cand_si[at] = o0 + f; }
-                }
-                if ((even || o1 >= 0) && !better(tv, ti, o.y, o1 + f)) {
-                    const int at = atomicAdd(&n_cand, 1);
-                    if (at < kPlaneCand) { cand_sv[at] = o.y; cand_si[at] = o1 + f; }
-                }
-            }
+            const int f = (zdigits(b) + r * zstep) * fmul;
+            offer(o.x, o0 + f);
+            if (even || o1 >= 0) offer(o.y, o1 + f);
         }
     }
     __syncthreads();
     const int nc = n_cand;
+    // lists 0 .. n - 1 (lv_s, li_s, ascending) merged pairwise into list 0
+    auto tree_merge = [&](int n_lists) {
+        for (int step = 1; step < n_lists; step <<= 1) {
+            __syncthreads();
+            if ((w & (2 * step - 1)) == 0 && w + step < n_lists) {
+                float sv = l < KC ? lv_s[w * KC + l] : lv_s[(w + step) * KC + 31 - l];
+                int si = l < KC ? li_s[w * KC + l] : li_s[(w + step) * KC + 31 - l];
+                warp_merge32(sv, si, l);
+                if (l < KC) {
+                    lv_s[w * KC + l] = sv;
+                    li_s[w * KC + l] = si;
+                }
+            }
+        }
+        __syncthreads();
+    };
     float* ov = cand_v + ((size_t)q * nx + x) * KC;
     int32_t* oi = cand_i + ((size_t)q * nx + x) * KC;
     if (nc <= kPlaneCand) {
@@ -653,6 +756,30 @@ __global__ void __launch_bounds__(kPlaneThreads, 3) plane_lines_kernel(
             oi[l] = tk.li;
         }
     }
+}
+
+// launch with the cluster shape of MODE (4 CTAs along x: the planes of a quad)
+template <int MODE, class... P, class... Args>
+cudaError_t launch_planes(void (*fn)(P...), dim3 grid, int threads, size_t sm, cudaStream_t s, Args... args) {
+    if (sm > 48 * 1024) {
+        cudaError_t e = cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+        if (e != cudaSuccess) return e;
+    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = sm;
+    cfg.stream = s;
+    cudaLaunchAttribute at[1];
+    if (MODE == kPlaneQuadCluster) {
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = 4;
+        at[0].val.clusterDim.y = 1;
+        at[0].val.clusterDim.z = 1;
+        cfg.attrs = at;
+        cfg.numAttrs = 1;
+    }
+    return cudaLaunchKernelEx(&cfg, fn, static_cast<P>(args)...);
 }
 
 }  // namespace fftdock

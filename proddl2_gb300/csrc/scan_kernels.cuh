@@ -25,19 +25,18 @@ namespace fftdock {
 
 constexpr int KC = 16;  // FP32 candidates kept per plane / per rotation
 
-// Warps per line transform along x/y (G) and along the half rows (GR);
-// G*G | N and GR*GR | N/2, GR | G.
+// Warps per line transform along x (and of the receptor's transforms): G*G | N.
 template <int N> struct SizeTraits;
-template <> struct SizeTraits<16> { static constexpr int G = 4, GR = 2; };
-template <> struct SizeTraits<24> { static constexpr int G = 2, GR = 2; };
-template <> struct SizeTraits<32> { static constexpr int G = 4, GR = 4; };
-template <> struct SizeTraits<48> { static constexpr int G = 4, GR = 2; };
-template <> struct SizeTraits<64> { static constexpr int G = 8, GR = 4; };
-template <> struct SizeTraits<80> { static constexpr int G = 4, GR = 2; };
-template <> struct SizeTraits<96> { static constexpr int G = 4, GR = 4; };
-template <> struct SizeTraits<112> { static constexpr int G = 4, GR = 2; };
-template <> struct SizeTraits<128> { static constexpr int G = 8, GR = 8; };
-template <> struct SizeTraits<144> { static constexpr int G = 12, GR = 6; };
+template <> struct SizeTraits<16> { static constexpr int G = 4; };
+template <> struct SizeTraits<24> { static constexpr int G = 2; };
+template <> struct SizeTraits<32> { static constexpr int G = 4; };
+template <> struct SizeTraits<48> { static constexpr int G = 4; };
+template <> struct SizeTraits<64> { static constexpr int G = 8; };
+template <> struct SizeTraits<80> { static constexpr int G = 4; };
+template <> struct SizeTraits<96> { static constexpr int G = 4; };
+template <> struct SizeTraits<112> { static constexpr int G = 4; };
+template <> struct SizeTraits<128> { static constexpr int G = 8; };
+template <> struct SizeTraits<144> { static constexpr int G = 12; };
 
 // Pencil kernel occupancy: exchange buffers (2: one barrier per term; 1: two
 // barriers per term but N*32 complex less shared memory) and the CTAs per SM
@@ -405,429 +404,7 @@ __global__ void __launch_bounds__(32 * SizeTraits<N>::G, PencilTraits<N>::MINB) 
         }
 }
 
-// ---------------------------------------------------------------------------
-// K3: plane kernel.  CTA = one (rotation, x) plane.  Inverse transform along
-// ky (columns kz; the real DC and Nyquist columns share one complex column),
-// then the half-spectrum rows along kz are turned into N reals through one
-// N/2-point complex transform each; the plane's KC smallest (value, offset)
-// cells are then selected exactly: the threads' own minima give an upper
-// bound on the KC-th value (bitonic warp sorts and a merge) and only cells at
-// or below it are sorted and merged into the plane's top KC.
-// (FFTW c2r of FFTCorrelator::correlate + CorrelationProcessor::
-// selectIntoQueue, docking_fft.hpp:452-468.)
-// Input layouts: QUAD = false, the FFT pencil stage's [B][N][PP] (each plane
-// contiguous); QUAD = true, the tensor pencil stage's x-quads
-// [B][N/4][N*H][4] (four consecutive planes interleaved per pencil), read by
-// clusters of 4 CTAs (planes 4c..4c+3) that each load a quarter of the
-// pencils as whole 32-byte groups and store every plane's value into that
-// plane's CTA through distributed shared memory.
-// ---------------------------------------------------------------------------
-template <int N, bool DBG, bool QUAD>
-__global__ void __launch_bounds__(32 * SizeTraits<N>::G) plane_kernel(
-    const float2* __restrict__ g2, const float2* __restrict__ tw, float* __restrict__ cand_v,
-    int32_t* __restrict__ cand_i, float* __restrict__ dbg) {
-    constexpr int PP = pencil_pitch(N);
-    using PC = LinePlan<N, SizeTraits<N>::G>;
-    using PR = LinePlan<N / 2, SizeTraits<N>::GR>;
-    constexpr int G = PC::G, R1 = PC::R1;
-    constexpr int GR = PR::G, R1R = PR::R1;
-    constexpr int H = N / 2 + 1, NS = N / 2;
-    constexpr int CC = (NS + 31) / 32;
-    constexpr int NG = G / GR;
-    constexpr int ROWS = 32 * NG;
-    constexpr int ROUNDS = (N + ROWS - 1) / ROWS;
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    float2* plane = reinterpret_cast<float2*>(smem_raw);  // [N][H]
-    float2* tws = plane + N * H;                          // [N]
-    float* lv_s = reinterpret_cast<float*>(tws + N);      // [G*KC]
-    int* li_s = reinterpret_cast<int*>(lv_s + G * KC);    // [G*KC]
-    constexpr int PCAND = 256;                            // candidate list capacity
-    __shared__ float cand_sv[PCAND];
-    __shared__ int cand_si[PCAND];
-    __shared__ int n_cand;
-
-    const int x = blockIdx.x;
-    const int q = blockIdx.y;
-    const int tid = threadIdx.x;
-    const int w = tid >> 5, l = tid & 31;
-    if constexpr (QUAD) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
-    for (int i = tid; i < N; i += blockDim.x) tws[i] = tw[i];
-    // element (ky, kz) of plane x at src[ky * H + kz]: global memory (FFT
-    // form) or this CTA's staged copy (x-quads)
-    const float2* src = QUAD ? plane : g2 + ((size_t)q * N + x) * PP;
-    if constexpr (QUAD) {
-        constexpr int NH = N * H;
-        static_assert(N % 4 == 0 && NH % 4 == 0, "x-quads need N % 4 == 0");
-        uint32_t rank;
-        asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
-        const int xb = x - (int)rank;  // the cluster's first plane
-        // this CTA's quarter of the pencils: NH / 2 16-byte halves (planes
-        // xb, xb + 1 | xb + 2, xb + 3), one per thread and step, coalesced
-        const float4* gs = reinterpret_cast<const float4*>(g2 + (size_t)q * NH * N + (size_t)(xb >> 2) * NH * 4) +
-                           (size_t)rank * (NH / 2);
-        const uint32_t loc = static_cast<uint32_t>(__cvta_generic_to_shared(plane)) + rank * (NH / 4) * 8u;
-        uint32_t rb[4];
-#pragma unroll
-        for (int j = 0; j < 4; ++j)
-            asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(rb[j]) : "r"(loc), "r"(j));
-        asm volatile("barrier.cluster.wait.aligned;" ::: "memory");  // every CTA of the cluster runs
-        // loads in batches ahead of their stores (a store's memory clobber
-        // would otherwise hold each load until the previous store)
-        constexpr int PER = (NH / 2 + 32 * G - 1) / (32 * G), BATCH = 9;
-#pragma unroll
-        for (int b0 = 0; b0 < PER; b0 += BATCH) {
-            float4 a[BATCH];
-#pragma unroll
-            for (int k = 0; k < BATCH; ++k) {
-                const int e = tid + (b0 + k) * 32 * G;
-                if (b0 + k < PER && e < NH / 2) a[k] = gs[e];
-            }
-#pragma unroll
-            for (int k = 0; k < BATCH; ++k) {
-                const int e = tid + (b0 + k) * 32 * G;
-                if (b0 + k < PER && e < NH / 2) {
-                    const uint32_t off = (uint32_t)(e >> 1) * 8u;
-                    const uint32_t d0 = (e & 1) ? rb[2] : rb[0], d1 = (e & 1) ? rb[3] : rb[1];
-                    asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(d0 + off), "f"(a[k].x), "f"(a[k].y)
-                                 : "memory");
-                    asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(d1 + off), "f"(a[k].z), "f"(a[k].w)
-                                 : "memory");
-                }
-            }
-        }
-        asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-    }
-    __syncthreads();
-
-    // Warp-local passes at N = 128 (8 lanes share a column or a row, so
-    // their exchanges need __syncwarp only).  A group's pass-1 outputs are
-    // stored swizzled within the line: position 16a + b (columns) or 8a + b
-    // (rows) at slot 16a + ((a + b) & 15) or 8a + ((a + b) & 7); with the
-    // half-warp's two lines 8 apart (column kz or row y), every 8-byte access
-    // of a half-warp hits distinct bank pairs.  Columns need the plane staged
-    // in shared memory (x-quads); the FFT form's columns stay lane-per-column
-    // for coalesced global loads.
-    constexpr bool WLR = N == 128 && G == 8 && GR == 8 && R1R == 8;
-    constexpr bool WLC = WLR && QUAD && R1 == 16;
-    const int lg = l >> 3, lm = l & 7;  // group (line) within the warp, thread within the group
-
-    // columns: inverse DFT along ky
-    if constexpr (WLC) {
-#pragma unroll 1
-        for (int c = 0; c < CC; ++c) {
-            const int s = 32 * c + w + 8 * lg;  // < NS
-            float2 v[16];
-#pragma unroll
-            for (int r = 0; r < 16; ++r) {
-                const int ky = lm + 8 * r;
-                if (s == 0) {
-                    const float2 d = plane[ky * H], ny = plane[ky * H + NS];
-                    v[r] = make_float2(d.x - ny.y, d.y + ny.x);
-                } else {
-                    v[r] = plane[ky * H + s];
-                }
-            }
-            dft<16, +1>(v);
-            __syncwarp();  // the group's column is read: its slots take the outputs
-#pragma unroll
-            for (int r = 0; r < 16; ++r) plane[(16 * lm + ((r + lm) & 15)) * H + s] = v[r];
-            __syncwarp();
-            float2 out[16];
-#pragma unroll
-            for (int i = 0; i < 2; ++i) {
-                const int j = lm + 8 * i;
-                float2 u[8];
-#pragma unroll
-                for (int r = 0; r < 8; ++r) {
-                    float2 a = plane[(16 * r + ((j + r) & 15)) * H + s];  // position j + 16 r
-                    if (r != 0) a = ctwiddle<+1>(a, tws[j * r]);
-                    u[r] = a;
-                }
-                dft<8, +1>(u);
-#pragma unroll
-                for (int r = 0; r < 8; ++r) out[i * 8 + r] = u[r];
-            }
-            __syncwarp();
-#pragma unroll
-            for (int i = 0; i < 2; ++i)
-#pragma unroll
-                for (int r = 0; r < 8; ++r) {
-                    const int y = lm + 8 * i + 16 * r;
-                    const float2 o = out[i * 8 + r];
-                    if (s == 0) {
-                        plane[y * H] = make_float2(o.x, 0.f);
-                        plane[y * H + NS] = make_float2(o.y, 0.f);
-                    } else {
-                        plane[y * H + s] = o;
-                    }
-                }
-        }
-    } else {
-#pragma unroll 1
-        for (int c = 0; c < CC; ++c) {
-            const int s = 32 * c + l;
-            const bool valid = s < NS;
-            float2 v[R1];
-#pragma unroll
-            for (int r = 0; r < R1; ++r) {
-                const int ky = w + G * r;
-                float2 a = make_float2(0.f, 0.f);
-                if (valid) {
-                    if (s == 0) {
-                        const float2 d = src[ky * H], ny = src[ky * H + NS];
-                        a = make_float2(d.x - ny.y, d.y + ny.x);
-                    } else {
-                        a = src[ky * H + s];
-                    }
-                }
-                v[r] = a;
-            }
-            dft<R1, +1>(v);
-            if constexpr (QUAD) __syncthreads();  // the staged columns are read: their slots take the outputs
-            if (valid) {
-#pragma unroll
-                for (int r = 0; r < R1; ++r) plane[(w * R1 + r) * H + s] = v[r];
-            }
-            __syncthreads();
-            if (valid) {
-                float2 out[R1];
-                line_pass2<PC, +1, 1, H>(plane, w, s, tws, out);
-#pragma unroll
-                for (int i = 0; i < PC::NB; ++i)
-#pragma unroll
-                    for (int r = 0; r < G; ++r) {
-                        const int y = w + G * i + R1 * r;
-                        const float2 o = out[i * G + r];
-                        if (s == 0) {
-                            plane[y * H] = make_float2(o.x, 0.f);
-                            plane[y * H + NS] = make_float2(o.y, 0.f);
-                        } else {
-                            plane[y * H + s] = o;
-                        }
-                    }
-            }
-        }
-    }
-    __syncthreads();
-
-    // rows: C2R along kz via an N/2-point complex inverse DFT.  Each row's N
-    // real outputs replace its spectrum in shared memory, and every thread
-    // keeps the smallest (value, offset) it produced.
-    const int gi = w / GR, m = WLR ? lm : w % GR;
-    // the row a thread works on in round ro
-    auto row_of = [&](int ro) { return WLR ? 32 * ro + w + 8 * lg : ro * ROWS + gi * 32 + l; };
-    float bmin_v = INFINITY;
-    int bmin_i = 0x7fffffff;
-#pragma unroll 1
-    for (int ro = 0; ro < ROUNDS; ++ro) {
-        const int y = row_of(ro);
-        const bool valid = y < N;
-        float2* row = plane + (valid ? y : 0) * H;
-        float2 v[R1R];
-#pragma unroll
-        for (int r = 0; r < R1R; ++r) {
-            const int k = m + GR * r;
-            float2 yk = make_float2(0.f, 0.f);
-            if (valid) {
-                const float2 X = row[k], Xm = row[NS - k];
-                // A = X + conj(Xm), B = X - conj(Xm), Y = A + i * conj(w^k) * B
-                const float2 A = make_float2(X.x + Xm.x, X.y - Xm.y);
-                const float2 B = make_float2(X.x - Xm.x, X.y + Xm.y);
-                const float2 cb = cmul_conj(B, tws[k]);
-                yk = make_float2(A.x - cb.y, A.y + cb.x);
-            }
-            v[r] = yk;
-        }
-        float2 out[R1R];
-        if constexpr (WLR) {
-            __syncwarp();
-            dft<8, +1>(v);
-#pragma unroll
-            for (int r = 0; r < 8; ++r) row[8 * m + ((r + m) & 7)] = v[r];
-            __syncwarp();
-#pragma unroll
-            for (int r = 0; r < 8; ++r) {
-                float2 a = row[8 * r + ((m + r) & 7)];  // position m + 8 r
-                if (r != 0) a = ctwiddle<+1>(a, tws[2 * m * r]);
-                out[r] = a;
-            }
-            dft<8, +1>(out);
-            __syncwarp();  // the row's spectrum is consumed: its slots take the real outputs
-        } else {
-            __syncthreads();
-            dft<R1R, +1>(v);
-            if (valid) {
-#pragma unroll
-                for (int r = 0; r < R1R; ++r) row[m * R1R + r] = v[r];
-            }
-            __syncthreads();
-            if (valid) line_pass2<PR, +1, 2, 1>(row, m, 0, tws, out);
-            __syncthreads();  // the row's spectrum is consumed: its slots take the real outputs
-        }
-        const int rowbase = (x * N + y) * N;
-#pragma unroll
-        for (int i = 0; i < PR::NB; ++i)
-#pragma unroll
-            for (int r = 0; r < GR; ++r) {
-                const int mm = m + GR * i + R1R * r;
-                const float2 o = out[i * GR + r];
-                if (valid) {
-                    row[mm] = o;
-                    if constexpr (DBG) reinterpret_cast<float2*>(dbg + (size_t)q * N * N * N + rowbase)[mm] = o;
-                    if (better(o.x, rowbase + 2 * mm, bmin_v, bmin_i)) { bmin_v = o.x; bmin_i = rowbase + 2 * mm; }
-                    if (better(o.y, rowbase + 2 * mm + 1, bmin_v, bmin_i)) { bmin_v = o.y; bmin_i = rowbase + 2 * mm + 1; }
-                }
-            }
-    }
-
-    // Selection.  The KC-th best of the threads' minima bounds the plane's
-    // KC-th best from above (at least KC cells lie at or below it), so only
-    // cells at or below it can enter the plane's top KC.
-    // Every warp sorts its threads' minima; warp 0 merges the warps' 16 best
-    // (the KC best of all minima are among them).
-    static_assert(KC == 16, "the bitonic selection keeps 16 of 32 lanes");
-    // lists 0 .. nl-1 of KC (lv_s, li_s, ascending) merged pairwise over
-    // log2(nl) levels into list 0 (warp w merges list w + step into list w);
-    // every thread calls it
-    auto tree_merge = [&](int nl) {
-        for (int step = 1; step < nl; step <<= 1) {
-            __syncthreads();
-            if ((w & (2 * step - 1)) == 0 && w + step < nl) {
-                float sv = l < KC ? lv_s[w * KC + l] : lv_s[(w + step) * KC + 31 - l];
-                int si = l < KC ? li_s[w * KC + l] : li_s[(w + step) * KC + 31 - l];
-                warp_merge32(sv, si, l);
-                if (l < KC) {
-                    lv_s[w * KC + l] = sv;
-                    li_s[w * KC + l] = si;
-                }
-            }
-        }
-        __syncthreads();
-    };
-    {
-        float sv = bmin_v;
-        int si = bmin_i;
-        warp_sort32(sv, si, l);
-        if (l < KC) {
-            lv_s[w * KC + l] = sv;
-            li_s[w * KC + l] = si;
-        }
-    }
-    if (tid == 0) n_cand = 0;
-    tree_merge(G);
-    const float tv = lv_s[KC - 1];
-    const int ti = li_s[KC - 1];
-    auto offer = [&](float v, int i) {
-        if (!better(tv, ti, v, i)) {
-            const int at = atomicAdd(&n_cand, 1);
-            if (at < PCAND) { cand_sv[at] = v; cand_si[at] = i; }
-        }
-    };
-    if constexpr (WLR) {
-        // only a thread whose own minimum is at or below the bound holds
-        // cells at or below it (usually a few per plane): the warp re-reads
-        // each such lane's 64 cells together, two per lane (lane j: round
-        // j / 8, radix position j % 8 of the row pass)
-        unsigned qual = __ballot_sync(0xffffffffu, !better(tv, ti, bmin_v, bmin_i));
-        while (qual) {
-            const int L = __ffs(qual) - 1;
-            qual &= qual - 1u;
-            const int y = 32 * (l >> 3) + w + 8 * (L >> 3);
-            const int mm = (L & 7) + 8 * (l & 7);
-            const float2 o = plane[y * H + mm];
-            const int rowbase = (x * N + y) * N;
-            offer(o.x, rowbase + 2 * mm);
-            offer(o.y, rowbase + 2 * mm + 1);
-        }
-    } else {
-        // every thread re-reads its own cells (the positions the row pass gave it)
-#pragma unroll 1
-        for (int ro = 0; ro < ROUNDS; ++ro) {
-            const int y = row_of(ro);
-            if (y >= N) continue;
-            const float2* row = plane + y * H;
-            const int rowbase = (x * N + y) * N;
-#pragma unroll
-            for (int i = 0; i < PR::NB; ++i)
-#pragma unroll
-                for (int r = 0; r < GR; ++r) {
-                    const int mm = m + GR * i + R1R * r;
-                    const float2 o = row[mm];
-                    offer(o.x, rowbase + 2 * mm);
-                    offer(o.y, rowbase + 2 * mm + 1);
-                }
-        }
-    }
-    __syncthreads();
-    const int nc = n_cand;
-    if (nc <= PCAND) {
-        // warp w sorts chunks w, w + G, .. of 32 candidates and keeps their
-        // best KC in list w; the lists are then tree-merged
-        const int nchunk = (nc + 31) >> 5;
-        float sv = INFINITY;
-        int si = 0x7fffffff;
-        for (int c = w; c < nchunk; c += G) {
-            const int e = 32 * c + l;
-            float cv = e < nc ? cand_sv[e] : INFINITY;
-            int ci = e < nc ? cand_si[e] : 0x7fffffff;
-            warp_sort32(cv, ci, l);
-            if (c == w) {
-                sv = cv;
-                si = ci;
-            } else {
-                const float rv = __shfl_sync(0xffffffffu, cv, 31 - l);
-                const int ri = __shfl_sync(0xffffffffu, ci, 31 - l);
-                if (l >= KC) {
-                    sv = rv;
-                    si = ri;
-                }
-                warp_merge32(sv, si, l);
-            }
-        }
-        if (l < KC) {
-            lv_s[w * KC + l] = sv;
-            li_s[w * KC + l] = si;
-        }
-        tree_merge(nchunk < G ? nchunk : G);
-        if (w == 0 && l < KC) {
-            cand_v[((size_t)q * N + x) * KC + l] = lv_s[l];
-            cand_i[((size_t)q * N + x) * KC + l] = li_s[l];
-        }
-        return;
-    }
-    // many cells tie at the bound (a flat plane): every warp offers its own
-    // cells, then warp 0 merges the warps' lists
-    WarpTopK tk;
-    tk.init();
-#pragma unroll 1
-    for (int ro = 0; ro < ROUNDS; ++ro) {
-        const int y = row_of(ro);
-        const bool valid = y < N;
-        const float2* row = plane + (valid ? y : 0) * H;
-        const int rowbase = (x * N + y) * N;
-#pragma unroll
-        for (int i = 0; i < PR::NB; ++i)
-#pragma unroll
-            for (int r = 0; r < GR; ++r) {
-                const int mm = m + GR * i + R1R * r;
-                const float2 o = valid ? row[mm] : make_float2(INFINITY, INFINITY);
-                tk.offer(o.x, valid ? rowbase + 2 * mm : 0x7fffffff, l);
-                tk.offer(o.y, valid ? rowbase + 2 * mm + 1 : 0x7fffffff, l);
-            }
-    }
-    if (l < KC) {
-        lv_s[w * KC + l] = tk.lv;
-        li_s[w * KC + l] = tk.li;
-    }
-    __syncthreads();
-    if (w == 0) {
-        merge_lists(lv_s, li_s, G * KC, tk, l);
-        if (l < KC) {
-            cand_v[((size_t)q * N + x) * KC + l] = tk.lv;
-            cand_i[((size_t)q * N + x) * KC + l] = tk.li;
-        }
-    }
-}
+// K3, the plane stage: plane_lines.cuh
 
 // ---------------------------------------------------------------------------
 // K4: per-rotation merge of the plane pools, FP64 direct-space rescoring of
