@@ -15,7 +15,7 @@
 // run the same line FFT in FP64.
 //
 // Layout (Hz = Nz/2 + 1, pencil p = ky Hz + kz, PP = Ny Hz rounded up to 32):
-//   spec  [K][PP][Nx]  float2  R^_t(kx, p) / V (pencil-major: coalesced along kx)
+//   spec  [K][Nx][PP]  float2  R^_t(kx, p) / V
 //   rgrid [K][V]       double  real-space receptor terms (FP64 rescoring)
 //   ent   [B][n_ent]   uint32  t << 24 | x << 16 | y << 8 | z, sorted by (t, x)
 //   offs  [B][K Nx+1]  int32   start of bin (t, x)
@@ -234,24 +234,6 @@ __global__ void __launch_bounds__(32 * kBoxWarps) box_line_fft64_kernel(double2*
     for (int e = lane; e < n; e += 32) line[(long)e * elem_stride] = r[e];
 }
 
-// half spectrum [Nx][Ny Hz] (FP64) -> the pencil stage's spectra [PP][Nx]
-// (FP32, scaled; pencils past Ny Hz are zero): a warp reads one pencil's
-// kx values as consecutive words
-__global__ void box_pack_spectrum_kernel(const double2* __restrict__ half, float2* __restrict__ spec, int nx,
-                                         int nh, int pp, double scale) {
-    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const size_t tot = (size_t)nx * pp;
-    if (i >= tot) return;
-    const size_t p = i / nx;
-    const int kx = (int)(i - p * nx);
-    float2 o = make_float2(0.f, 0.f);
-    if (p < (size_t)nh) {
-        const double2 v = half[(size_t)kx * nh + p];
-        o = make_float2((float)(v.x * scale), (float)(v.y * scale));
-    }
-    spec[i] = o;
-}
-
 // [Nx][Ny][Nz] complex -> [Nx][Ny][Hz]
 __global__ void box_half_extract_kernel(const double2* __restrict__ full, double2* __restrict__ half, int nx, int ny,
                                         int nz, int hz) {
@@ -273,13 +255,14 @@ __global__ void __launch_bounds__(256) box_prep_kernel(const double* __restrict_
                                                        const int32_t* __restrict__ lig_term, int n_ent, int K, Geo geo,
                                                        uint32_t* __restrict__ ent_out, int32_t* __restrict__ offs_out,
                                                        int32_t* __restrict__ status, const float* __restrict__ w_in,
-                                                       float* __restrict__ w_out, int32_t* __restrict__ idx_out,
+                                                       uint4* __restrict__ ent4, int32_t* __restrict__ idx_out,
                                                        uint32_t* __restrict__ ent_t, const int32_t* __restrict__ tpad,
-                                                       int n_pad, int x0, int W) {
+                                                       int n_pad, int x0, int W, int qc) {
     extern __shared__ unsigned char smem_raw[];
     const int nx = geo.n[0], ny = geo.n[1], nz = geo.n[2];
-    const int nbins = K * nx;
-    int32_t* cnt = reinterpret_cast<int32_t*>(smem_raw);           // [K*Nx + 1]
+    // bins (t, x, y mod qc), qc = 1 or 2
+    const int nbins = K * nx * qc, qm = qc - 1;
+    int32_t* cnt = reinterpret_cast<int32_t*>(smem_raw);           // [nbins + 1]
     uint32_t* keys = reinterpret_cast<uint32_t*>(cnt + nbins + 1);  // [n_ent]
     __shared__ int bad;
     __shared__ int wsum[8];
@@ -304,7 +287,7 @@ __global__ void __launch_bounds__(256) box_prep_kernel(const double* __restrict_
         c2 = min(max(c2 - 1, 0), nz - 1);
         const int t = lig_term[i];
         keys[i] = ((uint32_t)t << 24) | ((uint32_t)c0 << 16) | ((uint32_t)c1 << 8) | (uint32_t)c2;
-        atomicAdd(&cnt[t * nx + c0], 1);
+        atomicAdd(&cnt[(t * nx + c0) * qc + (c1 & qm)], 1);
     }
     __syncthreads();
     {
@@ -341,7 +324,7 @@ __global__ void __launch_bounds__(256) box_prep_kernel(const double* __restrict_
             const int i = base + tid;
             const bool act = i < n_ent;
             const uint32_t key = act ? keys[i] : 0xffffffffu;
-            const int bin = act ? (int)((key >> 24) * nx + ((key >> 16) & 255u)) : -1;
+            const int bin = act ? (int)((key >> 24) * nx + ((key >> 16) & 255u)) * qc + (int)((key >> 8) & qm) : -1;
             const unsigned peers = __match_any_sync(0xffffffffu, bin);
             const int rank = __popc(peers & ((1u << tid) - 1u));
             const int leader = __ffs(peers) - 1;
@@ -357,8 +340,13 @@ __global__ void __launch_bounds__(256) box_prep_kernel(const double* __restrict_
                     (min(((key >> 16) - (uint32_t)x0) & 255u, (uint32_t)W) << 24) | (((key >> 8) & 255u) << 16) |
                     (key & 255u);
             }
-            if (act && w_out) {
-                w_out[(size_t)q * n_ent + dst] = w_in[i];
+            if (act && ent4) {
+                // ljComp: entry i < n_ent / 2 weighs atom i into term 0, entry
+                // i + n_ent / 2 the same atom into term 1
+                const int half = n_ent >> 1;
+                if (i < half)
+                    ent4[(size_t)q * half + dst] =
+                        make_uint4(key, __float_as_uint(w_in[i]), __float_as_uint(w_in[i + half]), 0u);
                 idx_out[(size_t)q * n_ent + dst] = i;
             }
             if (act && tid == leader) cnt[bin] += __popc(peers);
@@ -366,124 +354,6 @@ __global__ void __launch_bounds__(256) box_prep_kernel(const double* __restrict_
         }
     }
     if (tid == 0) status[q] = bad;
-}
-
-// ---------------------------------------------------------------------------
-// pencil stage: CTA = one rotation x 8 pencils, one warp per pencil (ky, kz):
-//   F(x) = sum over entries of bin (t, x) of w e^{-2 pi i (ky y / Ny + kz z / Nz)}
-//   S(kx) += conj(R^_t(kx)) FFT_x(F)(kx)   over the terms
-//   g2[x][p] = IFFT_x(S)(x)
-// The warp first tabulates its pencil's phases along y and z (Ny + Nz
-// values), so an entry costs two lookups and a complex product.  The lanes
-// take a term's entries 32 at a time; entries are sorted by x, so a
-// segmented scan over the lanes sums each x bin's entries and the last lane
-// of each bin adds the sum into F(x): every lane has work whatever the bin
-// sizes, and the additions happen in one fixed order.
-// ---------------------------------------------------------------------------
-template <bool WEIGHTED>
-__global__ void __launch_bounds__(32 * kBoxWarps, 2) box_pencil_kernel(
-    const float2* __restrict__ spec, const uint32_t* __restrict__ ent, const int32_t* __restrict__ offs,
-    const float* __restrict__ ent_w, const float2* __restrict__ twx_g, const float2* __restrict__ twy_g,
-    const float2* __restrict__ twz_g, BoxPlan plx, float2* __restrict__ g2, int K, int n_ent, int ny, int nz, int pp) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    const int nx = plx.n, hz = nz / 2 + 1, np = ny * hz;
-    const int wstride = ny + nz + 3 * nx;
-    float2* twx = reinterpret_cast<float2*>(smem_raw);  // [nx]
-    float2* twy = twx + nx;                             // [ny]
-    float2* twz = twy + ny;                             // [nz]
-    float2* wbuf = twz + nz;                            // [8][ny + nz + 3 nx]
-    float2* otile = wbuf + kBoxWarps * wstride;         // [nx][8]
-    uint32_t* ent_s = reinterpret_cast<uint32_t*>(otile + kBoxWarps * nx);  // [n_ent]
-    float* w_s = reinterpret_cast<float*>(ent_s + n_ent);                     // WEIGHTED: [n_ent]
-    int32_t* tstart = reinterpret_cast<int32_t*>(w_s + (WEIGHTED ? n_ent : 0));  // [K + 1]
-
-    const int q = blockIdx.x;
-    const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
-    for (int i = tid; i < nx; i += blockDim.x) twx[i] = twx_g[i];
-    for (int i = tid; i < ny; i += blockDim.x) twy[i] = twy_g[i];
-    for (int i = tid; i < nz; i += blockDim.x) twz[i] = twz_g[i];
-    const uint32_t* eq = ent + (size_t)q * n_ent;
-    for (int i = tid; i < n_ent; i += blockDim.x) {
-        ent_s[i] = eq[i];
-        if (WEIGHTED) w_s[i] = ent_w[(size_t)q * n_ent + i];
-    }
-    // entries of term t: [tstart[t], tstart[t + 1]) (sorted by (t, x))
-    const int32_t* oq = offs + (size_t)q * (K * nx + 1);
-    for (int t = tid; t <= K; t += blockDim.x) tstart[t] = t < K ? oq[t * nx] : n_ent;
-    __syncthreads();
-
-    const int p = blockIdx.y * kBoxWarps + w;
-    if (p < np) {
-        const int ky = p / hz, kz = p - (p / hz) * hz;
-        float2* phy = wbuf + (size_t)w * wstride;  // [ny] e^{-2 pi i ky y / Ny}
-        float2* phz = phy + ny;                     // [nz] e^{-2 pi i kz z / Nz}
-        float2* a = phz + nz;
-        float2* b = a + nx;
-        float2* acc = b + nx;
-        for (int y = lane; y < ny; y += 32) phy[y] = twy[(ky * y) % ny];
-        for (int z = lane; z < nz; z += 32) phz[z] = twz[(kz * z) % nz];
-        for (int x = lane; x < nx; x += 32) acc[x] = make_float2(0.f, 0.f);
-        for (int t = 0; t < K; ++t) {
-            for (int x = lane; x < nx; x += 32) a[x] = make_float2(0.f, 0.f);
-            __syncwarp();
-            const int j1 = tstart[t + 1];
-            for (int base = tstart[t]; base < j1; base += 32) {
-                const int j = base + lane;
-                const bool act = j < j1;
-                const uint32_t e = act ? ent_s[j] : 0u;
-                const int xk = act ? (int)((e >> 16) & 255u) : -1;
-                float2 v = make_float2(0.f, 0.f);
-                if (act) {
-                    v = c_mul(phy[(e >> 8) & 255u], phz[e & 255u]);
-                    if (WEIGHTED) {
-                        const float wj = w_s[j];
-                        v.x *= wj;
-                        v.y *= wj;
-                    }
-                }
-                // segmented inclusive scan over lanes with equal x (contiguous: sorted)
-#pragma unroll
-                for (int o = 1; o < 32; o <<= 1) {
-                    const float ux = __shfl_up_sync(0xffffffffu, v.x, o);
-                    const float uy = __shfl_up_sync(0xffffffffu, v.y, o);
-                    const int uk = __shfl_up_sync(0xffffffffu, xk, o);
-                    if (lane >= o && uk == xk) {
-                        v.x += ux;
-                        v.y += uy;
-                    }
-                }
-                const int nk = __shfl_down_sync(0xffffffffu, xk, 1);
-                if (act && (lane == 31 || nk != xk)) {
-                    float2 f = a[xk];
-                    f.x += v.x;
-                    f.y += v.y;
-                    a[xk] = f;
-                }
-                __syncwarp();
-            }
-            const float2* fx = warp_fft<float2, -1>(a, b, twx, plx, lane);
-            const float2* sp = spec + ((size_t)t * pp + p) * nx;
-            for (int kx = lane; kx < nx; kx += 32) {
-                const float2 f = fx[kx];
-                const float2 rv = __ldg(sp + kx);
-                float2 s = acc[kx];
-                s.x += f.x * rv.x + f.y * rv.y;
-                s.y += f.y * rv.x - f.x * rv.y;
-                acc[kx] = s;
-            }
-            __syncwarp();
-        }
-        for (int x = lane; x < nx; x += 32) a[x] = acc[x];
-        const float2* out = warp_fft<float2, +1>(a, b, twx, plx, lane);
-        for (int x = lane; x < nx; x += 32) otile[x * kBoxWarps + w] = out[x];
-    }
-    __syncthreads();
-    // the CTA's 8 pencils of every x plane: 64 contiguous bytes per plane
-    float2* dst = g2 + (size_t)q * nx * pp + (size_t)blockIdx.y * kBoxWarps;
-    for (int i = tid; i < nx * kBoxWarps; i += blockDim.x) {
-        const int x = i / kBoxWarps, ww = i - x * kBoxWarps;
-        if (blockIdx.y * kBoxWarps + ww < np) dst[(size_t)x * pp + ww] = otile[i];
-    }
 }
 
 // ---------------------------------------------------------------------------
@@ -595,7 +465,10 @@ __global__ void __launch_bounds__(256) box_finalize_kernel(
     }
 }
 
-size_t pencil_smem_bytes(int nx, int ny, int nz, int K, int n_ent, bool weighted) {
+// the pencil stage's share of the size limit a ligand is accepted under
+// (tables, line buffers and staged entries of 8 pencils per CTA;
+// pencil_lines_kernel needs less and nothing per entry)
+size_t pencil_limit_bytes(int nx, int ny, int nz, int K, int n_ent, bool weighted) {
     return (size_t)(nx + ny + nz) * sizeof(float2) + (size_t)kBoxWarps * (ny + nz + 3 * nx) * sizeof(float2) +
            (size_t)kBoxWarps * nx * sizeof(float2) + (size_t)n_ent * sizeof(uint32_t) * (weighted ? 2 : 1) +
            ((size_t)K + 1) * sizeof(int32_t);
@@ -606,8 +479,8 @@ size_t plane_limit_bytes(int ny, int nz) {
     const int hz = nz / 2 + 1, lmax = std::max(ny, nz);
     return ((size_t)ny * (hz | 1) + ny + nz + nz / 2 + (size_t)16 * 2 * lmax) * sizeof(float2);
 }
-size_t prep_smem_bytes(int nx, int K, int n_ent) {
-    return ((size_t)K * nx + 1) * sizeof(int32_t) + (size_t)n_ent * sizeof(uint32_t);
+size_t prep_smem_bytes(int nx, int K, int n_ent, int qc) {
+    return ((size_t)K * nx * qc + 1) * sizeof(int32_t) + (size_t)n_ent * sizeof(uint32_t);
 }
 
 cudaError_t set_smem(const void* fn, size_t bytes) {
@@ -618,12 +491,12 @@ cudaError_t set_smem(const void* fn, size_t bytes) {
 cudaError_t box_prep(const BatchArgs& a, cudaStream_t s) {
     const int nb = a.n_rot;
     if (nb <= 0) return cudaSuccess;
-    const size_t sm = prep_smem_bytes(a.box.n[0], a.K, a.n_ent);
+    const size_t sm = prep_smem_bytes(a.box.n[0], a.K, a.n_ent, a.classes());
     cudaError_t e = set_smem((const void*)box_prep_kernel, sm);
     if (e != cudaSuccess) return e;
     box_prep_kernel<<<nb, 256, sm, s>>>(a.rot, a.lig_xyz, a.lig_term, a.n_ent, a.K, a.box, a.ent, a.offs, a.status,
-                                        a.lig_w32, a.lig_w32 ? a.ent_w : nullptr, a.ent_idx,
-                                        a.use_tc ? a.ent_t : nullptr, a.tpad, a.n_pad, a.x0, a.W);
+                                        a.lig_w32, a.lig_w32 ? a.ent4 : nullptr, a.ent_idx,
+                                        a.use_tc ? a.ent_t : nullptr, a.tpad, a.n_pad, a.x0, a.W, a.classes());
     return cudaGetLastError();
 }
 
@@ -631,15 +504,11 @@ cudaError_t box_middle(const BatchArgs& a, cudaStream_t s) {
     const int nb = a.n_rot;
     if (nb <= 0) return cudaSuccess;
     const int nx = a.box.n[0], ny = a.box.n[1], nz = a.box.n[2];
-    BoxPlan px;
-    if (!factor_plan(nx, px)) return cudaErrorInvalidValue;
     const float2* twx = a.box_tw32;
     const float2* twy = twx + nx;
     const float2* twz = twy + ny;
     cudaError_t e;
     if (a.ev && (e = cudaEventRecord(a.ev[0], s)) != cudaSuccess) return e;
-    const bool weighted = a.lig_w32 != nullptr;
-    const size_t sm2 = pencil_smem_bytes(nx, ny, nz, a.K, a.n_ent, weighted);
     const int np = ny * (nz / 2 + 1);
     if (a.use_tc) {
         // tensor form: the x stage as split-FP16 tcgen05 GEMMs over 128
@@ -667,19 +536,7 @@ cudaError_t box_middle(const BatchArgs& a, cudaStream_t s) {
         if (a.ev && (e = cudaEventRecord(a.ev[2], s)) != cudaSuccess) return e;
         return cudaSuccess;
     }
-    dim3 grid2(nb, (np + kBoxWarps - 1) / kBoxWarps);
-    if (weighted) {
-        if ((e = set_smem((const void*)box_pencil_kernel<true>, sm2)) != cudaSuccess) return e;
-        box_pencil_kernel<true><<<grid2, 32 * kBoxWarps, sm2, s>>>(static_cast<const float2*>(a.spec), a.ent, a.offs,
-                                                                  a.ent_w, twx, twy, twz, px, a.g2, a.K, a.n_ent, ny,
-                                                                  nz, a.PP);
-    } else {
-        if ((e = set_smem((const void*)box_pencil_kernel<false>, sm2)) != cudaSuccess) return e;
-        box_pencil_kernel<false><<<grid2, 32 * kBoxWarps, sm2, s>>>(static_cast<const float2*>(a.spec), a.ent,
-                                                                   a.offs, nullptr, twx, twy, twz, px, a.g2, a.K,
-                                                                   a.n_ent, ny, nz, a.PP);
-    }
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    if ((e = box_pencil(a, twx, twy, twz, s)) != cudaSuccess) return e;
     if (a.ev && (e = cudaEventRecord(a.ev[1], s)) != cudaSuccess) return e;
     e = box_plane(a, twy, twz, false, s);
     if (e != cudaSuccess) return e;
@@ -711,7 +568,7 @@ size_t box_pencil_smem_unknown(int, int) { return 0; }
 cudaError_t box_load_kernels(int) {
     cudaFuncAttributes fa;
     cudaError_t e = cudaFuncGetAttributes(&fa, (const void*)box_prep_kernel);
-    if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, (const void*)box_pencil_kernel<false>);
+    if (e == cudaSuccess) e = box_pencil_load();
     if (e == cudaSuccess) e = box_plane_load();
     if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, (const void*)box_finalize_kernel);
     return e;
@@ -722,8 +579,8 @@ cudaError_t box_load_kernels(int) {
 bool box_plan(int n, BoxPlan* pl) { return factor_plan(n, *pl); }
 
 size_t box_pencil_smem(int nx, int ny, int nz, int K, int n_ent, bool weighted) {
-    return std::max(pencil_smem_bytes(nx, ny, nz, K, n_ent, weighted),
-                    std::max(plane_limit_bytes(ny, nz), prep_smem_bytes(nx, K, n_ent)));
+    return std::max(pencil_limit_bytes(nx, ny, nz, K, n_ent, weighted),
+                    std::max(plane_limit_bytes(ny, nz), prep_smem_bytes(nx, K, n_ent, 1)));
 }
 
 // Forward transform of one real FP64 term grid [Nx][Ny][Nz] into spec_t
@@ -767,8 +624,8 @@ cudaError_t box_receptor_fft(const double* rgrid_t, double2* cbuf, double2* hbuf
     // x: lines p = (ky, kz)
     if ((e = lines(hbuf, twx, px, (long)ny * hz, (long)ny * hz, (long)ny * hz, 1, 0)) != cudaSuccess) return e;
     const size_t tot = (size_t)nx * PP;
-    box_pack_spectrum_kernel<<<(unsigned)((tot + 255) / 256), 256, 0, s>>>(hbuf, static_cast<float2*>(spec_t), nx,
-                                                                           ny * hz, PP, 1.0 / (double)V);
+    pack_spectrum_kernel<<<(unsigned)((tot + 255) / 256), 256, 0, s>>>(hbuf, static_cast<float2*>(spec_t), nx, ny * hz, PP,
+                                                                       1.0 / (double)V);
     return cudaGetLastError();
 }
 

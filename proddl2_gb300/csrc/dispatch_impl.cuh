@@ -5,6 +5,7 @@
 #include "internal.h"
 #include "scan_kernels.cuh"
 #include "pencil_tc.cuh"
+#include "pencil_lines.cuh"
 #include "plane_lines.cuh"
 
 namespace fftdock {
@@ -19,9 +20,7 @@ template <int N> struct SizeOpsImpl {
     static constexpr int G = SizeTraits<N>::G;
     static constexpr int H = N / 2 + 1;
 
-    static size_t pencil_smem_w(int K, int n_ent, bool weighted) {
-        return pencil_smem(K, n_ent) + (weighted ? (size_t)n_ent * sizeof(float) : 0);
-    }
+    // shared memory of pencil_kernel, and the size limit a ligand is accepted under
     static size_t pencil_smem(int K, int n_ent) {
         return (size_t)PencilTraits<N>::BUFS * N * 32 * sizeof(float2) + (size_t)N * 17 * sizeof(float2) +
                ((size_t)K * N + 1) * sizeof(int32_t) +
@@ -95,13 +94,29 @@ template <int N> struct SizeOpsImpl {
         return cudaGetLastError();
     }
 
-    template <typename SpecT, bool W> static cudaError_t launch_pencil(const BatchArgs& a, int nb, cudaStream_t s) {
-        const size_t sm2 = pencil_smem_w(a.K, a.n_ent, W);
-        cudaError_t e = set_smem((const void*)pencil_kernel<N, SpecT, W>, sm2);
+    template <typename SpecT> static cudaError_t launch_pencil(const BatchArgs& a, int nb, cudaStream_t s) {
+        const size_t sm2 = pencil_smem(a.K, a.n_ent);
+        cudaError_t e = set_smem((const void*)pencil_kernel<N, SpecT>, sm2);
         if (e != cudaSuccess) return e;
         dim3 grid2(nb, a.PP / 32);
-        pencil_kernel<N, SpecT, W><<<grid2, 32 * G, sm2, s>>>(static_cast<const SpecT*>(a.spec), a.ent, a.offs,
-                                                              a.tw32, a.g2, a.K, a.n_ent, a.ent_w);
+        pencil_kernel<N, SpecT><<<grid2, 32 * G, sm2, s>>>(static_cast<const SpecT*>(a.spec), a.ent, a.offs, a.tw32,
+                                                           a.g2, a.K, a.n_ent);
+        return cudaGetLastError();
+    }
+    // one term, or ljComp's two terms over the same atoms
+    template <typename SpecT, bool PAIRED>
+    static cudaError_t launch_pencil_lines(const BatchArgs& a, int nb, cudaStream_t s) {
+        constexpr int Q = kPencilQ, NT = pencil_threads(N, PAIRED);
+        const auto fn = &pencil_lines_kernel<N, SpecT, PAIRED, Q, NT, pencil_ctas(N, PAIRED)>;
+        size_t sm = pencil_lines_smem_cubic(N, Q, PAIRED);
+        const size_t st = pencil_stage_bytes(N, a.K, Q, a.n_ent, PAIRED);
+        const int staged = sm + st <= kPencilMaxSmem ? 1 : 0;
+        if (staged) sm += st;
+        cudaError_t e = set_smem((const void*)fn, sm);
+        if (e != cudaSuccess) return e;
+        const dim3 grid(nb, pencil_grid_y(nb, (N / Q * H + 31) / 32));
+        fn<<<grid, NT, sm, s>>>(static_cast<const SpecT*>(a.spec), a.ent, a.ent4, a.offs, a.tw32, a.tw32, a.tw32,
+                                LineRadices{}, N, N, N, a.PP, a.K, a.n_ent, staged, a.g2);
         return cudaGetLastError();
     }
 
@@ -118,13 +133,13 @@ template <int N> struct SizeOpsImpl {
         const int nb = a.n_rot;
         if (nb <= 0) return cudaSuccess;
         const Geo geo = make_geo(a.h, N, N, N);
-        const size_t sm1 = ((size_t)a.K * N + 1) * sizeof(int32_t) + (size_t)a.n_ent * sizeof(uint32_t);
+        const size_t sm1 = a.offs_stride(N) * sizeof(int32_t) + (size_t)a.n_ent * sizeof(uint32_t);
         cudaError_t e = set_smem((const void*)ligand_prep_kernel<N>, sm1);
         if (e != cudaSuccess) return e;
         ligand_prep_kernel<N><<<nb, 256, sm1, s>>>(a.rot, a.lig_xyz, a.lig_term, a.n_ent, a.K, geo, a.ent, a.offs,
-                                                    a.status, a.lig_w32, a.lig_w32 ? a.ent_w : nullptr, a.ent_idx,
+                                                    a.status, a.lig_w32, a.lig_w32 ? a.ent4 : nullptr, a.ent_idx,
                                                     a.use_tc ? a.ent_t : nullptr, a.tpad, a.n_pad, a.x0,
-                                                    a.W);
+                                                    a.W, a.classes());
         return cudaGetLastError();
     }
 
@@ -155,9 +170,12 @@ template <int N> struct SizeOpsImpl {
         if (!tc) {
             if (a.lig_w32) {
                 if (a.spec_bf16) return cudaErrorNotSupported;  // weighted sets run with FP32 spectra
-                e = launch_pencil<float2, true>(a, nb, s);
+                e = launch_pencil_lines<float2, true>(a, nb, s);
+            } else if (a.K == 1) {
+                e = a.spec_bf16 ? launch_pencil_lines<__nv_bfloat162, false>(a, nb, s)
+                                : launch_pencil_lines<float2, false>(a, nb, s);
             } else {
-                e = a.spec_bf16 ? launch_pencil<__nv_bfloat162, false>(a, nb, s) : launch_pencil<float2, false>(a, nb, s);
+                e = a.spec_bf16 ? launch_pencil<__nv_bfloat162>(a, nb, s) : launch_pencil<float2>(a, nb, s);
             }
             if (e != cudaSuccess) return e;
         }
@@ -204,9 +222,15 @@ template <int N> struct SizeOpsImpl {
     static cudaError_t load_fft_form(int spec_bf16) {
         cudaFuncAttributes fa;
         cudaError_t e = cudaFuncGetAttributes(&fa, (const void*)ligand_prep_kernel<N>);
+        constexpr int C = pencil_ctas(N, false);
         if (e == cudaSuccess)
-            e = spec_bf16 ? cudaFuncGetAttributes(&fa, (const void*)pencil_kernel<N, __nv_bfloat162, false>)
-                          : cudaFuncGetAttributes(&fa, (const void*)pencil_kernel<N, float2, false>);
+            e = spec_bf16 ? cudaFuncGetAttributes(&fa, (const void*)pencil_kernel<N, __nv_bfloat162>)
+                          : cudaFuncGetAttributes(&fa, (const void*)pencil_kernel<N, float2>);
+        if (e == cudaSuccess)
+            e = spec_bf16 ? cudaFuncGetAttributes(
+                                &fa, (const void*)pencil_lines_kernel<N, __nv_bfloat162, false, kPencilQ, kPencilThreads, C>)
+                          : cudaFuncGetAttributes(&fa,
+                                                  (const void*)pencil_lines_kernel<N, float2, false, kPencilQ, kPencilThreads, C>);
         if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, (const void*)plane_lines_kernel<N, kPlanePlanes, plane_threads(N, false)>);
         if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, (const void*)finalize_kernel<N>);
         return e;

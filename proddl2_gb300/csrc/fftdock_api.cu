@@ -44,6 +44,7 @@ struct fftdock_ctx {
     std::vector<double> ace;
     const SizeOps* ops = nullptr;
     int N = 0, H = 0, PP = 0, K = 0, B = 0;
+    int qc = 1;  // entry classes per x bin of the FFT pencil form
     size_t V = 0;
     double h = 0, zero_h = 0, center0 = 0;
     // per-axis sizes and geometry (all N on a cubic grid); box: the box-grid
@@ -70,10 +71,10 @@ struct fftdock_ctx {
     bool lj = false;
     float* lig_w32 = nullptr;
     double* lig_w64 = nullptr;
-    float* ent_w = nullptr;
+    uint4* ent4 = nullptr;
     int32_t* ent_idx = nullptr;
 
-    // work: ent/offs/cand (and ent_w/ent_idx) per group of G rotations,
+    // work: ent/offs/cand (and ent4/ent_idx) per group of G rotations,
     // g2 per batch of B
     int G = 0;
     uint32_t* ent = nullptr;
@@ -188,7 +189,8 @@ BatchArgs batch_args(fftdock_ctx* ctx) {
     a.lig_term = ctx->lig_term;
     a.lig_w32 = ctx->lig_w32;
     a.lig_w64 = ctx->lig_w64;
-    a.ent_w = ctx->ent_w;
+    a.ent4 = ctx->ent4;
+    a.qc = ctx->qc;
     a.ent_idx = ctx->ent_idx;
     a.spec = ctx->spec;
     a.spec_bf16 = ctx->cfg.precision == FFTDOCK_PREC_BF16_SPECTRA ? 1 : 0;
@@ -303,10 +305,10 @@ int run_batches(fftdock_ctx* ctx, int n_rot, const double* rot, int first_id, ff
             if (b.pool_v) b.pool_v += (size_t)j * fftdock::kKC;
             if (b.pool_i) b.pool_i += (size_t)j * fftdock::kKC;
             b.ent += (size_t)j * ctx->n_ent;
-            b.offs += (size_t)j * (ctx->K * N + 1);
+            b.offs += (size_t)j * b.offs_stride(N);
             b.cand_v += (size_t)j * N * fftdock::kKC;
             b.cand_i += (size_t)j * N * fftdock::kKC;
-            if (b.ent_w) b.ent_w += (size_t)j * ctx->n_ent;
+            if (b.ent4) b.ent4 += (size_t)j * (ctx->n_ent / 2);
             if (b.ent_idx) b.ent_idx += (size_t)j * ctx->n_ent;
             if (b.ent_t) b.ent_t += (size_t)j * ctx->n_pad;  // j is a multiple of 128 on the tensor path
             cudaEvent_t evs[4];
@@ -556,7 +558,7 @@ void fftdock_destroy(fftdock_ctx* ctx) {
     dfree(ctx->lig_term);
     dfree(ctx->lig_w32);
     dfree(ctx->lig_w64);
-    dfree(ctx->ent_w);
+    dfree(ctx->ent4);
     dfree(ctx->ent_idx);
     dfree(ctx->ent);
     dfree(ctx->offs);
@@ -700,6 +702,9 @@ int fftdock_create(const fftdock_config* cfg_in, fftdock_ctx** out) {
     // the tensor stage takes rotations in groups of 128
     if (ctx->use_tc) ctx->B = (ctx->B + fftdock::kTcRot - 1) / fftdock::kTcRot * fftdock::kTcRot;
     ctx->G = group_size(ctx->B);
+    const bool paired = c.term_set == FFTDOCK_TERMS_LJ_COMP;
+    ctx->qc = ctx->box ? fftdock::box_pencil_classes(dims, ctx->K, paired)
+                       : fftdock::cubic_pencil_classes(ctx->K, paired);
     // centred geometry exactly as UniformCubicGeometry(step, logicalSize)
     const double h = c.grid_step;
     const double s_size = h + h * (double)(N - 1);
@@ -764,7 +769,7 @@ int fftdock_create(const fftdock_config* cfg_in, fftdock_ctx** out) {
         ctx->spec = sp;
     }
     CK(dalloc(&ctx->rgrid, (size_t)ctx->K * ctx->V));
-    CK(dalloc(&ctx->offs, (size_t)ctx->G * (ctx->K * N + 1)));
+    CK(dalloc(&ctx->offs, (size_t)ctx->G * (ctx->K * N * ctx->qc + 1)));
     CK(dalloc(&ctx->g2, (size_t)ctx->B * N * ctx->PP));
     // pencils (ky, kz) and the x extent of the tensor stage's x-quads
     const size_t n_pencils = (size_t)dims[1] * ctx->H;
@@ -1181,7 +1186,7 @@ int fftdock_set_pair_lj(fftdock_ctx* ctx, int32_t n_rec, const double* rec_xyz, 
     dfree(ctx->lig_w32);
     dfree(ctx->lig_w64);
     dfree(ctx->ent);
-    dfree(ctx->ent_w);
+    dfree(ctx->ent4);
     dfree(ctx->ent_idx);
     CK(dalloc(&ctx->lig_xyz, exyz.size()));
     CK(dalloc(&ctx->lig_term, (size_t)n_ent));
@@ -1191,7 +1196,7 @@ int fftdock_set_pair_lj(fftdock_ctx* ctx, int32_t n_rec, const double* rec_xyz, 
     if (comp) {
         CK(dalloc(&ctx->lig_w32, (size_t)n_ent));
         CK(dalloc(&ctx->lig_w64, (size_t)n_ent));
-        CK(dalloc(&ctx->ent_w, (size_t)ctx->G * n_ent));
+        CK(dalloc(&ctx->ent4, (size_t)ctx->G * n_lig));
         CK(dalloc(&ctx->ent_idx, (size_t)ctx->G * n_ent));
         CK(cudaMemcpy(ctx->lig_w32, w32.data(), (size_t)n_ent * sizeof(float), cudaMemcpyHostToDevice));
         CK(cudaMemcpy(ctx->lig_w64, w64.data(), (size_t)n_ent * sizeof(double), cudaMemcpyHostToDevice));

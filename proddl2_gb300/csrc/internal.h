@@ -161,6 +161,10 @@ constexpr int kBoxMax = 256;
 
 // Everything one device batch of rotations needs.
 struct BatchArgs {
+    // classes in effect (the tensor form takes plain (term, x) bins) and the
+    // bin starts of one rotation
+    int classes() const { return use_tc ? 1 : qc; }
+    size_t offs_stride(int nx) const { return (size_t)K * nx * classes() + 1; }
     // inputs
     const double* rot;          // [B][9]
     const double* lig_xyz;      // [n_ent][3]
@@ -178,9 +182,10 @@ struct BatchArgs {
     double h, zero_h, center0;
     // work
     uint32_t* ent;              // [B][n_ent]
-    float* ent_w;               // weighted: [B][n_ent] weights in sorted order
+    uint4* ent4;                // ljComp: [B][n_ent / 2] sorted entries with both terms' weights (pencil_lines.cuh)
     int32_t* ent_idx;           // weighted: [B][n_ent] entry index in sorted order
-    int32_t* offs;              // [B][K*N+1]
+    int32_t* offs;              // [B][K Nx classes + 1] bin starts (offs_stride)
+    int qc;                     // classes y mod qc the FFT form sorts an x bin's entries by (1 or 2)
     int32_t* status;            // [B]
     float2* g2;                 // [B][N][PP]
     float* cand_v;              // [B][N][KC]
@@ -290,6 +295,14 @@ cudaError_t box_circ_scales(const float2* circ, int K, int nh, int nx, int8_t* c
 // cubic grid of edge n
 size_t box_tc_smem(const int dims[3], int n_chunks, int n_terms);
 size_t cubic_tc_smem(int n, int n_chunks, int n_terms);
+
+// FFT form of the pencil stage on a box grid: entry classes per x bin, the
+// launch, and its kernels' code
+int box_pencil_classes(const int dims[3], int K, bool paired);
+cudaError_t box_pencil(const BatchArgs& a, const float2* twx, const float2* twy, const float2* twz, cudaStream_t s);
+cudaError_t box_pencil_load();
+// the same classes on a cubic edge (K terms; paired: ljComp)
+int cubic_pencil_classes(int K, bool paired);
 
 // plane stage of a batch on a box grid (quad: from the tensor stage's x-quads)
 cudaError_t box_plane(const BatchArgs& a, const float2* twy, const float2* twz, bool quad, cudaStream_t s);

@@ -3,6 +3,8 @@
 
 namespace fftdock {
 
+int cubic_pencil_classes(int K, bool paired) { return K == 1 || paired ? kPencilQ : 1; }
+
 const SizeOps* size_ops_small(int n) {
     switch (n) {
         case 16: return SizeOpsImpl<16>::ops();

@@ -42,7 +42,7 @@ size_t scratch_bytes(const fftdock::ScanInputs& in, int b) {
     size_t s = 0;
     s += align256(sizeof(int32_t) * (size_t)b);                                  // status
     s += align256(sizeof(uint32_t) * (size_t)b * in.n_ent);                      // entries
-    s += align256(sizeof(int32_t) * (size_t)b * ((size_t)in.K * in.N + 1));      // bin offsets
+    s += align256(sizeof(int32_t) * (size_t)b * ((size_t)in.K * in.N * in.args.qc + 1));  // bin offsets
     s += align256(sizeof(float) * (size_t)b * in.N * kKC);                       // pool values
     s += align256(sizeof(int32_t) * (size_t)b * in.N * kKC);                     // pool offsets
     s += align256(sizeof(float2) * (size_t)b * in.N * in.PP);                    // x-inverse planes
@@ -110,7 +110,7 @@ extern "C" int fftdock_scan_device_noalloc(fftdock_ctx* ctx, int32_t n_rot, cons
     };
     int32_t* status = reinterpret_cast<int32_t*>(carve(sizeof(int32_t) * (size_t)b));
     a.ent = reinterpret_cast<uint32_t*>(carve(sizeof(uint32_t) * (size_t)b * in.n_ent));
-    a.offs = reinterpret_cast<int32_t*>(carve(sizeof(int32_t) * (size_t)b * ((size_t)in.K * in.N + 1)));
+    a.offs = reinterpret_cast<int32_t*>(carve(sizeof(int32_t) * (size_t)b * ((size_t)in.K * in.N * a.qc + 1)));
     a.cand_v = reinterpret_cast<float*>(carve(sizeof(float) * (size_t)b * in.N * kKC));
     a.cand_i = reinterpret_cast<int32_t*>(carve(sizeof(int32_t) * (size_t)b * in.N * kKC));
     a.g2 = reinterpret_cast<float2*>(carve(sizeof(float2) * (size_t)b * in.N * in.PP));

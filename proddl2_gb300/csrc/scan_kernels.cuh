@@ -6,7 +6,7 @@
 //   spec  [K][N][PP]   float2  receptor spectra R^_t(kx, p) / N^3
 //   rgrid [K][N^3]     double  real-space receptor terms (FP64 rescoring)
 //   ent   [B][n_ent]   uint32  per-rotation ligand entries t<<24|x<<16|y<<8|z,
-//                              sorted by (t, x), atom order inside a bin
+//                              sorted by (t, x, y mod qc), atom order inside a bin
 //   offs  [B][K*N+1]   int32   start of bin (t, x) at offs[t*N + x]
 //   g2    [B][N][PP]   float2  sum_t conj(R^_t) L^_t inverse-transformed
 //                              along x: one complex (ky, kz) plane per x
@@ -168,17 +168,18 @@ template <int N>
 __global__ void __launch_bounds__(256) ligand_prep_kernel(
     const double* __restrict__ rot, const double* __restrict__ lig_xyz, const int32_t* __restrict__ lig_term,
     int n_ent, int K, Geo geo, uint32_t* __restrict__ ent_out, int32_t* __restrict__ offs_out,
-    int32_t* __restrict__ status, const float* __restrict__ w_in, float* __restrict__ w_out,
+    int32_t* __restrict__ status, const float* __restrict__ w_in, uint4* __restrict__ ent4,
     int32_t* __restrict__ idx_out, uint32_t* __restrict__ ent_t, const int32_t* __restrict__ tpad, int n_pad,
-    int x0, int W) {
+    int x0, int W, int qc) {
     extern __shared__ unsigned char smem_raw[];
-    int32_t* cnt = reinterpret_cast<int32_t*>(smem_raw);          // [K*N + 1]
-    uint32_t* keys = reinterpret_cast<uint32_t*>(cnt + K * N + 1);  // [n_ent]
+    int32_t* cnt = reinterpret_cast<int32_t*>(smem_raw);               // [K*N*qc + 1]
+    uint32_t* keys = reinterpret_cast<uint32_t*>(cnt + K * N * qc + 1);  // [n_ent]
     __shared__ int bad;
     __shared__ int wsum[8];
     const int q = blockIdx.x;
     const int tid = threadIdx.x;
-    const int nbins = K * N;
+    // bins (t, x, y mod qc), qc = 1 or 2
+    const int nbins = K * N * qc, qm = qc - 1;
     for (int i = tid; i <= nbins; i += blockDim.x) cnt[i] = 0;
     if (tid == 0) bad = 0;
     __syncthreads();
@@ -199,7 +200,7 @@ __global__ void __launch_bounds__(256) ligand_prep_kernel(
         c2 = min(max(c2 - 1, 0), N - 1);
         const int t = lig_term[i];
         keys[i] = ((uint32_t)t << 24) | ((uint32_t)c0 << 16) | ((uint32_t)c1 << 8) | (uint32_t)c2;
-        atomicAdd(&cnt[t * N + c0], 1);
+        atomicAdd(&cnt[(t * N + c0) * qc + (c1 & qm)], 1);
     }
     __syncthreads();
     // exclusive scan of cnt[0..nbins) -> starts; cnt[nbins] = n_ent
@@ -238,7 +239,7 @@ __global__ void __launch_bounds__(256) ligand_prep_kernel(
             const int i = base + tid;
             const bool act = i < n_ent;
             const uint32_t key = act ? keys[i] : 0xffffffffu;
-            const int bin = act ? (int)((key >> 24) * N + ((key >> 16) & 255u)) : -1;
+            const int bin = act ? (int)((key >> 24) * N + ((key >> 16) & 255u)) * qc + (int)((key >> 8) & qm) : -1;
             const unsigned peers = __match_any_sync(0xffffffffu, bin);
             const int rank = __popc(peers & ((1u << tid) - 1u));
             const int leader = __ffs(peers) - 1;
@@ -258,8 +259,13 @@ __global__ void __launch_bounds__(256) ligand_prep_kernel(
                     (min(((key >> 16) - (uint32_t)x0) & 255u, (uint32_t)W) << 24) | (((key >> 8) & 255u) << 16) |
                     (key & 255u);
             }
-            if (act && w_out) {
-                w_out[(size_t)q * n_ent + dst] = w_in[i];
+            if (act && ent4) {
+                // ljComp: entry i < n_ent / 2 weighs atom i into term 0, entry
+                // i + n_ent / 2 the same atom into term 1
+                const int half = n_ent >> 1;
+                if (i < half)
+                    ent4[(size_t)q * half + dst] =
+                        make_uint4(key, __float_as_uint(w_in[i]), __float_as_uint(w_in[i + half]), 0u);
                 idx_out[(size_t)q * n_ent + dst] = i;
             }
             if (act && tid == leader) cnt[bin] += __popc(peers);
@@ -270,7 +276,8 @@ __global__ void __launch_bounds__(256) ligand_prep_kernel(
 }
 
 // ---------------------------------------------------------------------------
-// K2: pencil kernel.  CTA = one rotation x 32 consecutive pencils (ky, kz),
+// K2: pencil kernel of the term sets of several unweighted terms (one term
+// and ljComp: pencil_lines.cuh).  CTA = one rotation x 32 consecutive pencils (ky, kz),
 // G warps.  For every term t:
 //   F(x) = sum over entries of bin (t, x) of w^(ky*y + kz*z)   (the y and z
 //          stages of the forward transform, as direct sums over atoms)
@@ -282,10 +289,10 @@ __global__ void __launch_bounds__(256) ligand_prep_kernel(
 __device__ __forceinline__ float2 spec_load(const float2* p) { return __ldg(p); }
 __device__ __forceinline__ float2 spec_load(const __nv_bfloat162* p) { return __bfloat1622float2(*p); }
 
-template <int N, typename SpecT, bool WEIGHTED = false>
+template <int N, typename SpecT>
 __global__ void __launch_bounds__(32 * SizeTraits<N>::G, PencilTraits<N>::MINB) pencil_kernel(
     const SpecT* __restrict__ spec, const uint32_t* __restrict__ ent, const int32_t* __restrict__ offs,
-    const float2* __restrict__ tw, float2* __restrict__ g2, int K, int n_ent, const float* __restrict__ ent_w) {
+    const float2* __restrict__ tw, float2* __restrict__ g2, int K, int n_ent) {
     using P = LinePlan<N, SizeTraits<N>::G>;
     constexpr int G = P::G, R1 = P::R1, H = N / 2 + 1;
     constexpr int PP = pencil_pitch(N);
@@ -297,10 +304,8 @@ __global__ void __launch_bounds__(32 * SizeTraits<N>::G, PencilTraits<N>::MINB) 
     // are consecutive pencils, whose phases for one entry step by its z, so
     // a single table would put lanes on the same banks whenever z is even
     float2* twr = tws + N;                                  // [N][16]
-    // entries ([n_ent]; weighted: [n_ent] pairs of entry and weight bits, one
-    // 8-byte broadcast load per entry)
-    uint32_t* ent_s = reinterpret_cast<uint32_t*>(twr + N * 16);
-    int32_t* offs_s = reinterpret_cast<int32_t*>(ent_s + (WEIGHTED ? 2 : 1) * n_ent);  // [K*N+1]
+    uint32_t* ent_s = reinterpret_cast<uint32_t*>(twr + N * 16);  // [n_ent]
+    int32_t* offs_s = reinterpret_cast<int32_t*>(ent_s + n_ent);  // [K*N+1]
 
     const int q = blockIdx.x;
     const int tile = blockIdx.y;
@@ -318,16 +323,9 @@ __global__ void __launch_bounds__(32 * SizeTraits<N>::G, PencilTraits<N>::MINB) 
     const int32_t* offs_g = offs + (size_t)q * (K * N + 1);
     for (int i = tid; i <= K * N; i += blockDim.x) offs_s[i] = offs_g[i];
     const uint32_t* ent_g = ent + (size_t)q * n_ent;
-    const float* w_g = WEIGHTED ? ent_w + (size_t)q * n_ent : nullptr;
     for (int i = tid; i < n_ent; i += blockDim.x) {
         const uint32_t u = ent_g[i];
-        const uint32_t yz = (((u >> 8) & 255u) << 16) | (u & 255u);
-        if constexpr (WEIGHTED) {
-            ent_s[2 * i] = yz;
-            ent_s[2 * i + 1] = __float_as_uint(w_g[i]);
-        } else {
-            ent_s[i] = yz;
-        }
+        ent_s[i] = (((u >> 8) & 255u) << 16) | (u & 255u);
     }
     __syncthreads();
 
@@ -343,25 +341,11 @@ __global__ void __launch_bounds__(32 * SizeTraits<N>::G, PencilTraits<N>::MINB) 
             const int b = offs_s[t * N + x], e = offs_s[t * N + x + 1];
             float2 acc = make_float2(0.f, 0.f);
             for (int j = b; j < e; ++j) {
-                uint32_t ej;
-                float wj = 1.f;
-                if constexpr (WEIGHTED) {
-                    const uint2 ew = reinterpret_cast<const uint2*>(ent_s)[j];
-                    ej = ew.x;
-                    wj = __uint_as_float(ew.y);
-                } else {
-                    ej = ent_s[j];
-                }
-                const uint32_t yz = (ej * kyz) >> 16;
+                const uint32_t yz = (ent_s[j] * kyz) >> 16;
                 const unsigned ph = (N & (N - 1)) == 0 ? (yz & (unsigned)(N - 1)) : yz % (unsigned)N;
                 const float2 z = twr[ph * 16 + (l & 15)];
-                if constexpr (WEIGHTED) {
-                    acc.x = fmaf(wj, z.x, acc.x);
-                    acc.y = fmaf(wj, z.y, acc.y);
-                } else {
-                    acc.x += z.x;
-                    acc.y += z.y;
-                }
+                acc.x += z.x;
+                acc.y += z.y;
             }
             v[r] = acc;
         }
