@@ -37,214 +37,6 @@ namespace {
 
 constexpr int kBoxWarps = 8;  // lines (pencils, columns, rows) per CTA
 
-// radices in Stockham stage order; false if n has another prime factor
-bool factor_plan(int n, BoxPlan& pl) {
-    static const int radices[] = {4, 6, 2, 9, 3, 5, 7, 11, 13};
-    pl.n = n;
-    pl.nf = 0;
-    int m = n;
-    for (int r : radices)
-        while (m % r == 0 && pl.nf < kBoxMaxFactors) {
-            pl.f[pl.nf++] = r;
-            m /= r;
-        }
-    return m == 1 && n >= 2;
-}
-
-template <typename T2> __device__ __forceinline__ T2 c_mul(T2 a, T2 b) {
-    T2 r;
-    r.x = a.x * b.x - a.y * b.y;
-    r.y = a.x * b.y + a.y * b.x;
-    return r;
-}
-// table entry W_n^m = e^{-2 pi i m / n}, conjugated for the inverse transform
-template <typename T2, int SIGN> __device__ __forceinline__ T2 tw_at(const T2* tw, int m) {
-    T2 w = tw[m];
-    if (SIGN > 0) w.y = -w.y;
-    return w;
-}
-
-// one Stockham stage of radix R over a line of n points held in src:
-// butterfly j reads src[j + r n/R], applies the twiddles W^(j mod Ns) r n/(Ns R),
-// and writes its R-point DFT to dst[(j / Ns) Ns R + j mod Ns + k Ns].  The
-// twiddle index (j mod Ns) r n/(Ns R) stays below n; the R-th roots of unity
-// are held in registers for the whole stage, radices 2 and 4 need none, 6
-// is two 3-point DFTs joined by W6 twiddles.
-template <typename T2, int SIGN, int R>
-__device__ __forceinline__ void stockham_stage(const T2* src, T2* dst, const T2* tw, int n, int ns, int lane) {
-    using S = decltype(T2::x);
-    const int nb = n / R;
-    const int tstep = n / (ns * R);
-    // j / ns as a multiply-high by ceil(2^32 / ns) (ns > 1): exact for
-    // j < 2^32 / ns^2 (here j < 256 and ns <= 256)
-    const unsigned magic = ns > 1 ? 0xffffffffu / (unsigned)ns + 1u : 0u;
-    T2 root[R];
-    root[0].x = 1;  // W^0 (a composite odd radix pairs some q k = 0 mod R)
-    root[0].y = 0;
-#pragma unroll
-    for (int m = 1; m < R; ++m) root[m] = tw_at<T2, SIGN>(tw, m * nb);
-    for (int j = lane; j < nb; j += 32) {
-        T2 v[R];
-#pragma unroll
-        for (int r = 0; r < R; ++r) v[r] = src[j + r * nb];
-        const int jq = ns > 1 ? (int)__umulhi((unsigned)j, magic) : j;
-        const int jm = j - jq * ns;
-        const int step = jm * tstep;
-#pragma unroll
-        for (int r = 1; r < R; ++r) v[r] = c_mul(v[r], tw_at<T2, SIGN>(tw, step * r));
-        T2* out = dst + jq * ns * R + jm;
-        if constexpr (R == 2) {
-            T2 o0 = v[0], o1 = v[0];
-            o0.x += v[1].x; o0.y += v[1].y;
-            o1.x -= v[1].x; o1.y -= v[1].y;
-            out[0] = o0;
-            out[ns] = o1;
-        } else if constexpr (R == 6) {
-            // two 3-point DFTs of the even and odd inputs, the odd ones
-            // turned by W6^k (W6 = e^(SIGN i pi / 3)): out_k = e_k + W6^k o_k,
-            // out_(k+3) = e_k - W6^k o_k
-            constexpr S c3 = (S)0.86602540378443864676;  // sin(pi / 3)
-            constexpr S sg = SIGN < 0 ? (S)-1 : (S)1;
-            T2 e3[3], o3[3];
-#pragma unroll
-            for (int t = 0; t < 2; ++t) {
-                const T2 x0 = v[t], x1 = v[t + 2], x2 = v[t + 4];
-                T2 sm, df, u;
-                sm.x = x1.x + x2.x; sm.y = x1.y + x2.y;
-                df.x = sg * c3 * (x1.x - x2.x); df.y = sg * c3 * (x1.y - x2.y);
-                u.x = x0.x - (S)0.5 * sm.x; u.y = x0.y - (S)0.5 * sm.y;
-                T2* y = t == 0 ? e3 : o3;
-                y[0].x = x0.x + sm.x; y[0].y = x0.y + sm.y;
-                // y1 = u + i df, y2 = u - i df
-                y[1].x = u.x - df.y; y[1].y = u.y + df.x;
-                y[2].x = u.x + df.y; y[2].y = u.y - df.x;
-            }
-            // W6 = (1/2, sg c3), W6^2 = (-1/2, sg c3)
-            T2 t1, t2;
-            t1.x = (S)0.5 * o3[1].x - sg * c3 * o3[1].y; t1.y = (S)0.5 * o3[1].y + sg * c3 * o3[1].x;
-            t2.x = (S)-0.5 * o3[2].x - sg * c3 * o3[2].y; t2.y = (S)-0.5 * o3[2].y + sg * c3 * o3[2].x;
-            T2 o;
-            o.x = e3[0].x + o3[0].x; o.y = e3[0].y + o3[0].y; out[0] = o;
-            o.x = e3[1].x + t1.x; o.y = e3[1].y + t1.y; out[ns] = o;
-            o.x = e3[2].x + t2.x; o.y = e3[2].y + t2.y; out[2 * ns] = o;
-            o.x = e3[0].x - o3[0].x; o.y = e3[0].y - o3[0].y; out[3 * ns] = o;
-            o.x = e3[1].x - t1.x; o.y = e3[1].y - t1.y; out[4 * ns] = o;
-            o.x = e3[2].x - t2.x; o.y = e3[2].y - t2.y; out[5 * ns] = o;
-        } else if constexpr (R == 4) {
-            // W4 = e^(SIGN i pi / 2): out1 = (v0 - v2) + W4 (v1 - v3), out3 = (v0 - v2) - W4 (v1 - v3)
-            T2 a, b, c, d, e;
-            a.x = v[0].x + v[2].x; a.y = v[0].y + v[2].y;
-            b.x = v[0].x - v[2].x; b.y = v[0].y - v[2].y;
-            c.x = v[1].x + v[3].x; c.y = v[1].y + v[3].y;
-            e.x = v[1].x - v[3].x; e.y = v[1].y - v[3].y;
-            if (SIGN < 0) { d.x = e.y; d.y = -e.x; } else { d.x = -e.y; d.y = e.x; }
-            T2 o;
-            o.x = a.x + c.x; o.y = a.y + c.y; out[0] = o;
-            o.x = b.x + d.x; o.y = b.y + d.y; out[ns] = o;
-            o.x = a.x - c.x; o.y = a.y - c.y; out[2 * ns] = o;
-            o.x = b.x - d.x; o.y = b.y - d.y; out[3 * ns] = o;
-        } else {
-            // odd R: pairs a_q = v_q + v_(R-q), b_q = v_q - v_(R-q); with
-            // root[m] = (cos, s sin) of the stage's direction,
-            // out_k = v0 + sum_q cos(qk) a_q + i sum_q s sin(qk) b_q and
-            // out_(R-k) the same with - i
-            constexpr int P = (R - 1) / 2;
-            T2 o0 = v[0];
-#pragma unroll
-            for (int q = 1; q <= P; ++q) {
-                o0.x += v[q].x + v[R - q].x;
-                o0.y += v[q].y + v[R - q].y;
-            }
-            out[0] = o0;
-#pragma unroll
-            for (int k = 1; k <= P; ++k) {
-                T2 re = v[0];
-                S ix = 0, iy = 0;
-#pragma unroll
-                for (int q = 1; q <= P; ++q) {
-                    const T2 w = root[(q * k) % R];
-                    re.x += w.x * (v[q].x + v[R - q].x);
-                    re.y += w.x * (v[q].y + v[R - q].y);
-                    ix += w.y * (v[q].x - v[R - q].x);
-                    iy += w.y * (v[q].y - v[R - q].y);
-                }
-                // i (ix + i iy) = (-iy, ix)
-                T2 o;
-                o.x = re.x - iy; o.y = re.y + ix; out[k * ns] = o;
-                o.x = re.x + iy; o.y = re.y - ix; out[(R - k) * ns] = o;
-            }
-        }
-    }
-}
-
-// Unnormalised DFT of the warp's line in a (n points), b a second buffer of
-// n points; returns the buffer that holds the result.  SIGN -1: forward
-// e^{-2 pi i jk/n}; +1: inverse.  Ends with __syncwarp..
-template <typename T2, int SIGN>
-__device__ T2* warp_fft(T2* a, T2* b, const T2* tw, const BoxPlan& pl, int lane) {
-    T2* src = a;
-    T2* dst = b;
-    int ns = 1;
-    __syncwarp();
-    for (int s = 0; s < pl.nf; ++s) {
-        const int R = pl.f[s];
-        switch (R) {
-            case 4: stockham_stage<T2, SIGN, 4>(src, dst, tw, pl.n, ns, lane); break;
-            case 6: stockham_stage<T2, SIGN, 6>(src, dst, tw, pl.n, ns, lane); break;
-            case 2: stockham_stage<T2, SIGN, 2>(src, dst, tw, pl.n, ns, lane); break;
-            case 3: stockham_stage<T2, SIGN, 3>(src, dst, tw, pl.n, ns, lane); break;
-            case 5: stockham_stage<T2, SIGN, 5>(src, dst, tw, pl.n, ns, lane); break;
-            case 7: stockham_stage<T2, SIGN, 7>(src, dst, tw, pl.n, ns, lane); break;
-            case 9: stockham_stage<T2, SIGN, 9>(src, dst, tw, pl.n, ns, lane); break;
-            case 11: stockham_stage<T2, SIGN, 11>(src, dst, tw, pl.n, ns, lane); break;
-            default: stockham_stage<T2, SIGN, 13>(src, dst, tw, pl.n, ns, lane); break;
-        }
-        __syncwarp();
-        T2* t = src;
-        src = dst;
-        dst = t;
-        ns *= R;
-    }
-    return src;
-}
-
-// ---------------------------------------------------------------------------
-// receptor transforms (FP64), one warp per line: line L starts at
-// (L / inner_count) outer_stride + (L % inner_count) inner_stride, element e
-// at + e elem_stride; in place
-// ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(32 * kBoxWarps) box_line_fft64_kernel(double2* __restrict__ data,
-                                                                       const double2* __restrict__ tw, BoxPlan pl,
-                                                                       long n_lines, long elem_stride,
-                                                                       long inner_count, long inner_stride,
-                                                                       long outer_stride) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    const int n = pl.n;
-    double2* tws = reinterpret_cast<double2*>(smem_raw);  // [n]
-    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    double2* a = tws + n + (size_t)w * 2 * n;
-    double2* b = a + n;
-    for (int i = threadIdx.x; i < n; i += blockDim.x) tws[i] = tw[i];
-    __syncthreads();
-    const long L = (long)blockIdx.x * kBoxWarps + w;
-    if (L >= n_lines) return;
-    double2* line = data + (L / inner_count) * outer_stride + (L % inner_count) * inner_stride;
-    for (int e = lane; e < n; e += 32) a[e] = line[(long)e * elem_stride];
-    const double2* r = warp_fft<double2, -1>(a, b, tws, pl, lane);
-    for (int e = lane; e < n; e += 32) line[(long)e * elem_stride] = r[e];
-}
-
-// [Nx][Ny][Nz] complex -> [Nx][Ny][Hz]
-__global__ void box_half_extract_kernel(const double2* __restrict__ full, double2* __restrict__ half, int nx, int ny,
-                                        int nz, int hz) {
-    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const size_t tot = (size_t)nx * ny * hz;
-    if (i >= tot) return;
-    const size_t row = i / hz;
-    const int kz = (int)(i - row * hz);
-    half[i] = full[row * nz + kz];
-}
-
 // ---------------------------------------------------------------------------
 // ligand prep: rotate (the reference's operation order, no FMA), toLogical
 // per axis, bins (t, x), stable sort (one CTA per rotation)
@@ -576,62 +368,15 @@ cudaError_t box_load_kernels(int) {
 
 }  // namespace
 
-bool box_plan(int n, BoxPlan* pl) { return factor_plan(n, *pl); }
+bool box_size(int n) {
+    for (int p : {2, 3, 5, 7, 11, 13})
+        while (n % p == 0 && n > 1) n /= p;
+    return n == 1;
+}
 
 size_t box_pencil_smem(int nx, int ny, int nz, int K, int n_ent, bool weighted) {
     return std::max(pencil_limit_bytes(nx, ny, nz, K, n_ent, weighted),
                     std::max(plane_limit_bytes(ny, nz), prep_smem_bytes(nx, K, n_ent, 1)));
-}
-
-// Forward transform of one real FP64 term grid [Nx][Ny][Nz] into spec_t
-// ([Nx][PP] float2, scaled 1 / V): complex z transforms, the half spectrum
-// kz < Hz, then y and x transforms, each a batch of line FFTs.
-cudaError_t box_receptor_fft(const double* rgrid_t, double2* cbuf, double2* hbuf, const double2* tw64,
-                             const int dims[3], void* spec_t, int PP, float2* circ_t, cudaStream_t s) {
-    const int nx = dims[0], ny = dims[1], nz = dims[2], hz = nz / 2 + 1;
-    BoxPlan px, py, pz;
-    if (!factor_plan(nx, px) || !factor_plan(ny, py) || !factor_plan(nz, pz)) return cudaErrorInvalidValue;
-    const double2* twx = tw64;
-    const double2* twy = twx + nx;
-    const double2* twz = twy + ny;
-    const size_t V = (size_t)nx * ny * nz;
-    complexify_kernel<<<(unsigned)((V + 255) / 256), 256, 0, s>>>(rgrid_t, cbuf, V);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-    auto lines = [&](double2* data, const double2* tw, const BoxPlan& pl, long n_lines, long es, long ic, long is,
-                     long os) -> cudaError_t {
-        const size_t sm = ((size_t)pl.n + (size_t)kBoxWarps * 2 * pl.n) * sizeof(double2);
-        cudaError_t e2 = set_smem((const void*)box_line_fft64_kernel, sm);
-        if (e2 != cudaSuccess) return e2;
-        const long blocks = (n_lines + kBoxWarps - 1) / kBoxWarps;
-        box_line_fft64_kernel<<<(unsigned)blocks, 32 * kBoxWarps, sm, s>>>(data, tw, pl, n_lines, es, ic, is, os);
-        return cudaGetLastError();
-    };
-    // z: lines (x, y), contiguous
-    if ((e = lines(cbuf, twz, pz, (long)nx * ny, 1, 1, 0, nz)) != cudaSuccess) return e;
-    const size_t nh = (size_t)nx * ny * hz;
-    box_half_extract_kernel<<<(unsigned)((nh + 255) / 256), 256, 0, s>>>(cbuf, hbuf, nx, ny, nz, hz);
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    // y: lines (x, kz) of [Nx][Ny][Hz]
-    if ((e = lines(hbuf, twy, py, (long)nx * hz, hz, hz, 1, (long)ny * hz)) != cudaSuccess) return e;
-    if (circ_t) {
-        // transformed along z and y only: the tensor stage's circulant samples
-        const size_t tot = (size_t)nx * ny * hz;
-        pack_circ_kernel<<<(unsigned)((tot + 255) / 256), 256, 0, s>>>(hbuf, circ_t, nx, ny * hz,
-                                                                     1.0 / ((double)ny * nz));
-        if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    }
-    // x: lines p = (ky, kz)
-    if ((e = lines(hbuf, twx, px, (long)ny * hz, (long)ny * hz, (long)ny * hz, 1, 0)) != cudaSuccess) return e;
-    const size_t tot = (size_t)nx * PP;
-    pack_spectrum_kernel<<<(unsigned)((tot + 255) / 256), 256, 0, s>>>(hbuf, static_cast<float2*>(spec_t), nx, ny * hz, PP,
-                                                                       1.0 / (double)V);
-    return cudaGetLastError();
-}
-
-cudaError_t box_circ_scales(const float2* circ, int K, int nh, int nx, int8_t* cscale, cudaStream_t s) {
-    circ_scale_box_kernel<<<(nh + 127) / 128, 128, 0, s>>>(circ, K, nh, nx, cscale);
-    return cudaGetLastError();
 }
 
 size_t box_tc_smem(const int dims[3], int n_chunks, int n_terms) {
@@ -641,7 +386,7 @@ size_t box_tc_smem(const int dims[3], int n_chunks, int n_terms) {
 size_t cubic_tc_smem(int n, int n_chunks, int n_terms) { return tc_smem_bytes(n, n_chunks, n_terms); }
 
 const SizeOps* box_ops() {
-    static const SizeOps o{0, nullptr, nullptr, false, &box_scan_batch, &box_pencil_smem_unknown, &box_prep,
+    static const SizeOps o{0, false, &box_scan_batch, &box_pencil_smem_unknown, &box_prep,
                            &box_middle, &box_finish, &box_load_kernels};
     return &o;
 }

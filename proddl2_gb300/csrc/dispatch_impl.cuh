@@ -26,73 +26,15 @@ template <int N> struct SizeOpsImpl {
                ((size_t)K * N + 1) * sizeof(int32_t) +
                (size_t)n_ent * sizeof(uint32_t);
     }
-    template <typename T> static size_t line_smem() { return (size_t)(N * 32 + N) * sizeof(cplx_t<T>); }
 
     static cudaError_t set_smem(const void* fn, size_t bytes) {
         if (bytes <= 48 * 1024) return cudaSuccess;
         return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
     }
 
-    template <typename T, int SIGN>
-    static cudaError_t line_fft(cplx_t<T>* data, const cplx_t<T>* tw, long n_lines, long elem_stride,
-                                long inner_count, long inner_stride, long outer_stride, cudaStream_t s) {
-        const size_t sm = line_smem<T>();
-        cudaError_t e = set_smem((const void*)line_fft_kernel<T, N, SIGN>, sm);
-        if (e != cudaSuccess) return e;
-        const long blocks = (n_lines + 31) / 32;
-        line_fft_kernel<T, N, SIGN><<<(unsigned)blocks, 32 * G, sm, s>>>(data, tw, n_lines, elem_stride,
-                                                                        inner_count, inner_stride, outer_stride);
-        return cudaGetLastError();
-    }
-
     // the tensor pencil stage: one 128-row x tile up to 128, two up to 256
     static constexpr bool kHasTc = N <= 256;
 
-
-    static cudaError_t circ_scales(const float2* circ, int K, int8_t* cscale, cudaStream_t s) {
-        if constexpr (kHasTc) {
-            const int nh = N * H;
-            circ_scale_kernel<N><<<(nh + 127) / 128, 128, 0, s>>>(circ, K, cscale);
-            return cudaGetLastError();
-        } else {
-            return cudaErrorNotSupported;
-        }
-    }
-
-    static cudaError_t receptor_fft(const double* rgrid_t, double2* cbuf, double2* hbuf, const double2* tw64,
-                                    void* spec_t, int spec_bf16, int PP, float2* circ_t, cudaStream_t s) {
-        const size_t V = (size_t)N * N * N;
-        complexify_kernel<<<(unsigned)((V + 255) / 256), 256, 0, s>>>(rgrid_t, cbuf, V);
-        cudaError_t e = cudaGetLastError();
-        if (e != cudaSuccess) return e;
-        // z: lines (x, y), contiguous elements
-        e = line_fft<double, -1>(cbuf, tw64, (long)N * N, 1, N, N, (long)N * N, s);
-        if (e != cudaSuccess) return e;
-        const size_t NHt = (size_t)N * N * H;
-        half_extract_kernel<<<(unsigned)((NHt + 255) / 256), 256, 0, s>>>(cbuf, hbuf, N, H);
-        if ((e = cudaGetLastError()) != cudaSuccess) return e;
-        // y: lines (x, kz) of [N][N][H]
-        e = line_fft<double, -1>(hbuf, tw64, (long)N * H, H, H, 1, (long)N * H, s);
-        if (e != cudaSuccess) return e;
-        if (circ_t) {
-            // receptor transformed along z and y only: circulant samples of the tensor path
-            const size_t tot = (size_t)N * N * H;
-            pack_circ_kernel<<<(unsigned)((tot + 255) / 256), 256, 0, s>>>(hbuf, circ_t, N, N * H,
-                                                                         1.0 / ((double)N * N));
-            if ((e = cudaGetLastError()) != cudaSuccess) return e;
-        }
-        // x: lines p = (ky, kz)
-        e = line_fft<double, -1>(hbuf, tw64, (long)N * H, (long)N * H, (long)N * H, 1, 0, s);
-        if (e != cudaSuccess) return e;
-        const size_t tot = (size_t)N * PP;
-        if (spec_bf16)
-            pack_spectrum_kernel<<<(unsigned)((tot + 255) / 256), 256, 0, s>>>(
-                hbuf, static_cast<__nv_bfloat162*>(spec_t), N, N * H, PP, 1.0 / (double)V);
-        else
-            pack_spectrum_kernel<<<(unsigned)((tot + 255) / 256), 256, 0, s>>>(
-                hbuf, static_cast<float2*>(spec_t), N, N * H, PP, 1.0 / (double)V);
-        return cudaGetLastError();
-    }
 
     template <typename SpecT> static cudaError_t launch_pencil(const BatchArgs& a, int nb, cudaStream_t s) {
         const size_t sm2 = pencil_smem(a.K, a.n_ent);
@@ -237,7 +179,7 @@ template <int N> struct SizeOpsImpl {
     }
 
     static const SizeOps* ops() {
-        static const SizeOps o{N, &receptor_fft, &circ_scales, kHasTc, &scan_batch, &pencil_smem, &prep, &middle,
+        static const SizeOps o{N, kHasTc, &scan_batch, &pencil_smem, &prep, &middle,
                                &finish, &load_fft_form};
         return &o;
     }

@@ -113,6 +113,19 @@ struct fftdock_ctx {
     // queue + clustering path (cfg.cluster_trans)
     fftdock::WideArgs wide{};
 
+    // work of the receptor set-up, grown on demand and kept for the next pair
+    template <typename T> struct Grown {
+        T* p = nullptr;
+        size_t cap = 0;
+    };
+    struct RecWork {
+        Grown<double> xyz, lj;
+        Grown<int32_t> type;
+        Grown<int> flags, bin_start, bin_atoms, cmax;
+        Grown<fftdock::AtomCell> cells;
+        Grown<double2> half;
+    } rec;
+
     // kernel timing (fftdock_profile): event pool and (stage, from, to)
     // records of pool indices
     bool profiling = false;
@@ -151,6 +164,15 @@ template <typename T> cudaError_t dalloc(T** p, size_t n) {
 template <typename T> void dfree(T*& p) {
     if (p) cudaFree(p);
     p = nullptr;
+}
+
+template <typename T> cudaError_t grow(fftdock_ctx::Grown<T>& g, size_t n) {
+    if (n <= g.cap && g.p) return cudaSuccess;
+    dfree(g.p);
+    g.cap = 0;
+    cudaError_t e = dalloc(&g.p, n);
+    if (e == cudaSuccess) g.cap = n;
+    return e;
 }
 
 bool finite3(const double* p, int n) {
@@ -336,6 +358,27 @@ int run_batches(fftdock_ctx* ctx, int n_rot, const double* rot, int first_id, ff
         }
     }
     return FFTDOCK_OK;
+}
+
+// transforms of the K term grids in ctx->rgrid (work: ctx->rec.half, .cmax)
+cudaError_t receptor_transforms(fftdock_ctx* ctx, cudaStream_t s) {
+    cudaError_t e = grow(ctx->rec.half, fftdock::receptor_fft_work(ctx->dims, ctx->K) / sizeof(double2));
+    if (e == cudaSuccess) e = grow(ctx->rec.cmax, (size_t)ctx->dims[1] * ctx->H);
+    if (e != cudaSuccess) return e;
+    fftdock::ReceptorFftArgs f{};
+    for (int d = 0; d < 3; ++d) f.dims[d] = ctx->dims[d];
+    f.K = ctx->K;
+    f.rgrid = ctx->rgrid;
+    f.half = ctx->rec.half.p;
+    f.tw64 = ctx->box ? ctx->btw64 : ctx->tw64;
+    f.shared_tw = !ctx->box;
+    f.spec = ctx->spec;
+    f.spec_bf16 = ctx->cfg.precision == FFTDOCK_PREC_BF16_SPECTRA ? 1 : 0;
+    f.pp = ctx->PP;
+    f.circ = ctx->use_tc ? ctx->circ : nullptr;
+    f.cmax = ctx->rec.cmax.p;
+    f.cscale = ctx->cscale;
+    return fftdock::receptor_fft(f, s);
 }
 
 int check_ready(fftdock_ctx* ctx) {
@@ -526,8 +569,7 @@ int fftdock_supported_dims(int32_t nx, int32_t ny, int32_t nz) {
     if (nx == ny && ny == nz && fftdock::size_ops(nx)) return 1;
     const int n[3] = {nx, ny, nz};
     for (int d = 0; d < 3; ++d) {
-        fftdock::BoxPlan pl;
-        if (n[d] < fftdock::kBoxMin || n[d] > fftdock::kBoxMax || !fftdock::box_plan(n[d], &pl)) return 0;
+        if (n[d] < fftdock::kBoxMin || n[d] > fftdock::kBoxMax || !fftdock::box_size(n[d])) return 0;
     }
     return 1;
 }
@@ -578,6 +620,15 @@ void fftdock_destroy(fftdock_ctx* ctx) {
     dfree(ctx->tinfo);
     dfree(ctx->tpad);
     dfree(ctx->err_dev);
+    dfree(ctx->rec.xyz.p);
+    dfree(ctx->rec.lj.p);
+    dfree(ctx->rec.type.p);
+    dfree(ctx->rec.flags.p);
+    dfree(ctx->rec.bin_start.p);
+    dfree(ctx->rec.bin_atoms.p);
+    dfree(ctx->rec.cmax.p);
+    dfree(ctx->rec.cells.p);
+    dfree(ctx->rec.half.p);
     dfree(ctx->wide.corr);
     dfree(ctx->wide.hist);
     dfree(ctx->wide.st);
@@ -823,73 +874,47 @@ int fftdock_set_receptor(fftdock_ctx* ctx, int32_t n, const double* xyz, const i
     fftdock::DeviceScope dev_scope(c.device);
     CK(dev_scope.status());
     ctx->have_rec = false;
-    const int N = ctx->N;
-    const size_t V = ctx->V;
     cudaStream_t s = ctx->stream;
-    const fftdock::Geo g = ctx->geo;
-    double* d_xyz = nullptr;
-    int32_t* d_type = nullptr;
-    int* flags = nullptr;
-    double* dens = nullptr;
-    double2* cbuf = nullptr;
-    double2* hbuf = nullptr;
-    int* bin_start = nullptr;
-    int* bin_atoms = nullptr;
-    int* box = nullptr;
-    int rc = FFTDOCK_OK;
-    auto cleanup = [&]() {
-        cudaStreamSynchronize(s);
-        dfree(d_xyz);
-        dfree(d_type);
-        dfree(flags);
-        dfree(dens);
-        dfree(cbuf);
-        dfree(hbuf);
-        dfree(bin_start);
-        dfree(bin_atoms);
-        dfree(box);
+    fftdock_ctx::RecWork& w = ctx->rec;
+    // a failed call leaves work queued on the context's stream: wait for it,
+    // since it may read the caller's arrays and the host bins below
+    struct Drain {
+        cudaStream_t s;
+        ~Drain() { cudaStreamSynchronize(s); }
     };
-#define CKR(expr)                                 \
-    do {                                          \
-        cudaError_t e_ = (expr);                  \
-        if (e_ != cudaSuccess) {                  \
-            rc = cuda_fail(ctx, e_, #expr);       \
-            cleanup();                            \
-            return rc;                            \
-        }                                         \
-    } while (0)
-    CKR(dalloc(&d_xyz, (size_t)n * 3));
-    CKR(dalloc(&d_type, (size_t)n));
-    CKR(dalloc(&flags, V));
-    if (n > 0) {
-        CKR(cudaMemcpyAsync(d_xyz, xyz, (size_t)n * 3 * sizeof(double), cudaMemcpyHostToDevice, s));
-        if (ace) CKR(cudaMemcpyAsync(d_type, type, (size_t)n * sizeof(int32_t), cudaMemcpyHostToDevice, s));
-    }
     fftdock::HostAtomBins hb;
+    Drain drain{s};
+    CK(grow(w.xyz, (size_t)n * 3));
+    CK(grow(w.type, (size_t)n));
+    CK(grow(w.flags, ctx->V));
+    if (n > 0) {
+        CK(cudaMemcpyAsync(w.xyz.p, xyz, (size_t)n * 3 * sizeof(double), cudaMemcpyHostToDevice, s));
+        if (ace) CK(cudaMemcpyAsync(w.type.p, type, (size_t)n * sizeof(int32_t), cudaMemcpyHostToDevice, s));
+    }
     if (ace) {
-        CKR(dalloc(&dens, (size_t)c.n_types * V));
         fftdock::bin_atoms(xyz, n, c.ace_cut, hb);
-        CKR(dalloc(&bin_start, hb.start.size()));
-        CKR(dalloc(&bin_atoms, hb.atoms.size()));
-        CKR(dalloc(&box, (size_t)6 * n));
-        CKR(cudaMemcpyAsync(bin_start, hb.start.data(), hb.start.size() * sizeof(int), cudaMemcpyHostToDevice, s));
+        CK(grow(w.bin_start, hb.start.size()));
+        CK(grow(w.bin_atoms, hb.atoms.size()));
+        CK(grow(w.cells, (size_t)n));
+        CK(cudaMemcpyAsync(w.bin_start.p, hb.start.data(), hb.start.size() * sizeof(int), cudaMemcpyHostToDevice, s));
         if (n > 0)
-            CKR(cudaMemcpyAsync(bin_atoms, hb.atoms.data(), hb.atoms.size() * sizeof(int), cudaMemcpyHostToDevice, s));
+            CK(cudaMemcpyAsync(w.bin_atoms.p, hb.atoms.data(), hb.atoms.size() * sizeof(int), cudaMemcpyHostToDevice,
+                               s));
     }
     {
         fftdock::ReceptorGridArgs ra{};
-        ra.xyz = d_xyz;
-        ra.type = d_type;
+        ra.xyz = w.xyz.p;
+        ra.type = w.type.p;
         ra.n = n;
         for (int d = 0; d < 3; ++d) {
             ra.bins.lo[d] = hb.lo[d];
             ra.bins.nb[d] = hb.nb[d];
         }
         ra.bins.size = hb.size;
-        ra.bins.start = bin_start;
-        ra.bins.atoms = bin_atoms;
-        ra.box = box;
-        ra.geo = g;
+        ra.bins.start = w.bin_start.p;
+        ra.bins.atoms = w.bin_atoms.p;
+        ra.cells = w.cells.p;
+        ra.geo = ctx->geo;
         ra.term_set = c.term_set;
         ra.n_types = c.n_types;
         ra.K = ctx->K;
@@ -900,34 +925,12 @@ int fftdock_set_receptor(fftdock_ctx* ctx, int32_t n, const double* xyz, const i
         ra.ace_a = c.ace_a;
         ra.ace_cut = c.ace_cut;
         ra.emat = ctx->emat;
-        ra.flags = flags;
-        ra.dens = dens;
+        ra.flags = w.flags.p;
         ra.rgrid = ctx->rgrid;
-        CKR(fftdock::build_receptor_grids(ra, s));
+        CK(fftdock::build_receptor_grids(ra, s));
     }
-    CKR(dalloc(&cbuf, V));
-    CKR(dalloc(&hbuf, (size_t)ctx->dims[0] * ctx->dims[1] * ctx->H));
-    for (int t = 0; t < ctx->K; ++t) {
-        const size_t elem = c.precision == FFTDOCK_PREC_BF16_SPECTRA ? 4 : 8;
-        void* spec_t = static_cast<unsigned char*>(ctx->spec) + (size_t)t * N * ctx->PP * elem;
-        // the tensor stage's circulant samples of term t: [pencils][Nx]
-        float2* circ_t = ctx->use_tc ? ctx->circ + (size_t)t * ctx->dims[1] * ctx->H * ctx->dims[0] : nullptr;
-        if (ctx->box)
-            CKR(fftdock::box_receptor_fft(ctx->rgrid + (size_t)t * V, cbuf, hbuf, ctx->btw64, ctx->dims, spec_t,
-                                          ctx->PP, circ_t, s));
-        else
-            CKR(ctx->ops->receptor_fft(ctx->rgrid + (size_t)t * V, cbuf, hbuf, ctx->tw64, spec_t,
-                                       c.precision == FFTDOCK_PREC_BF16_SPECTRA ? 1 : 0, ctx->PP, circ_t, s));
-    }
-    if (ctx->use_tc) {
-        if (ctx->box)
-            CKR(fftdock::box_circ_scales(ctx->circ, ctx->K, ctx->dims[1] * ctx->H, ctx->dims[0], ctx->cscale, s));
-        else
-            CKR(ctx->ops->circ_scales(ctx->circ, ctx->K, ctx->cscale, s));
-    }
-    CKR(cudaStreamSynchronize(s));
-    cleanup();
-#undef CKR
+    CK(receptor_transforms(ctx, s));
+    CK(cudaStreamSynchronize(s));
     ctx->have_rec = true;
     return FFTDOCK_OK;
 }
@@ -1083,51 +1086,29 @@ int fftdock_set_pair_lj(fftdock_ctx* ctx, int32_t n_rec, const double* rec_xyz, 
     ctx->have_rec = ctx->have_lig = false;
     CK(cudaStreamSynchronize(ctx->stream));
     const int N = ctx->N;
-    const size_t V = ctx->V;
     cudaStream_t s = ctx->stream;
-    double* d_xyz = nullptr;
-    double* d_lc = nullptr;
-    int* bin_start = nullptr;
-    int* bin_atoms = nullptr;
-    int* box = nullptr;
-    double2* cbuf = nullptr;
-    double2* hbuf = nullptr;
-    int rc = FFTDOCK_OK;
-    auto cleanup = [&]() {
-        cudaStreamSynchronize(s);
-        dfree(d_xyz);
-        dfree(d_lc);
-        dfree(bin_start);
-        dfree(bin_atoms);
-        dfree(box);
-        dfree(cbuf);
-        dfree(hbuf);
+    fftdock_ctx::RecWork& w = ctx->rec;
+    struct Drain {
+        cudaStream_t s;
+        ~Drain() { cudaStreamSynchronize(s); }
     };
-#define CKR(expr)                                 \
-    do {                                          \
-        cudaError_t e_ = (expr);                  \
-        if (e_ != cudaSuccess) {                  \
-            rc = cuda_fail(ctx, e_, #expr);       \
-            cleanup();                            \
-            return rc;                            \
-        }                                         \
-    } while (0)
     fftdock::HostAtomBins hb;
+    Drain drain{s};
     fftdock::bin_atoms(rec_xyz, n_rec, cut, hb);
-    CKR(dalloc(&d_xyz, (size_t)n_rec * 3));
-    CKR(dalloc(&d_lc, lc.size()));
-    CKR(dalloc(&bin_start, hb.start.size()));
-    CKR(dalloc(&bin_atoms, hb.atoms.size()));
-    CKR(dalloc(&box, (size_t)6 * n_rec));
-    CKR(cudaMemcpyAsync(bin_start, hb.start.data(), hb.start.size() * sizeof(int), cudaMemcpyHostToDevice, s));
+    CK(grow(w.xyz, (size_t)n_rec * 3));
+    CK(grow(w.lj, lc.size()));
+    CK(grow(w.bin_start, hb.start.size()));
+    CK(grow(w.bin_atoms, hb.atoms.size()));
+    CK(grow(w.cells, (size_t)n_rec));
+    CK(cudaMemcpyAsync(w.bin_start.p, hb.start.data(), hb.start.size() * sizeof(int), cudaMemcpyHostToDevice, s));
     if (n_rec > 0) {
-        CKR(cudaMemcpyAsync(d_xyz, rec_xyz, (size_t)n_rec * 3 * sizeof(double), cudaMemcpyHostToDevice, s));
-        CKR(cudaMemcpyAsync(d_lc, lc.data(), lc.size() * sizeof(double), cudaMemcpyHostToDevice, s));
-        CKR(cudaMemcpyAsync(bin_atoms, hb.atoms.data(), hb.atoms.size() * sizeof(int), cudaMemcpyHostToDevice, s));
+        CK(cudaMemcpyAsync(w.xyz.p, rec_xyz, (size_t)n_rec * 3 * sizeof(double), cudaMemcpyHostToDevice, s));
+        CK(cudaMemcpyAsync(w.lj.p, lc.data(), lc.size() * sizeof(double), cudaMemcpyHostToDevice, s));
+        CK(cudaMemcpyAsync(w.bin_atoms.p, hb.atoms.data(), hb.atoms.size() * sizeof(int), cudaMemcpyHostToDevice, s));
     }
     {
         fftdock::ReceptorGridArgs ra{};
-        ra.xyz = d_xyz;
+        ra.xyz = w.xyz.p;
         ra.n = n_rec;
         ra.geo = ctx->geo;
         ra.term_set = c.term_set;
@@ -1137,28 +1118,16 @@ int fftdock_set_pair_lj(fftdock_ctx* ctx, int32_t n_rec, const double* rec_xyz, 
             ra.bins.nb[d] = hb.nb[d];
         }
         ra.bins.size = hb.size;
-        ra.bins.start = bin_start;
-        ra.bins.atoms = bin_atoms;
-        ra.box = box;
-        ra.lj_c = d_lc;
+        ra.bins.start = w.bin_start.p;
+        ra.bins.atoms = w.bin_atoms.p;
+        ra.cells = w.cells.p;
+        ra.lj_c = w.lj.p;
         ra.lj_cut = cut;
         ra.rgrid = ctx->rgrid;
-        CKR(fftdock::build_receptor_grids(ra, s));
+        CK(fftdock::build_receptor_grids(ra, s));
     }
-    CKR(dalloc(&cbuf, V));
-    CKR(dalloc(&hbuf, (size_t)ctx->dims[0] * ctx->dims[1] * ctx->H));
-    for (int t = 0; t < ctx->K; ++t) {
-        void* spec_t = static_cast<unsigned char*>(ctx->spec) + (size_t)t * N * ctx->PP * 8;
-        if (ctx->box)
-            CKR(fftdock::box_receptor_fft(ctx->rgrid + (size_t)t * V, cbuf, hbuf, ctx->btw64, ctx->dims, spec_t,
-                                          ctx->PP, nullptr, s));
-        else
-            CKR(ctx->ops->receptor_fft(ctx->rgrid + (size_t)t * V, cbuf, hbuf, ctx->tw64, spec_t, 0, ctx->PP,
-                                       nullptr, s));
-    }
-    CKR(cudaStreamSynchronize(s));
-    cleanup();
-#undef CKR
+    CK(receptor_transforms(ctx, s));
+    CK(cudaStreamSynchronize(s));
 
     // ligand entries: one per (atom, term); ljComp weighs each atom into both
     // terms, ljAvg has unit weights (the unweighted path)

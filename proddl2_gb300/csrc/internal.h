@@ -79,12 +79,20 @@ struct HostAtomBins {
 };
 void bin_atoms(const double* xyz, int n, double cut, HostAtomBins& out);
 
+// what the gather of the radial fields reads of an atom
+struct __align__(16) AtomCell {
+    float x, y, z;   // rounded coordinates
+    int type;
+    int lo[3], hi[3];  // cropped projection box
+    int pad[2];
+};
+
 struct ReceptorGridArgs {
     const double* xyz;     // [n][3]
     const int32_t* type;   // [n]
     int n;
     AtomBins bins;         // shape+ACE and LJ: cell list of the atoms (device arrays)
-    int* box;              // shape+ACE and LJ: [n][6] work (each atom's projection box)
+    AtomCell* cells;       // shape+ACE and LJ: [n] work
     const double* lj_c;    // LJ: [n][5] per-atom field constants (as6, 4es6, 4es12, fshift, gshift)
     double lj_cut;         // LJ: field cutoff
     Geo geo;
@@ -95,11 +103,28 @@ struct ReceptorGridArgs {
     double ace_b, ace_k, ace_a, ace_cut;
     const double* emat;    // [n_types][n_types]
     int* flags;            // [N^3] work
-    double* dens;          // [n_types][N^3] work (shape+ACE)
     double* rgrid;         // [K][N^3] out
 };
 
 cudaError_t build_receptor_grids(const ReceptorGridArgs& a, cudaStream_t s);
+
+// the transforms of all K term grids (receptor_fft.cu)
+struct ReceptorFftArgs {
+    int dims[3];
+    int K;
+    const double* rgrid;   // [K][V]
+    double2* half;         // [K][Nx][Ny][Hz] work (receptor_fft_work bytes)
+    const double2* tw64;   // e^{-2 pi i m / n}: [Nx | Ny | Nz], or one table of a cubic edge (shared_tw)
+    bool shared_tw;
+    void* spec;            // [K][Nx][pp] out, scaled 1 / V
+    int spec_bf16;
+    int pp;
+    float2* circ;          // tensor form (or null): [K][Ny Hz][Nx] out
+    int* cmax;             // tensor form: [Ny Hz] work
+    int8_t* cscale;        // tensor form: [Ny Hz] out
+};
+size_t receptor_fft_work(const int dims[3], int K);
+cudaError_t receptor_fft(const ReceptorFftArgs& a, cudaStream_t s);
 
 // Exact per-rotation queue of up to kWideMax entries ("maxNTransInp") and
 // the translational clustering applied to it (TranClust,
@@ -147,14 +172,6 @@ struct WideArgs {
     double rad2;               // squared neighbour radius of the clustering
 };
 
-// Mixed-radix plan of one transform length of the box-grid path: radices in
-// Stockham stage order (4, 2, 3, 5, 7, 11, 13).
-constexpr int kBoxMaxFactors = 12;
-struct BoxPlan {
-    int n;
-    int nf;
-    int f[kBoxMaxFactors];
-};
 // Box-grid sizes each axis may take: [kBoxMin, kBoxMax], factors 2..13.
 constexpr int kBoxMin = 8;
 constexpr int kBoxMax = 256;
@@ -255,11 +272,6 @@ cudaError_t wide_select_batch(const BatchArgs& a, int N, cudaStream_t s);
 
 struct SizeOps {
     int n;
-    // forward 3-D FFT of one real FP64 term grid into spec_t ([N][PP], scaled 1/V)
-    cudaError_t (*receptor_fft)(const double* rgrid_t, double2* cbuf, double2* hbuf, const double2* tw64,
-                                void* spec_t, int spec_bf16, int PP, float2* circ_t, cudaStream_t s);
-    // per-pencil scale exponents of the circulant samples (tensor path)
-    cudaError_t (*circ_scales)(const float2* circ, int K, int8_t* cscale, cudaStream_t s);
     bool has_tc;
     cudaError_t (*scan_batch)(const BatchArgs& a, cudaStream_t s);
     // shared-memory bytes of the pencil kernel for (K, n_ent)
@@ -280,17 +292,9 @@ const SizeOps* size_ops(int n);
 // Box grids (box_grid.cu): sizes per axis, any length of factors 2..13 in
 // [kBoxMin, kBoxMax]; the pipeline's stages read the sizes from BatchArgs.box.
 const SizeOps* box_ops();
-bool box_plan(int n, BoxPlan* pl);
+bool box_size(int n);  // a product of 2, 3, 5, 7, 11 and 13
 // largest dynamic shared memory of the box-grid kernels for a ligand
 size_t box_pencil_smem(int nx, int ny, int nz, int K, int n_ent, bool weighted);
-// forward transform of one real FP64 term grid into spec_t ([Nx][PP] float2,
-// scaled 1/V); tw64 = the FP64 twiddle tables [Nx | Ny | Nz]; circ_t (tensor
-// form): the term's circulant samples [Ny Hz][Nx] (the grid transformed
-// along z and y only, conjugated, / (Ny Nz))
-cudaError_t box_receptor_fft(const double* rgrid_t, double2* cbuf, double2* hbuf, const double2* tw64,
-                             const int dims[3], void* spec_t, int PP, float2* circ_t, cudaStream_t s);
-// per-pencil scale exponents of the box grid's circulant samples
-cudaError_t box_circ_scales(const float2* circ, int K, int nh, int nx, int8_t* cscale, cudaStream_t s);
 // dynamic shared memory of the tensor pencil stage on a box grid, and on a
 // cubic grid of edge n
 size_t box_tc_smem(const int dims[3], int n_chunks, int n_terms);

@@ -81,16 +81,15 @@ struct Work {
     double* rgrid = nullptr;
     void* spec = nullptr;
     int* flags = nullptr;
-    double* dens = nullptr;
-    double2* cbuf = nullptr;
-    double2* hbuf = nullptr;
+    double2* half = nullptr;    // all terms' half spectra during the set-up
+    int* cmax = nullptr;
     uint32_t* ent = nullptr;
     int32_t* offs = nullptr;
     float2* g2 = nullptr;
     float* cand_v = nullptr;
     int32_t* cand_i = nullptr;
     int* err = nullptr;
-    int* box = nullptr;
+    fftdock::AtomCell* cells = nullptr;
     // tensor form
     float2* circ = nullptr;
     int8_t* cscale = nullptr;
@@ -101,14 +100,13 @@ struct Work {
         dfree(cscale);
         dfree(ent_t);
         dfree(g2t);
-        dfree(box);
+        dfree(cells);
+        dfree(cmax);
         dfree(rgrid);
         if (spec) cudaFree(spec);
         spec = nullptr;
         dfree(flags);
-        dfree(dens);
-        dfree(cbuf);
-        dfree(hbuf);
+        dfree(half);
         dfree(ent);
         dfree(offs);
         dfree(g2);
@@ -130,7 +128,6 @@ struct Staged {
     double* emat = nullptr;
     int* bin_start = nullptr;   // all pairs' cell lists, concatenated
     int* bin_atoms = nullptr;
-    int* box = nullptr;         // [sum n_rec][6]
     std::vector<size_t> rec_off, lig_off, rot_off, bin_off;
     std::vector<fftdock::HostAtomBins> bins;
     // tensor form: per pair its window and entry tables (concatenated on the device)
@@ -143,7 +140,6 @@ struct Staged {
         dfree(tpad);
         dfree(bin_start);
         dfree(bin_atoms);
-        dfree(box);
         dfree(rec_xyz);
         dfree(rec_type);
         dfree(lig_xyz);
@@ -206,11 +202,10 @@ int alloc_work(Run& r, Work& w, const SizeData& sd, int B) {
     }
     PCK(dalloc(&w.flags, V));
     if (r.ace) {
-        PCK(dalloc(&w.dens, (size_t)r.cfg.n_types * V));
-        PCK(dalloc(&w.box, (size_t)6 * sd.max_rec));
+        PCK(dalloc(&w.cells, (size_t)sd.max_rec));
     }
-    PCK(dalloc(&w.cbuf, V));
-    PCK(dalloc(&w.hbuf, (size_t)N * N * sd.H));
+    const int dims[3] = {N, N, N};
+    PCK(dalloc(&w.half, fftdock::receptor_fft_work(dims, K) / sizeof(double2)));
     PCK(dalloc(&w.ent, (size_t)B * sd.max_lig));
     PCK(dalloc(&w.offs, (size_t)B * (K * N * fftdock::cubic_pencil_classes(K, false) + 1)));
     PCK(dalloc(&w.g2, (size_t)B * N * sd.PP));
@@ -222,6 +217,7 @@ int alloc_work(Run& r, Work& w, const SizeData& sd, int B) {
         const size_t nh = (size_t)N * sd.H;
         PCK(dalloc(&w.circ, (size_t)K * nh * N));
         PCK(dalloc(&w.cscale, nh));
+        PCK(dalloc(&w.cmax, nh));
         PCK(dalloc(&w.g2t, (size_t)B * nh * N));
         // 16 spare rows of 128: the tensor stage's loads run up to 16 rows past a range
         PCK(dalloc(&w.ent_t, (size_t)B * sd.max_pad + 16 * fftdock::kTcRot));
@@ -260,25 +256,29 @@ cudaError_t enqueue_pair(Run& r, const fftdock_pair& p, int i, Work& w, const Si
         ra.bins.size = hb.size;
         ra.bins.start = r.st.bin_start + r.st.bin_off[i];
         ra.bins.atoms = r.st.bin_atoms + r.st.rec_off[i];
-        ra.box = w.box;
+        ra.cells = w.cells;
     }
     ra.flags = w.flags;
-    ra.dens = w.dens;
     ra.rgrid = w.rgrid;
     cudaError_t e = fftdock::build_receptor_grids(ra, s);
     if (e != cudaSuccess) return e;
     const bool bf = c.precision == FFTDOCK_PREC_BF16_SPECTRA;
-    const size_t elem = bf ? 4 : 8;
     const bool tc = sd.tc && r.st.tct[i].ok;
-    const size_t nh = (size_t)N * sd.H;
-    for (int t = 0; t < r.K; ++t) {
-        e = sd.ops->receptor_fft(w.rgrid + (size_t)t * sd.V, w.cbuf, w.hbuf, sd.tw64,
-                                 static_cast<unsigned char*>(w.spec) + (size_t)t * N * sd.PP * elem, bf ? 1 : 0,
-                                 sd.PP, tc ? w.circ + (size_t)t * nh * N : nullptr, s);
-        if (e != cudaSuccess) return e;
-    }
+    fftdock::ReceptorFftArgs f{};
+    f.dims[0] = f.dims[1] = f.dims[2] = N;
+    f.K = r.K;
+    f.rgrid = w.rgrid;
+    f.half = w.half;
+    f.tw64 = sd.tw64;
+    f.shared_tw = true;
+    f.spec = w.spec;
+    f.spec_bf16 = bf ? 1 : 0;
+    f.pp = sd.PP;
+    f.circ = tc ? w.circ : nullptr;
+    f.cmax = w.cmax;
+    f.cscale = w.cscale;
+    if ((e = fftdock::receptor_fft(f, s)) != cudaSuccess) return e;
     if (tc) {
-        if ((e = sd.ops->circ_scales(w.circ, r.K, w.cscale, s)) != cudaSuccess) return e;
         const fftdock::TcTables& tt = r.st.tct[i];
         // this pair's padding rows (x' = its window width) over the rows its batches use
         e = fftdock::fill_padding(w.ent_t, tt.W, (size_t)B * tt.n_pad + 16 * fftdock::kTcRot, s);

@@ -602,60 +602,4 @@ __global__ void __launch_bounds__(TC_THREADS, MT == 1 ? 2 : 1) pencil_tc_kernel(
     if (warp == 0) tc::tmem_dealloc(tmem, TM_COLS);
 }
 
-// per-pencil power-of-two exponent so that the largest circulant component
-// of the pencil (over all terms) scales to about 2^13
-template <int N>
-__global__ void circ_scale_kernel(const float2* __restrict__ circ, int K, int8_t* __restrict__ cscale) {
-    constexpr int NH = N * (N / 2 + 1);
-    const int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= NH) return;
-    float m = 0.f;
-    for (int t = 0; t < K; ++t)
-        for (int d = 0; d < N; ++d) {
-            const float2 c = circ[((size_t)t * NH + p) * N + d];
-            m = fmaxf(m, fmaxf(fabsf(c.x), fabsf(c.y)));
-        }
-    int e = 0;
-    if (m > 0.f) {
-        int ex;
-        frexpf(m, &ex);  // m in [2^(ex-1), 2^ex)
-        e = 13 - ex;
-    }
-    e = e < -100 ? -100 : (e > 100 ? 100 : e);
-    cscale[p] = (int8_t)e;
-}
-
-// box grids: the same per pencil p < nh over samples d < nx
-static __global__ void circ_scale_box_kernel(const float2* __restrict__ circ, int K, int nh, int nx,
-                                      int8_t* __restrict__ cscale) {
-    const int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= nh) return;
-    float m = 0.f;
-    for (int t = 0; t < K; ++t)
-        for (int d = 0; d < nx; ++d) {
-            const float2 c = circ[((size_t)t * nh + p) * nx + d];
-            m = fmaxf(m, fmaxf(fabsf(c.x), fabsf(c.y)));
-        }
-    int e = 0;
-    if (m > 0.f) {
-        int ex;
-        frexpf(m, &ex);
-        e = 13 - ex;
-    }
-    e = e < -100 ? -100 : (e > 100 ? 100 : e);
-    cscale[p] = (int8_t)e;
-}
-
-// circ[t][p][d] = conj(R2_t(d, p)) / N^2 from the y/z-transformed half grid [N][N*H]
-static __global__ void pack_circ_kernel(const double2* __restrict__ half, float2* __restrict__ circ_t, int n, int nh,
-                                        double scale) {
-    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const size_t tot = (size_t)n * nh;
-    if (i >= tot) return;
-    const size_t p = i / n;
-    const int d = (int)(i - p * n);
-    const double2 v = half[(size_t)d * nh + p];
-    circ_t[i] = make_float2((float)(v.x * scale), (float)(-v.y * scale));
-}
-
 }  // namespace fftdock

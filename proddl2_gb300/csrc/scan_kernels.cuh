@@ -495,75 +495,7 @@ __global__ void __launch_bounds__(256) finalize_kernel(
     }
 }
 
-// generic batched line transform: line L -> base (L / inner_count) *
-// outer_stride + (L % inner_count) * inner_stride, element e at base +
-// e * elem_stride.  In place.  CTA = G warps x 32 lines.
-template <typename T, int N, int SIGN>
-__global__ void __launch_bounds__(32 * SizeTraits<N>::G) line_fft_kernel(
-    cplx_t<T>* __restrict__ data, const cplx_t<T>* __restrict__ tw, long n_lines, long elem_stride, long inner_count,
-    long inner_stride, long outer_stride) {
-    using C = cplx_t<T>;
-    using P = LinePlan<N, SizeTraits<N>::G>;
-    constexpr int G = P::G, R1 = P::R1;
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    C* buf = reinterpret_cast<C*>(smem_raw);  // [N][32]
-    C* tws = buf + N * 32;                    // [N]
-    const int tid = threadIdx.x, w = tid >> 5, l = tid & 31;
-    for (int i = tid; i < N; i += blockDim.x) tws[i] = tw[i];
-    const long L = (long)blockIdx.x * 32 + l;
-    const bool valid = L < n_lines;
-    const long base = valid ? (L / inner_count) * outer_stride + (L % inner_count) * inner_stride : 0;
-    C v[R1];
-#pragma unroll
-    for (int r = 0; r < R1; ++r) v[r] = valid ? data[base + (long)(w + G * r) * elem_stride] : cmake<C>(0, 0);
-    dft<R1, SIGN>(v);
-#pragma unroll
-    for (int r = 0; r < R1; ++r) buf[(w * R1 + r) * 32 + l] = v[r];
-    __syncthreads();
-    C out[R1];
-    line_pass2<P, SIGN, 1, 32>(buf, w, l, tws, out);
-    if (valid) {
-#pragma unroll
-        for (int i = 0; i < P::NB; ++i)
-#pragma unroll
-            for (int r = 0; r < G; ++r) data[base + (long)(w + G * i + R1 * r) * elem_stride] = out[i * G + r];
-    }
-}
-
-static __global__ void complexify_kernel(const double* __restrict__ re, double2* __restrict__ out, size_t V) {
-    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < V) out[i] = make_double2(re[i], 0.0);
-}
-
-// [N][N][N] complex -> [N][N][H] (kz < H)
-static __global__ void half_extract_kernel(const double2* __restrict__ full, double2* __restrict__ half, int n, int h2) {
-    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const size_t tot = (size_t)n * n * h2;
-    if (i >= tot) return;
-    const size_t row = i / h2;
-    const int kz = (int)(i - row * h2);
-    half[i] = full[row * n + kz];
-}
-
 __device__ __forceinline__ void spec_store(float2* p, float x, float y) { *p = make_float2(x, y); }
 __device__ __forceinline__ void spec_store(__nv_bfloat162* p, float x, float y) { *p = __floats2bfloat162_rn(x, y); }
-
-// [N][N*H] double -> [N][PP] FP32 or BF16 pairs scaled by 1/V
-template <typename SpecT>
-static __global__ void pack_spectrum_kernel(const double2* __restrict__ half, SpecT* __restrict__ spec, int n, int nh,
-                                     int pp, double scale) {
-    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const size_t tot = (size_t)n * pp;
-    if (i >= tot) return;
-    const size_t kx = i / pp;
-    const int p = (int)(i - kx * pp);
-    float ox = 0.f, oy = 0.f;
-    if (p < nh) {
-        const double2 v = half[kx * nh + p];
-        ox = (float)(v.x * scale);
-        oy = (float)(v.y * scale);
-    }
-    spec_store(spec + i, ox, oy);
-}
 
 }  // namespace fftdock
