@@ -29,6 +29,7 @@
 #include "fft_core.cuh"
 #include "internal.h"
 #include "pencil_tc.cuh"
+#include "pencil_tcp.cuh"
 #include "scan_kernels.cuh"
 
 namespace fftdock {
@@ -49,7 +50,8 @@ __global__ void __launch_bounds__(256) box_prep_kernel(const double* __restrict_
                                                        int32_t* __restrict__ status, const float* __restrict__ w_in,
                                                        uint4* __restrict__ ent4, int32_t* __restrict__ idx_out,
                                                        uint32_t* __restrict__ ent_t, const int32_t* __restrict__ tpad,
-                                                       int n_pad, int x0, int W, int qc) {
+                                                       int n_pad, int x0, int W, int qc, const int32_t* __restrict__ tinfo,
+                                                       int ka) {
     extern __shared__ unsigned char smem_raw[];
     const int nx = geo.n[0], ny = geo.n[1], nz = geo.n[2];
     // bins (t, x, y mod qc), qc = 1 or 2
@@ -108,7 +110,22 @@ __global__ void __launch_bounds__(256) box_prep_kernel(const double* __restrict_
         __syncthreads();
     }
     int32_t* offs = offs_out + (size_t)q * (nbins + 1);
-    for (int i = tid; i <= nbins; i += blockDim.x) offs[i] = cnt[i];
+    if (!ent_t)  // (the tensor form does not read them)
+        for (int i = tid; i <= nbins; i += blockDim.x) offs[i] = cnt[i];
+    // pencil pairs: which staging rows of each term hold an entry, one bit per
+    // row, after the term rows (a quad of rows per term)
+    for (int i = tid; i < 3 * ka; i += blockDim.x) {
+        const int kk = i / 3, word = i - 3 * kk, t = tinfo[ka + 1 + kk];
+        uint32_t m = 0;
+        for (int j = 0; j < 16; ++j) {
+            const int xr = 16 * word + j, c = xr + x0;
+            if (xr < W && c >= 0 && c < nx) {
+                const int b = (t * nx + c) * qc;
+                m |= (uint32_t)(cnt[b + 1] > cnt[b]) << (2 * j) | (uint32_t)(cnt[b + 2] > cnt[b + 1]) << (2 * j + 1);
+            }
+        }
+        ent_t[(((size_t)(q >> 7) * (n_pad >> 2) + (tinfo[ka] >> 2) + kk) * 128 + (q & 127)) * 4 + word] = m;
+    }
     __syncthreads();
     if (tid < 32) {
         uint32_t* ent = ent_out + (size_t)q * n_ent;
@@ -128,9 +145,10 @@ __global__ void __launch_bounds__(256) box_prep_kernel(const double* __restrict_
             // outside the window at the dummy row W), as in ligand_prep_kernel
             if (act && ent_t) {
                 const size_t row = (size_t)(dst + __ldg(tpad + (key >> 24)));
+                uint32_t xr = min(((key >> 16) - (uint32_t)x0) & 255u, (uint32_t)W);
+                if (ka) xr = 2 * xr + (xr < (uint32_t)W ? (key >> 8) & 1u : 0u);
                 ent_t[(((size_t)(q >> 7) * (n_pad >> 2) + (row >> 2)) * 128 + (q & 127)) * 4 + (row & 3)] =
-                    (min(((key >> 16) - (uint32_t)x0) & 255u, (uint32_t)W) << 24) | (((key >> 8) & 255u) << 16) |
-                    (key & 255u);
+                    (xr << 24) | (((key >> 8) & 255u) << 16) | (key & 255u);
             }
             if (act && ent4) {
                 // ljComp: entry i < n_ent / 2 weighs atom i into term 0, entry
@@ -288,7 +306,8 @@ cudaError_t box_prep(const BatchArgs& a, cudaStream_t s) {
     if (e != cudaSuccess) return e;
     box_prep_kernel<<<nb, 256, sm, s>>>(a.rot, a.lig_xyz, a.lig_term, a.n_ent, a.K, a.box, a.ent, a.offs, a.status,
                                         a.lig_w32, a.lig_w32 ? a.ent4 : nullptr, a.ent_idx,
-                                        a.use_tc ? a.ent_t : nullptr, a.tpad, a.n_pad, a.x0, a.W, a.classes());
+                                        a.use_tc ? a.ent_t : nullptr, a.tpad, a.n_pad, a.x0, a.W, a.classes(), a.tinfo,
+                                        a.mask_terms());
     return cudaGetLastError();
 }
 
@@ -310,7 +329,9 @@ cudaError_t box_middle(const BatchArgs& a, cudaStream_t s) {
         dim3 gridt(np, (nb + TC_ROT - 1) / TC_ROT);
         const int tg = a.tc_group > 0 ? a.tc_group : FFTDOCK_TC_TERMS_PER_SUM_DEFAULT;
         const TcBox bx{nx, ny, nz, nz / 2 + 1, np, nxp, twy, twz};
-        if (tc_tiles(nx) == 1) {
+        if (a.tc_pair) {
+            if ((e = launch_pencil_tcp<0>(a, nx, ny, nz, nullptr, bx, s)) != cudaSuccess) return e;
+        } else if (tc_tiles(nx) == 1) {
             if ((e = set_smem((const void*)pencil_tc_kernel<0, 1>, smt)) != cudaSuccess) return e;
             pencil_tc_kernel<0, 1><<<gridt, TC_THREADS, smt, s>>>(a.circ, a.cscale, a.ent_t, a.tinfo, a.n_tc_terms,
                                                                  nullptr, a.g2t, a.n_pad, nb, a.x0, a.W, tg,
@@ -384,6 +405,15 @@ size_t box_tc_smem(const int dims[3], int n_chunks, int n_terms) {
 }
 
 size_t cubic_tc_smem(int n, int n_chunks, int n_terms) { return tc_smem_bytes(n, n_chunks, n_terms); }
+
+// Pencil pairs measured faster than one pencil at a time at every cubic edge from
+// 24 to 128 (figures in pencil_tcp.cuh), so wherever they fit
+bool tc_pairs_fit(const int dims[3], bool box, int K, int n_ent, int n_chunks, int n_terms) {
+    if (dims[0] > TC_ROT || dims[1] % 2 != 0 || n_chunks > TP_MAX_CHUNKS) return false;
+    if (prep_smem_bytes(dims[0], K, n_ent, 2) > kTpMaxSmem) return false;
+    return (box ? tp_smem_box(dims[0], dims[1], dims[2], n_chunks, n_terms, 8)
+                : tp_smem_cubic(dims[0], n_chunks, n_terms)) <= kTpMaxSmem;
+}
 
 const SizeOps* box_ops() {
     static const SizeOps o{0, false, &box_scan_batch, &box_pencil_smem_unknown, &box_prep,

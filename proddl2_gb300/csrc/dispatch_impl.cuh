@@ -5,6 +5,7 @@
 #include "internal.h"
 #include "scan_kernels.cuh"
 #include "pencil_tc.cuh"
+#include "pencil_tcp.cuh"
 #include "pencil_lines.cuh"
 #include "plane_lines.cuh"
 
@@ -81,7 +82,7 @@ template <int N> struct SizeOpsImpl {
         ligand_prep_kernel<N><<<nb, 256, sm1, s>>>(a.rot, a.lig_xyz, a.lig_term, a.n_ent, a.K, geo, a.ent, a.offs,
                                                     a.status, a.lig_w32, a.lig_w32 ? a.ent4 : nullptr, a.ent_idx,
                                                     a.use_tc ? a.ent_t : nullptr, a.tpad, a.n_pad, a.x0,
-                                                    a.W, a.classes());
+                                                    a.W, a.classes(), a.tinfo, a.mask_terms());
         return cudaGetLastError();
     }
 
@@ -91,22 +92,27 @@ template <int N> struct SizeOpsImpl {
     static cudaError_t middle(const BatchArgs& a, cudaStream_t s) {
         const int nb = a.n_rot;
         if (nb <= 0) return cudaSuccess;
-        cudaError_t e;
+        cudaError_t e = cudaSuccess;
         if (a.ev && (e = cudaEventRecord(a.ev[0], s)) != cudaSuccess) return e;
         bool tc = false;
         if constexpr (kHasTc) {
             if (a.use_tc) {
                 tc = true;
-                const size_t smt = tc_smem_bytes(N, a.W / 8, a.n_tc_terms);
                 constexpr int MT = tc_tiles(N);
-                if ((e = set_smem((const void*)pencil_tc_kernel<N, MT>, smt)) != cudaSuccess) return e;
-                dim3 gridt(N * H, (nb + TC_ROT - 1) / TC_ROT);
-                const int tg = a.tc_group > 0 ? a.tc_group : FFTDOCK_TC_TERMS_PER_SUM_DEFAULT;
-                pencil_tc_kernel<N, MT><<<gridt, TC_THREADS, smt, s>>>(a.circ, a.cscale, a.ent_t, a.tinfo,
-                                                                      a.n_tc_terms, a.tw32, a.g2t, a.n_pad, nb, a.x0,
-                                                                      a.W, tg, a.tc_slots, a.tc_n_slots, TcBox{},
-                                                                      a.err);
-                if ((e = cudaGetLastError()) != cudaSuccess) return e;
+                if (MT == 1 && a.tc_pair) {
+                    if constexpr (MT == 1) e = launch_pencil_tcp<N>(a, N, N, N, a.tw32, TcBox{}, s);
+                    if (e != cudaSuccess) return e;
+                } else {
+                    const size_t smt = tc_smem_bytes(N, a.W / 8, a.n_tc_terms);
+                    if ((e = set_smem((const void*)pencil_tc_kernel<N, MT>, smt)) != cudaSuccess) return e;
+                    dim3 gridt(N * H, (nb + TC_ROT - 1) / TC_ROT);
+                    const int tg = a.tc_group > 0 ? a.tc_group : FFTDOCK_TC_TERMS_PER_SUM_DEFAULT;
+                    pencil_tc_kernel<N, MT><<<gridt, TC_THREADS, smt, s>>>(a.circ, a.cscale, a.ent_t, a.tinfo,
+                                                                          a.n_tc_terms, a.tw32, a.g2t, a.n_pad, nb, a.x0,
+                                                                          a.W, tg, a.tc_slots, a.tc_n_slots, TcBox{},
+                                                                          a.err);
+                    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+                }
             }
         }
         if (!tc) {

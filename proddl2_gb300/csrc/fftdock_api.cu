@@ -101,6 +101,7 @@ struct fftdock_ctx {
     int tc_n_slots = 0;
     int* err_dev = nullptr;
     int x0 = 0, W = 0;
+    bool tc_pair = false;        // over pencil pairs
     bool tc_ready = false;       // the ligand fits the tensor stage (window, terms, unweighted)
     uint32_t* ent_t = nullptr;   // [G/128][n_pad][128]
     int32_t* tinfo = nullptr;    // non-empty terms: padded entry starts, then term ids
@@ -238,6 +239,7 @@ BatchArgs batch_args(fftdock_ctx* ctx) {
     a.x0 = ctx->x0;
     a.W = ctx->W;
     a.use_tc = ctx->use_tc && ctx->tc_ready ? 1 : 0;
+    a.tc_pair = a.use_tc && ctx->tc_pair ? 1 : 0;
     a.ent_t = ctx->ent_t;
     a.tinfo = ctx->tinfo;
     a.tpad = ctx->tpad;
@@ -399,8 +401,8 @@ __global__ void fill_u32_kernel(uint32_t* p, uint32_t v, size_t n) {
 }
 }  // namespace
 
-cudaError_t fill_padding(uint32_t* ent_t, int W, size_t n, cudaStream_t s) {
-    fill_u32_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(ent_t, (uint32_t)W << 24, n);
+cudaError_t fill_padding(uint32_t* ent_t, int dummy_row, size_t n, cudaStream_t s) {
+    fill_u32_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(ent_t, (uint32_t)dummy_row << 24, n);
     return cudaGetLastError();
 }
 
@@ -481,6 +483,8 @@ TcTables tc_tables(const double* xyz, const int32_t* term, int n, int K, int N, 
     t.info.insert(t.info.end(), ids.begin(), ids.end());
     t.ok = W / 8 <= kTcMaxChunks && t.ka <= kTcMaxTerms && t.ka >= 1 &&
            cubic_tc_smem(N, W / 8, t.ka) <= kMaxSmem;
+    const int dims[3] = {N, N, N};
+    t.set_pair(t.ok && tc_pairs_fit(dims, false, K, n, W / 8, t.ka));
     return t;
 }
 
@@ -970,6 +974,7 @@ int fftdock_set_ligand(fftdock_ctx* ctx, int32_t n, const double* xyz, const int
     fftdock::TcTables tt = fftdock::tc_tables(xyz, term.data(), n, ctx->K, ctx->N, ctx->h, ctx->zero_h);
     // box grids: the tensor stage's phase tables grow with Ny + Nz
     if (ctx->box && tt.ok && fftdock::box_tc_smem(ctx->dims, tt.W / 8, tt.ka) > fftdock::kMaxSmem) tt.ok = false;
+    if (ctx->box) tt.set_pair(tt.ok && fftdock::tc_pairs_fit(ctx->dims, true, ctx->K, n, tt.W / 8, tt.ka));
     ctx->x0 = tt.x0;
     ctx->W = tt.W;
     ctx->n_ent = n;
@@ -984,7 +989,7 @@ int fftdock_set_ligand(fftdock_ctx* ctx, int32_t n, const double* xyz, const int
         // to 16 rows past a range
         const size_t n_t = (size_t)ctx->G * tt.n_pad + 16 * fftdock::kTcRot;
         CK(dalloc(&ctx->ent_t, n_t));
-        CK(fftdock::fill_padding(ctx->ent_t, tt.W, n_t, ctx->stream));
+        CK(fftdock::fill_padding(ctx->ent_t, tt.dummy_row(), n_t, ctx->stream));
         CK(cudaStreamSynchronize(ctx->stream));
         CK(dalloc(&ctx->tinfo, tt.info.size()));
         CK(dalloc(&ctx->tpad, tt.tpad.size()));
@@ -993,6 +998,7 @@ int fftdock_set_ligand(fftdock_ctx* ctx, int32_t n, const double* xyz, const int
         ctx->n_tc_terms = tt.ka;
         ctx->n_pad = tt.n_pad;
         ctx->tc_ready = true;
+        ctx->tc_pair = tt.pair;
     }
     ctx->have_lig = true;
     return FFTDOCK_OK;

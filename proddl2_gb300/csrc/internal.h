@@ -178,9 +178,11 @@ constexpr int kBoxMax = 256;
 
 // Everything one device batch of rotations needs.
 struct BatchArgs {
-    // classes in effect (the tensor form takes plain (term, x) bins) and the
-    // bin starts of one rotation
-    int classes() const { return use_tc ? 1 : qc; }
+    // classes in effect (the tensor form: y parity for pencil pairs, else
+    // plain (term, x) bins) and the bin starts of one rotation
+    int classes() const { return use_tc ? (tc_pair ? 2 : 1) : qc; }
+    // terms whose occupied staging rows ligand prep marks
+    int mask_terms() const { return use_tc && tc_pair ? n_tc_terms : 0; }
     size_t offs_stride(int nx) const { return (size_t)K * nx * classes() + 1; }
     // inputs
     const double* rot;          // [B][9]
@@ -226,6 +228,7 @@ struct BatchArgs {
     const float2* circ;         // [K][N*H][N] receptor circulant samples
     const int8_t* cscale;       // [N*H] power-of-two scale exponents
     int x0, W;                  // ligand window along x
+    int tc_pair;                // tensor form over pencil pairs (pencil_tcp.cuh), else pencil_tc_kernel
     uint32_t* ent_t;            // [B/128][n_pad][128] entries transposed per group of 128 rotations
     const int32_t* tinfo;       // padded entry starts of the n_tc_terms non-empty terms, then their term ids
     const int32_t* tpad;        // [K] padded start - start of each term's entries
@@ -233,7 +236,7 @@ struct BatchArgs {
     int tc_group;               // terms per tensor-memory sum (<= 0: FFTDOCK_TC_TERMS_PER_SUM_DEFAULT)
     float2* tc_slots;           // [tc_n_slots][128][128] running sums of the tensor stage's CTAs
     int tc_n_slots;             // 2 per SM id (tc_slot_count)
-    int n_pad;                  // entries per rotation with every term padded to a multiple of 8
+    int n_pad;                  // entries per rotation with every term padded to a multiple of 8 (+ 4 n_tc_terms: tc_pair)
     int* err;                   // device word: nonzero after a pipeline timeout
     WideArgs wide;              // queue + clustering path (wide.corr != nullptr)
     // box-grid path (box.n[0] > 0): per-axis geometry and the FP32 twiddle
@@ -248,16 +251,24 @@ struct BatchArgs {
 // 8).  ok = the window and the term count fit the stage.
 struct TcTables {
     int x0 = 0, W = 0;
-    int n_pad = 0;                 // padded rows per rotation
+    int n_pad = 0;                 // rows per rotation
     int ka = 0;                    // non-empty terms
     std::vector<int32_t> info;     // [ka + 1] padded starts, then [ka] term ids
     std::vector<int32_t> tpad;     // [K] padded start - start of each term
     bool ok = false;
+    bool pair = false;             // pencil pairs fit (pencil_tcp.cuh)
+    // pencil pairs: a quad of rows per term more, for its occupied staging rows
+    void set_pair(bool p) {
+        pair = p;
+        n_pad = info[ka] + (p ? 4 * ka : 0);
+    }
+    // staging row that takes padding and cells outside the window
+    int dummy_row() const { return pair ? 2 * W : W; }
 };
 TcTables tc_tables(const double* xyz, const int32_t* term, int n, int K, int N, double h, double zero_h);
-// the padding rows of the transposed entries: x' = W (the tensor stage's
-// dummy staging row), y = z = 0
-cudaError_t fill_padding(uint32_t* ent_t, int W, size_t n, cudaStream_t s);
+// the padding rows of the transposed entries: the tensor stage's dummy
+// staging row, y = z = 0
+cudaError_t fill_padding(uint32_t* ent_t, int dummy_row, size_t n, cudaStream_t s);
 // slots of the tensor stage's running sums on the current device: two per SM
 // id (%nsmid, which bounds %smid), one per tensor-memory half
 cudaError_t tc_slot_count(int* n_slots);
@@ -299,6 +310,9 @@ size_t box_pencil_smem(int nx, int ny, int nz, int K, int n_ent, bool weighted);
 // cubic grid of edge n
 size_t box_tc_smem(const int dims[3], int n_chunks, int n_terms);
 size_t cubic_tc_smem(int n, int n_chunks, int n_terms);
+// whether the tensor stage runs over pencil pairs: Nx <= 128, even Ny, and it
+// and ligand prep's two-class bins (K terms, n_ent entries) fit shared memory
+bool tc_pairs_fit(const int dims[3], bool box, int K, int n_ent, int n_chunks, int n_terms);
 
 // FFT form of the pencil stage on a box grid: entry classes per x bin, the
 // launch, and its kernels' code

@@ -281,7 +281,7 @@ cudaError_t enqueue_pair(Run& r, const fftdock_pair& p, int i, Work& w, const Si
     if (tc) {
         const fftdock::TcTables& tt = r.st.tct[i];
         // this pair's padding rows (x' = its window width) over the rows its batches use
-        e = fftdock::fill_padding(w.ent_t, tt.W, (size_t)B * tt.n_pad + 16 * fftdock::kTcRot, s);
+        e = fftdock::fill_padding(w.ent_t, tt.dummy_row(), (size_t)B * tt.n_pad + 16 * fftdock::kTcRot, s);
         if (e != cudaSuccess) return e;
     }
     BatchArgs a{};
@@ -310,6 +310,7 @@ cudaError_t enqueue_pair(Run& r, const fftdock_pair& p, int i, Work& w, const Si
     if (tc) {
         const fftdock::TcTables& tt = r.st.tct[i];
         a.use_tc = 1;
+        a.tc_pair = tt.pair ? 1 : 0;
         a.circ = w.circ;
         a.cscale = w.cscale;
         a.tc_slots = r.tc_slots;

@@ -170,7 +170,8 @@ __global__ void __launch_bounds__(256) ligand_prep_kernel(
     int n_ent, int K, Geo geo, uint32_t* __restrict__ ent_out, int32_t* __restrict__ offs_out,
     int32_t* __restrict__ status, const float* __restrict__ w_in, uint4* __restrict__ ent4,
     int32_t* __restrict__ idx_out, uint32_t* __restrict__ ent_t, const int32_t* __restrict__ tpad, int n_pad,
-    int x0, int W, int qc) {
+    int x0, int W, int qc, const int32_t* __restrict__ tinfo,
+    int ka) {
     extern __shared__ unsigned char smem_raw[];
     int32_t* cnt = reinterpret_cast<int32_t*>(smem_raw);               // [K*N*qc + 1]
     uint32_t* keys = reinterpret_cast<uint32_t*>(cnt + K * N * qc + 1);  // [n_ent]
@@ -230,7 +231,22 @@ __global__ void __launch_bounds__(256) ligand_prep_kernel(
         __syncthreads();
     }
     int32_t* offs = offs_out + (size_t)q * (nbins + 1);
-    for (int i = tid; i <= nbins; i += blockDim.x) offs[i] = cnt[i];
+    if (!ent_t)  // (the tensor form does not read them)
+        for (int i = tid; i <= nbins; i += blockDim.x) offs[i] = cnt[i];
+    // pencil pairs: which staging rows of each term hold an entry, one bit per
+    // row, after the term rows (a quad of rows per term)
+    for (int i = tid; i < 3 * ka; i += blockDim.x) {
+        const int kk = i / 3, word = i - 3 * kk, t = tinfo[ka + 1 + kk];
+        uint32_t m = 0;
+        for (int j = 0; j < 16; ++j) {
+            const int xr = 16 * word + j, c = xr + x0;
+            if (xr < W && c >= 0 && c < N) {
+                const int b = (t * N + c) * qc;
+                m |= (uint32_t)(cnt[b + 1] > cnt[b]) << (2 * j) | (uint32_t)(cnt[b + 2] > cnt[b + 1]) << (2 * j + 1);
+            }
+        }
+        ent_t[(((size_t)(q >> 7) * (n_pad >> 2) + (tinfo[ka] >> 2) + kk) * 128 + (q & 127)) * 4 + word] = m;
+    }
     __syncthreads();
     // stable scatter by one warp: ranks within equal keys follow atom order
     if (tid < 32) {
@@ -251,13 +267,15 @@ __global__ void __launch_bounds__(256) ligand_prep_kernel(
             // [q / 128][row / 4][q % 128][row % 4], with each term's rows
             // padded to a multiple of 8; the term is implied by the row and
             // x is stored relative to the window start x0 (mod 256: cells
-            // outside the window stay outside it); entry = x' << 24 | y << 16
-            // | z, so that one multiply by kz << 16 | ky gives the phase
+            // outside the window stay outside it); entry = row << 24 | y << 16
+            // | z, so that one multiply by kz << 16 | ky gives the phase; row =
+            // x', or 2 x' + y mod 2 for pencil pairs
             if (act && ent_t) {
                 const size_t row = (size_t)(dst + __ldg(tpad + (key >> 24)));
+                uint32_t xr = min(((key >> 16) - (uint32_t)x0) & 255u, (uint32_t)W);
+                if (ka) xr = 2 * xr + (xr < (uint32_t)W ? (key >> 8) & 1u : 0u);
                 ent_t[(((size_t)(q >> 7) * (n_pad >> 2) + (row >> 2)) * 128 + (q & 127)) * 4 + (row & 3)] =
-                    (min(((key >> 16) - (uint32_t)x0) & 255u, (uint32_t)W) << 24) | (((key >> 8) & 255u) << 16) |
-                    (key & 255u);
+                    (xr << 24) | (((key >> 8) & 255u) << 16) | (key & 255u);
             }
             if (act && ent4) {
                 // ljComp: entry i < n_ent / 2 weighs atom i into term 0, entry
