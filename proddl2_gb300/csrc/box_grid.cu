@@ -294,7 +294,7 @@ size_t prep_smem_bytes(int nx, int K, int n_ent, int qc) {
 }
 
 cudaError_t set_smem(const void* fn, size_t bytes) {
-    if (bytes <= 48 * 1024) return cudaSuccess;
+    if (bytes <= kDynSmemNoOptIn) return cudaSuccess;
     return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
 }
 

@@ -29,7 +29,7 @@ template <int N> struct SizeOpsImpl {
     }
 
     static cudaError_t set_smem(const void* fn, size_t bytes) {
-        if (bytes <= 48 * 1024) return cudaSuccess;
+        if (bytes <= kDynSmemNoOptIn) return cudaSuccess;
         return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
     }
 
