@@ -255,7 +255,9 @@ int fftdock_n_terms(const fftdock_ctx* ctx);
 typedef struct fftdock_scan_info {
     int32_t grid_n;
     int32_t n_terms;       /* K correlation terms */
-    int32_t pencil_path;   /* FFTDOCK_PENCIL_FFT or FFTDOCK_PENCIL_TENSOR (the form that runs) */
+    int32_t pencil_path;   /* FFTDOCK_PENCIL_FFT or FFTDOCK_PENCIL_TENSOR (the form that runs; under
+                            * FFTDOCK_PENCIL_AUTO a scan's last few rotations beside whole groups of 128
+                            * run the FFT form, which is faster for them) */
     int32_t rot_batch;     /* rotations per device batch */
     int32_t n_entries;     /* ligand entries (0 before fftdock_set_ligand) */
     int32_t window_x0;     /* tensor path: first x cell of the ligand window */

@@ -295,10 +295,18 @@ int run_batches(fftdock_ctx* ctx, int n_rot, const double* rot, int first_id, ff
     const int N = ctx->N, stride = ctx->cfg.peaks_per_rot;
     int rc;
     size_t ev = 0;
-    for (int g0 = 0; g0 < n_rot; g0 += ctx->G) {
+    // (not where FP32 correlations are returned or order a queue: those are one
+    // form's for any number of rotations)
+    const bool fp64_only = !dbg && !pool_v && !a.wide.corr;
+    const int few = a.use_tc && fp64_only && ctx->cfg.pencil_mode == FFTDOCK_PENCIL_AUTO
+                        ? fftdock::few_rotations(ctx->dims)
+                        : 0;
+    for (int g0 = 0, ng; g0 < n_rot; g0 += ng) {
         BatchArgs ga = a;
         ga.ev = nullptr;
-        ga.n_rot = std::min(ctx->G, n_rot - g0);
+        ng = fftdock::whole_groups(std::min(ctx->G, n_rot - g0), few);
+        ga.n_rot = ng;
+        if (ng <= few) ga.run_fft_form();
         ga.rot = rot + (size_t)g0 * 9;
         ga.status = status + g0;
         ga.peaks = peaks + (size_t)g0 * stride;

@@ -183,6 +183,11 @@ struct BatchArgs {
     int classes() const { return use_tc ? (tc_pair ? 2 : 1) : qc; }
     // terms whose occupied staging rows ligand prep marks
     int mask_terms() const { return use_tc && tc_pair ? n_tc_terms : 0; }
+    // the FFT form, whichever was selected (its tables and work memory are there)
+    void run_fft_form() {
+        use_tc = 0;
+        ent_t = nullptr;
+    }
     size_t offs_stride(int nx) const { return (size_t)K * nx * classes() + 1; }
     // inputs
     const double* rot;          // [B][9]
@@ -276,6 +281,23 @@ cudaError_t tc_slot_count(int* n_slots);
 // spectra, an unweighted term set with at least kTcMinTerms terms (at 64^3
 // with the single shape term the FFT form measured faster)
 constexpr int kTcMinTerms = 4;
+// Under AUTO with the tensor form selected, up to this many rotations (a call's
+// last rotations after whole groups of 128, or a whole call) run the FFT form:
+// the tensor stage costs a whole group's time for any part of one, the FFT form
+// a rotation's time each.  Pencil stage at 19 terms, FFT / tensor, GB300:
+// 48^3 8 rotations 0.028 / 0.149 ms, 32: 0.065 / 0.149; 96^3 32: 0.60 / 0.93, 48:
+// 0.87 / 0.94; 112^3 16: 0.81 / 1.50, 32: 1.55 / 1.50; 128^3 16: 0.72 / 1.91; box
+// 50x44x36 16: 0.073 / 0.088, 32: 0.107 / 0.088; box 112x120x126 16: 0.92 / 1.96,
+// 32: 1.78 / 1.98.
+inline int few_rotations(const int dims[3]) {
+    return dims[0] == dims[1] && dims[0] == dims[2] && dims[0] <= 96 ? 32 : 16;
+}
+// rotations of the next pass over n: without the last few (<= few, 0: none)
+// when whole groups of kTcRot come before them
+inline int whole_groups(int n, int few) {
+    const int tail = n % kTcRot;
+    return n > kTcRot && tail > 0 && tail <= few ? n - tail : n;
+}
 
 // queue + clustering stage of one batch, after the correlation grids of the
 // batch are in a.wide.corr; writes a.peaks / a.n_peaks

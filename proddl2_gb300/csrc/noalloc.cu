@@ -119,8 +119,7 @@ extern "C" int fftdock_scan_device_noalloc(fftdock_ctx* ctx, int32_t n_rot, cons
     a.pool_i = nullptr;
     a.ev = nullptr;
     // the FFT form of the pencil stage: its work memory fits the static array
-    a.use_tc = 0;
-    a.ent_t = nullptr;
+    a.run_fft_form();
     cudaStream_t s = stream ? (cudaStream_t)stream : in.stream;
     for (int b0 = 0; b0 < n_rot; b0 += b) {
         a.n_rot = n_rot - b0 < b ? n_rot - b0 : b;
