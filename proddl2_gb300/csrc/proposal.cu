@@ -98,13 +98,23 @@ __device__ __forceinline__ uint64_t mix64(uint64_t z) {
     return z ^ (z >> 31);
 }
 
+// input position of output position (oz, oy, ox) under tap t of a stride-2,
+// pad-1 3^3 convolution over a din^3 grid; -1 outside
+__device__ __forceinline__ int tap_source(int din, int oz, int oy, int ox, int t) {
+    const int z = 2 * oz - 1 + t / 9, y = 2 * oy - 1 + (t / 3) % 3, x = 2 * ox - 1 + t % 3;
+    if (z < 0 || z >= din || y < 0 || y >= din || x < 0 || x >= din) return -1;
+    return (z * din + y) * din + x;
+}
+
 // ---------------------------------------------------------------------------
 // GEMM: C[M][N] = A[M][K] x B[K][N], BF16 operands, FP32 accumulation on the
-// tensor cores.  A is row-major (AT = false: A[m * lda + k]) or stored
-// transposed (AT = true: A[k * lda + m]); B likewise ("KN", BT = false:
-// B[k * ldb + n]; "NK", BT = true: B[n * ldb + k]).  The contiguous extent of
-// each operand and its leading dimension are multiples of 8 and its base is
-// 16-byte aligned (checked by the host), so every copy is 16 bytes.
+// tensor cores.  A is row-major (AT = false: element (m, k)) or stored
+// transposed (AT = true: (k, m)); B likewise ("KN", BT = false: (k, n); "NK", BT =
+// true: (n, k)).  An operand is a matrix in memory (Dense: its contiguous extent
+// and leading dimension are multiples of 8 and its base is 16-byte aligned) or
+// the im2col matrix of an activation, whose elements are gathered as they are
+// copied (Im2col: 4,096 predictions no longer write and read 310 MB of them, 77
+// us), so every copy is 16 bytes.
 // CTA tile BM x BN x 32, four warps of WM x WN.  These GEMMs are short and
 // narrow (K of 32 to 1,024 per CTA, N from 16), so they are bound by the latency
 // of their K steps: four stages of tiles are in flight (cp.async, out-of-range
@@ -119,6 +129,23 @@ __device__ __forceinline__ uint64_t mix64(uint64_t z) {
 // its index.
 // ---------------------------------------------------------------------------
 constexpr int GBK = 32, GTHREADS = 128, GSTAGES = 4;
+
+struct Dense {
+    const bf16* p;
+    int ld;
+    __device__ __forceinline__ const bf16* at(int row, int col) const { return p + (size_t)row * ld + col; }
+};
+// im2col of a channel-last activation act[s * PIN + pos_in][CIN]: row s * POUT +
+// pos, column tap * CIN + ci; nullptr where the tap lies outside (zero)
+template <int CIN, int DIN> struct Im2col {
+    const bf16* act;
+    __device__ __forceinline__ const bf16* at(int row, int col) const {
+        constexpr int DOUT = DIN / 2, POUT = DOUT * DOUT * DOUT, PIN = DIN * DIN * DIN;
+        const int s = row / POUT, pos = row % POUT;
+        const int src = tap_source(DIN, pos / (DOUT * DOUT), (pos / DOUT) % DOUT, pos % DOUT, col / CIN);
+        return src < 0 ? nullptr : act + ((size_t)s * PIN + src) * CIN + col % CIN;
+    }
+};
 
 __device__ __forceinline__ void mma_bf16(float (&d)[4], const uint32_t (&a)[4], const uint32_t (&b)[2]) {
     asm volatile(
@@ -141,29 +168,31 @@ template <bool TRANS> __device__ __forceinline__ void ldmatrix4(uint32_t (&r)[4]
                      : "memory");
 }
 
-// operand tile of ROWS rows x 32 k: T = false [ROWS][32 + 8] of p[row * ld + k],
-// T = true [32][ROWS + 8] of p[k * ld + row]
+// operand tile of ROWS rows x 32 k: T = false [ROWS][32 + 8] of (row, k), T = true
+// [32][ROWS + 8] of (k, row)
 template <int ROWS, bool T> constexpr int gemm_tile_elems() { return T ? GBK * (ROWS + 8) : ROWS * (GBK + 8); }
 
-template <int ROWS, bool T>
-__device__ __forceinline__ void copy_tile(uint32_t dst, const bf16* __restrict__ p, int ld, int r0, int rows, int k0,
-                                          int k1) {
+template <int ROWS, bool T, class Op>
+__device__ __forceinline__ void copy_tile(uint32_t dst, const Op& op, const bf16* any, int r0, int rows, int k0, int k1) {
     constexpr int CH = ROWS * GBK / 8;  // 16-byte chunks
 #pragma unroll
     for (int e0 = 0; e0 < CH; e0 += GTHREADS) {
         const int e = e0 + (int)threadIdx.x;
         if (CH % GTHREADS != 0 && e >= CH) break;
         const int rr = T ? (e % (ROWS / 8)) * 8 : e >> 2, kk = T ? e / (ROWS / 8) : (e & 3) * 8;
-        const bool in = r0 + rr < rows && k0 + kk < k1;
-        const bf16* src = in ? (T ? p + (size_t)(k0 + kk) * ld + r0 + rr : p + (size_t)(r0 + rr) * ld + k0 + kk) : p;
+        const bf16* src = nullptr;
+        if (r0 + rr < rows && k0 + kk < k1) src = T ? op.at(k0 + kk, r0 + rr) : op.at(r0 + rr, k0 + kk);
         const uint32_t d = dst + 2u * (uint32_t)(T ? kk * (ROWS + 8) + rr : rr * (GBK + 8) + kk);
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(in ? 16 : 0) : "memory");
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src ? src : any),
+                     "r"(src ? 16 : 0)
+                     : "memory");
     }
 }
 
-template <int BM, int BN, int WM, int WN, bool AT, bool BT, class Epi>
-__global__ void __launch_bounds__(GTHREADS) gemm_kernel(int M, int N, int K, const bf16* __restrict__ A, int lda,
-                                                        const bf16* __restrict__ B, int ldb, int k_chunk, Epi epi) {
+// any: a readable address for zero-filled copies
+template <int BM, int BN, int WM, int WN, bool AT, bool BT, class OpA, class OpB, class Epi>
+__global__ void __launch_bounds__(GTHREADS) gemm_kernel(int M, int N, int K, OpA A, OpB B, const bf16* any, int k_chunk,
+                                                        Epi epi) {
     static_assert((BM / WM) * (BN / WN) * 32 == GTHREADS && WM % 16 == 0 && WN % 16 == 0, "four warps");
     constexpr int EA = gemm_tile_elems<BM, AT>(), EB = gemm_tile_elems<BN, !BT>();
     constexpr int FM = WM / 16, FN = WN / 8;
@@ -192,8 +221,8 @@ __global__ void __launch_bounds__(GTHREADS) gemm_kernel(int M, int N, int K, con
     auto copy_step = [&](int t) {
         if (t < steps) {
             const uint32_t d = base + (uint32_t)(t % GSTAGES) * STAGE;
-            copy_tile<BM, AT>(d, A, lda, m0, M, kb + t * GBK, ke);
-            copy_tile<BN, !BT>(d + 2u * EA, B, ldb, n0, N, kb + t * GBK, ke);
+            copy_tile<BM, AT>(d, A, any, m0, M, kb + t * GBK, ke);
+            copy_tile<BN, !BT>(d + 2u * EA, B, any, n0, N, kb + t * GBK, ke);
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
@@ -323,7 +352,7 @@ struct EpiWgrad {  // column tap * cin + ci of output channel r -> g[(r * cin + 
 };
 
 // ---------------------------------------------------------------------------
-// samples, occupancy and the im2col / col2im gathers
+// samples, occupancy and the col2im gather
 // ---------------------------------------------------------------------------
 struct Ligands {
     const double* xyz;    // all ligands' atoms, concatenated
@@ -389,14 +418,6 @@ __device__ void occupancy(const double* __restrict__ xyz, int n, double L, const
     __syncthreads();
 }
 
-// input position of output position (oz, oy, ox) under tap t of a stride-2,
-// pad-1 3^3 convolution over a din^3 grid; -1 outside
-__device__ __forceinline__ int tap_source(int din, int oz, int oy, int ox, int t) {
-    const int z = 2 * oz - 1 + t / 9, y = 2 * oy - 1 + (t / 3) % 3, x = 2 * ox - 1 + t % 3;
-    if (z < 0 || z >= din || y < 0 || y >= din || x < 0 || x >= din) return -1;
-    return (z * din + y) * din + x;
-}
-
 // one CTA per sample: occupancy -> x0 (BF16) -> conv1's im2col rows
 // x1c[s * P1 + pos][tap]: column 27 is 1 (its weight is zero, and the
 // weight-gradient GEMM gets the bias gradient there), 28..31 zero; the
@@ -443,23 +464,6 @@ __global__ void __launch_bounds__(THREADS) prep_kernel(Ligands lg, SampleSrc src
         }
         *reinterpret_cast<uint4*>(x1c + ((size_t)b * P1 + pos) * K1 + t0) = make_uint4(q[0], q[1], q[2], q[3]);
     }
-}
-
-// im2col of a channel-last activation act[s * PIN + pos_in][CIN] into
-// col[s * POUT + pos][tap * CIN + ci]; one thread per (row, tap)
-template <int CIN, int DIN>
-__global__ void im2col_kernel(const bf16* __restrict__ act, bf16* __restrict__ col, int n_samples) {
-    constexpr int DOUT = DIN / 2, POUT = DOUT * DOUT * DOUT, PIN = DIN * DIN * DIN;
-    const size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= (size_t)n_samples * POUT * 27) return;
-    const int t = (int)(e % 27);
-    const size_t row = e / 27;
-    const int s = (int)(row / POUT), pos = (int)(row % POUT);
-    const int src_i = tap_source(DIN, pos / (DOUT * DOUT), (pos / DOUT) % DOUT, pos % DOUT, t);
-    uint4* dst = reinterpret_cast<uint4*>(col + row * (27 * CIN) + t * CIN);
-    const uint4* sp = reinterpret_cast<const uint4*>(act + ((size_t)s * PIN + (src_i < 0 ? 0 : src_i)) * CIN);
-#pragma unroll
-    for (int i = 0; i < CIN / 8; ++i) dst[i] = src_i >= 0 ? sp[i] : make_uint4(0u, 0u, 0u, 0u);
 }
 
 // col2im: the input gradient of a convolution from the gradient of its
@@ -651,9 +655,7 @@ struct Work {
     bool grads = false;  // the backward buffers are allocated
     bf16* x1c = nullptr;  // [cap * P1][K1]
     bf16* a1 = nullptr;   // [cap * P1][C1]
-    bf16* x2c = nullptr;  // [cap * P2][K2]
     bf16* a2 = nullptr;   // [cap * P2][C2]
-    bf16* x3c = nullptr;  // [cap * P3][K3]
     bf16* u = nullptr;    // [cap][NU]
     bf16* h1 = nullptr;   // [cap][HID]
     int* sidx = nullptr;  // [cap] sample index of each slot
@@ -671,9 +673,7 @@ struct Work {
     void release() {
         dfree(x1c);
         dfree(a1);
-        dfree(x2c);
         dfree(a2);
-        dfree(x3c);
         dfree(u);
         dfree(h1);
         dfree(sidx);
@@ -811,9 +811,7 @@ int grow_work(fftdock_proposal* p, int cap, bool grads) {
     drop_graph(p);
     PK(dalloc(&w.x1c, (size_t)c * P1 * K1));
     PK(dalloc(&w.a1, (size_t)c * P1 * C1));
-    PK(dalloc(&w.x2c, (size_t)c * P2 * K2));
     PK(dalloc(&w.a2, (size_t)c * P2 * C2));
-    PK(dalloc(&w.x3c, (size_t)c * P3 * K3));
     PK(dalloc(&w.u, (size_t)c * NU));
     PK(dalloc(&w.h1, (size_t)c * HID));
     PK(dalloc(&w.sidx, (size_t)c));
@@ -834,42 +832,43 @@ int grow_work(fftdock_proposal* p, int cap, bool grads) {
     return FFTDOCK_OK;
 }
 
-template <int BM, int BN, int WM, int WN, bool AT, bool BT, class Epi>
-cudaError_t gemm_tiled(int M, int N, int K, const bf16* A, int lda, const bf16* B, int ldb, int kc, int splits, Epi epi,
+template <int BM, int BN, int WM, int WN, bool AT, bool BT, class OpA, class OpB, class Epi>
+cudaError_t gemm_tiled(int M, int N, int K, const OpA& A, const OpB& B, const bf16* any, int kc, int splits, Epi epi,
                        cudaStream_t s) {
     const dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM, splits);
-    gemm_kernel<BM, BN, WM, WN, AT, BT, Epi><<<grid, GTHREADS, 0, s>>>(M, N, K, A, lda, B, ldb, kc, epi);
+    gemm_kernel<BM, BN, WM, WN, AT, BT><<<grid, GTHREADS, 0, s>>>(M, N, K, A, B, any, kc, epi);
     return cudaGetLastError();
 }
 
 // Tile of a GEMM: 128 x 16 for the 16-channel outputs of many rows, otherwise 64
 // rows and 32 or 64 columns where that fills the GPU twice over (2 x 152 CTAs),
 // else 32 x 32, which gives four times the CTAs.
-template <bool AT, bool BT, class Epi>
-cudaError_t gemm_launch(int M, int N, int K, const bf16* A, int lda, const bf16* B, int ldb, int kc, int splits, Epi epi,
+template <bool AT, bool BT, class OpA, class OpB, class Epi>
+cudaError_t gemm_launch(int M, int N, int K, const OpA& A, const OpB& B, const bf16* any, int kc, int splits, Epi epi,
                         cudaStream_t s) {
     constexpr int kFill = 2 * 152;
     const int m64 = (M + 63) / 64 * splits;
     if (N <= 16 && m64 / 2 >= kFill)
-        return gemm_tiled<128, 16, 32, 16, AT, BT>(M, N, K, A, lda, B, ldb, kc, splits, epi, s);
+        return gemm_tiled<128, 16, 32, 16, AT, BT>(M, N, K, A, B, any, kc, splits, epi, s);
     if (N <= 32 && m64 >= kFill)
-        return gemm_tiled<64, 32, 32, 16, AT, BT>(M, N, K, A, lda, B, ldb, kc, splits, epi, s);
+        return gemm_tiled<64, 32, 32, 16, AT, BT>(M, N, K, A, B, any, kc, splits, epi, s);
     if (m64 * ((N + 63) / 64) >= kFill)
-        return gemm_tiled<64, 64, 32, 32, AT, BT>(M, N, K, A, lda, B, ldb, kc, splits, epi, s);
-    return gemm_tiled<32, 32, 16, 16, AT, BT>(M, N, K, A, lda, B, ldb, kc, splits, epi, s);
+        return gemm_tiled<64, 64, 32, 32, AT, BT>(M, N, K, A, B, any, kc, splits, epi, s);
+    return gemm_tiled<32, 32, 16, 16, AT, BT>(M, N, K, A, B, any, kc, splits, epi, s);
 }
 
 // C = A x B through gemm_kernel, K split into `splits` parts (partial sums
-// reduced in split order into the epilogue)
-template <bool AT, bool BT, class Epi>
-cudaError_t gemm(int M, int N, int K, const bf16* A, int lda, const bf16* B, int ldb, Epi epi, int splits, float* ws,
+// reduced in split order into the epilogue); any: a readable 16-byte aligned
+// address
+template <bool AT, bool BT, class OpA, class OpB, class Epi>
+cudaError_t gemm(int M, int N, int K, const OpA& A, const OpB& B, const bf16* any, Epi epi, int splits, float* ws,
                  cudaStream_t s) {
     // the partial sums fit the workspace
     splits = std::max(1, std::min({splits, RMAXS, (int)((size_t)WS_FLOATS / ((size_t)M * N))}));
     const int kc = ((K + splits * GBK - 1) / (splits * GBK)) * GBK;
     splits = (K + kc - 1) / kc;
-    if (splits == 1) return gemm_launch<AT, BT>(M, N, K, A, lda, B, ldb, kc, 1, epi, s);
-    cudaError_t e = gemm_launch<AT, BT>(M, N, K, A, lda, B, ldb, kc, splits, EpiPartial{ws, M, N}, s);
+    if (splits == 1) return gemm_launch<AT, BT>(M, N, K, A, B, any, kc, 1, epi, s);
+    cudaError_t e = gemm_launch<AT, BT>(M, N, K, A, B, any, kc, splits, EpiPartial{ws, M, N}, s);
     if (e != cudaSuccess) return e;
     splitk_reduce_kernel<Epi><<<(M * N / 2 + RPAIRS - 1) / RPAIRS, 16 * RPAIRS, 0, s>>>(ws, splits, M, N, epi);
     return cudaGetLastError();
@@ -881,22 +880,17 @@ cudaError_t launch_forward(fftdock_proposal* p, int n, const SampleSrc& src, cud
     cudaError_t e;
     prep_kernel<<<n, THREADS, 0, s>>>(ligands(p), src, w.x1c, w.u, w.sidx);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    if ((e = gemm<false, true>(n * P1, C1, K1, w.x1c, K1, p->wp + OP1, K1, EpiBiasRelu{w.a1, C1, p->wb + OB1}, 1,
-                               nullptr, s)) != cudaSuccess)
+    if ((e = gemm<false, true>(n * P1, C1, K1, Dense{w.x1c, K1}, Dense{p->wp + OP1, K1}, p->wp,
+                               EpiBiasRelu{w.a1, C1, p->wb + OB1}, 1, nullptr, s)) != cudaSuccess)
         return e;
-    const size_t c2 = (size_t)n * P2 * 27, c3 = (size_t)n * P3 * 27;
-    im2col_kernel<C1, D1><<<(unsigned)((c2 + 255) / 256), 256, 0, s>>>(w.a1, w.x2c, n);
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    if ((e = gemm<false, true>(n * P2, C2, K2, w.x2c, K2, p->wp + OP2, K2, EpiBiasRelu{w.a2, C2, p->wb + OB2}, 1,
-                               nullptr, s)) != cudaSuccess)
+    if ((e = gemm<false, true>(n * P2, C2, K2, Im2col<C1, D1>{w.a1}, Dense{p->wp + OP2, K2}, p->wp,
+                               EpiBiasRelu{w.a2, C2, p->wb + OB2}, 1, nullptr, s)) != cudaSuccess)
         return e;
-    im2col_kernel<C2, D2><<<(unsigned)((c3 + 255) / 256), 256, 0, s>>>(w.a2, w.x3c, n);
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    if ((e = gemm<false, true>(n * P3, C3, K3, w.x3c, K3, p->wp + OP3, K3, EpiConv3{w.u, p->wb + OB3}, 1, nullptr,
-                               s)) != cudaSuccess)
+    if ((e = gemm<false, true>(n * P3, C3, K3, Im2col<C2, D2>{w.a2}, Dense{p->wp + OP3, K3}, p->wp,
+                               EpiConv3{w.u, p->wb + OB3}, 1, nullptr, s)) != cudaSuccess)
         return e;
-    return gemm<false, false>(n, HID, NU, w.u, NU, p->wb + OF1, HID, EpiBiasRelu{w.h1, HID, p->wb + OFB1}, 1, nullptr,
-                              s);
+    return gemm<false, false>(n, HID, NU, Dense{w.u, NU}, Dense{p->wb + OF1, HID}, p->wp,
+                              EpiBiasRelu{w.h1, HID, p->wb + OFB1}, 1, nullptr, s);
 }
 
 // K split of a weight gradient over rows samples x positions
@@ -924,37 +918,38 @@ cudaError_t launch_gradients(fftdock_proposal* p, int B, const SampleSrc& src, c
     fc2_wgrad_kernel<<<HID / 32, THREADS, 0, s>>>(w.h1, w.dy, B, g);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     // fc1: dW1 = u^T dzf, db1 = column sums of dzf, du -> dz3 (masked by a3 > 0)
-    if ((e = gemm<true, false>(NU, HID, B, w.u, NU, w.dzf, HID, EpiF32{g + OF1, HID}, 1, nullptr, s)) != cudaSuccess)
+    if ((e = gemm<true, false>(NU, HID, B, Dense{w.u, NU}, Dense{w.dzf, HID}, p->wp, EpiF32{g + OF1, HID}, 1, nullptr,
+                               s)) != cudaSuccess)
         return e;
     if ((e = colsum(w.dzf, B, HID, w.cs, g + OFB1, s)) != cudaSuccess) return e;
-    if ((e = gemm<false, true>(B, NA3, HID, w.dzf, HID, p->wb + OF1, HID, EpiDz3{w.dz3, w.u}, 1, nullptr, s)) !=
-        cudaSuccess)
+    if ((e = gemm<false, true>(B, NA3, HID, Dense{w.dzf, HID}, Dense{p->wb + OF1, HID}, p->wp, EpiDz3{w.dz3, w.u}, 1,
+                               nullptr, s)) != cudaSuccess)
         return e;
     // conv3
     const int r3 = B * P3, r2 = B * P2, r1 = B * P1;
-    if ((e = gemm<true, false>(C3, K3, r3, w.dz3, C3, w.x3c, K3, EpiWgrad{g + OW3, C2, nullptr}, wgrad_splits(r3),
-                               w.ws, s)) != cudaSuccess)
+    if ((e = gemm<true, false>(C3, K3, r3, Dense{w.dz3, C3}, Im2col<C2, D2>{w.a2}, p->wp,
+                               EpiWgrad{g + OW3, C2, nullptr}, wgrad_splits(r3), w.ws, s)) != cudaSuccess)
         return e;
     if ((e = colsum(w.dz3, r3, C3, w.cs, g + OB3, s)) != cudaSuccess) return e;
-    if ((e = gemm<false, false>(r3, K3, C3, w.dz3, C3, p->wp + OP3, K3, EpiF32{w.dx3, K3}, 1, nullptr, s)) !=
-        cudaSuccess)
+    if ((e = gemm<false, false>(r3, K3, C3, Dense{w.dz3, C3}, Dense{p->wp + OP3, K3}, p->wp, EpiF32{w.dx3, K3}, 1,
+                                nullptr, s)) != cudaSuccess)
         return e;
     const size_t e2 = (size_t)B * P2 * C2 / 4, e1 = (size_t)B * P1 * C1 / 4;
     col2im_kernel<C2, D2><<<(unsigned)((e2 + 255) / 256), 256, 0, s>>>(w.dx3, w.a2, w.dz2, B);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     // conv2
-    if ((e = gemm<true, false>(C2, K2, r2, w.dz2, C2, w.x2c, K2, EpiWgrad{g + OW2, C1, nullptr}, wgrad_splits(r2),
-                               w.ws, s)) != cudaSuccess)
+    if ((e = gemm<true, false>(C2, K2, r2, Dense{w.dz2, C2}, Im2col<C1, D1>{w.a1}, p->wp,
+                               EpiWgrad{g + OW2, C1, nullptr}, wgrad_splits(r2), w.ws, s)) != cudaSuccess)
         return e;
     if ((e = colsum(w.dz2, r2, C2, w.cs, g + OB2, s)) != cudaSuccess) return e;
-    if ((e = gemm<false, false>(r2, K2, C2, w.dz2, C2, p->wp + OP2, K2, EpiF32{w.dx2, K2}, 1, nullptr, s)) !=
-        cudaSuccess)
+    if ((e = gemm<false, false>(r2, K2, C2, Dense{w.dz2, C2}, Dense{p->wp + OP2, K2}, p->wp, EpiF32{w.dx2, K2}, 1,
+                                nullptr, s)) != cudaSuccess)
         return e;
     col2im_kernel<C1, D1><<<(unsigned)((e1 + 255) / 256), 256, 0, s>>>(w.dx2, w.a1, w.dz1, B);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     // conv1 (the input needs no gradient; the bias gradient is column 27)
-    return gemm<true, false>(C1, K1, r1, w.dz1, C1, w.x1c, K1, EpiWgrad{g + OW1, 1, g + OB1}, wgrad_splits(r1), w.ws,
-                             s);
+    return gemm<true, false>(C1, K1, r1, Dense{w.dz1, C1}, Dense{w.x1c, K1}, p->wp, EpiWgrad{g + OW1, 1, g + OB1},
+                             wgrad_splits(r1), w.ws, s);
 }
 
 }  // namespace
