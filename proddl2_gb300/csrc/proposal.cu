@@ -418,14 +418,21 @@ __device__ void occupancy(const double* __restrict__ xyz, int n, double L, const
     __syncthreads();
 }
 
-// one CTA per sample: occupancy -> x0 (BF16) -> conv1's im2col rows
-// x1c[s * P1 + pos][tap]: column 27 is 1 (its weight is zero, and the
-// weight-gradient GEMM gets the bias gradient there), 28..31 zero; the
-// descriptor -> u[s][NA3..]
-__global__ void __launch_bounds__(THREADS) prep_kernel(Ligands lg, SampleSrc src, bf16* __restrict__ x1c,
-                                                       bf16* __restrict__ u, int* __restrict__ sidx) {
+// one CTA per sample: occupancy -> x0 (BF16, in shared memory with a border of
+// zeros) -> a1[s * P1 + pos][C1], conv1 with bias and ReLU: each warp multiplies 64
+// positions' taps, gathered from x0 into the fragments, by the weights w1 [C1][K1]
+// (columns 27..31 zero); the sums' order is gemm_kernel's.  The descriptor ->
+// u[s][NA3..].  Training (x1c) also stores conv1's im2col rows x1c[s * P1 +
+// pos][tap] for the weight gradient: column 27 is 1 (the bias gradient comes out
+// there), 28..31 zero.  4,096 predictions: 134 MB of rows no longer written and
+// read, 67 + 93 us (this kernel and a GEMM) -> 64 us.
+constexpr int GP = G0 + 2;
+__global__ void __launch_bounds__(THREADS) prep_kernel(Ligands lg, SampleSrc src, const bf16* __restrict__ w1,
+                                                       const bf16* __restrict__ b1, bf16* __restrict__ a1,
+                                                       bf16* __restrict__ x1c, bf16* __restrict__ u,
+                                                       int* __restrict__ sidx) {
     __shared__ float occ[NX0];
-    __shared__ bf16 x0[NX0];
+    __shared__ bf16 xp[GP * GP * GP];
     __shared__ float rs[11];
     const int b = blockIdx.x;
     int idx, lig;
@@ -446,20 +453,70 @@ __global__ void __launch_bounds__(THREADS) prep_kernel(Ligands lg, SampleSrc src
     }
     if (threadIdx.x == 0 && sidx) sidx[b] = idx;
     occupancy(lg.xyz + 3 * (size_t)lg.start[lig], lg.count[lig], lg.half[lig], rot, occ, rs);
-    for (int i = threadIdx.x; i < NX0; i += THREADS) x0[i] = f2b(0.25f * occ[i]);
+    for (int i = threadIdx.x; i < GP * GP * GP; i += THREADS) {
+        const int z = i / (GP * GP) - 1, y = (i / GP) % GP - 1, x = i % GP - 1;
+        const bool in = z >= 0 && z < G0 && y >= 0 && y < G0 && x >= 0 && x < G0;
+        xp[i] = f2b(in ? 0.25f * occ[(z * G0 + y) * G0 + x] : 0.f);
+    }
     for (int i = threadIdx.x; i < DESC; i += THREADS) u[(size_t)b * NU + NA3 + i] = f2b(lg.desc[(size_t)lig * DESC + i]);
     __syncthreads();
+    // x0 under tap t of an output position: xp[origin(pos) + tap_off(t)]
+    auto origin = [](int pos) { return 2 * (((pos / (D1 * D1)) * GP + (pos / D1) % D1) * GP + pos % D1); };
+    auto tap_off = [](int t) { return t < 27 ? ((t / 9) * GP + (t / 3) % 3) * GP + t % 3 : 0; };
+    auto bits = [](bf16 v) { return (uint32_t)__bfloat16_as_ushort(v); };
+    {
+        const int w = threadIdx.x >> 5, gid = (threadIdx.x >> 2) & 7, tig = threadIdx.x & 3;
+        int off[2][4];  // taps 2 tig, 2 tig + 1, and 8 more, of each 16
+        uint32_t wf[2][2][2];
+#pragma unroll
+        for (int ks = 0; ks < 2; ++ks) {
+#pragma unroll
+            for (int q = 0; q < 4; ++q) off[ks][q] = tap_off(16 * ks + 2 * tig + (q & 1) + 8 * (q >> 1));
+#pragma unroll
+            for (int j = 0; j < 2; ++j)
+#pragma unroll
+                for (int h = 0; h < 2; ++h)
+                    wf[ks][j][h] = *reinterpret_cast<const uint32_t*>(w1 + (8 * j + gid) * K1 + 16 * ks + 2 * tig + 8 * h);
+        }
+        float bias[2][2];
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+#pragma unroll
+            for (int c = 0; c < 2; ++c) bias[j][c] = b2f(b1[8 * j + 2 * tig + c]);
+#pragma unroll
+        for (int i = 0; i < P1 / (THREADS / 32) / 16; ++i) {
+            const int pos = (P1 / (THREADS / 32)) * w + 16 * i + gid;
+            const bf16 *x_lo = xp + origin(pos), *x_hi = xp + origin(pos + 8);
+            float acc[2][4] = {};
+#pragma unroll
+            for (int ks = 0; ks < 2; ++ks) {
+                const uint32_t a[4] = {bits(x_lo[off[ks][0]]) | bits(x_lo[off[ks][1]]) << 16,
+                                       bits(x_hi[off[ks][0]]) | bits(x_hi[off[ks][1]]) << 16,
+                                       bits(x_lo[off[ks][2]]) | bits(x_lo[off[ks][3]]) << 16,
+                                       bits(x_hi[off[ks][2]]) | bits(x_hi[off[ks][3]]) << 16};
+#pragma unroll
+                for (int j = 0; j < 2; ++j) mma_bf16(acc[j], a, wf[ks][j]);
+            }
+#pragma unroll
+            for (int j = 0; j < 2; ++j)
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const float v0 = acc[j][2 * h] + bias[j][0], v1 = acc[j][2 * h + 1] + bias[j][1];
+                    *reinterpret_cast<__nv_bfloat162*>(a1 + ((size_t)b * P1 + pos + 8 * h) * C1 + 8 * j + 2 * tig) =
+                        __halves2bfloat162(f2b(v0 > 0.f ? v0 : 0.f), f2b(v1 > 0.f ? v1 : 0.f));
+                }
+        }
+    }
+    if (!x1c) return;
     // rows of 32 taps as 4 groups of 8
     for (int e = threadIdx.x; e < P1 * 4; e += THREADS) {
         const int pos = e >> 2, t0 = (e & 3) * 8;
-        const int oz = pos / (D1 * D1), oy = (pos / D1) % D1, ox = pos % D1;
+        const bf16* x = xp + origin(pos);
         uint32_t q[4] = {0u, 0u, 0u, 0u};
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
             const int t = t0 + i;
-            const int src_i = t < 27 ? tap_source(G0, oz, oy, ox, t) : -1;
-            const uint32_t h = t == 27 ? (uint32_t)__bfloat16_as_ushort(f2b(1.f))
-                                       : (src_i >= 0 ? (uint32_t)__bfloat16_as_ushort(x0[src_i]) : 0u);
+            const uint32_t h = t == 27 ? bits(f2b(1.f)) : (t < 27 ? bits(x[tap_off(t)]) : 0u);
             q[i >> 1] |= h << (16 * (i & 1));
         }
         *reinterpret_cast<uint4*>(x1c + ((size_t)b * P1 + pos) * K1 + t0) = make_uint4(q[0], q[1], q[2], q[3]);
@@ -653,7 +710,7 @@ template <typename T> void dfree(T*& p) {
 struct Work {
     int cap = 0;
     bool grads = false;  // the backward buffers are allocated
-    bf16* x1c = nullptr;  // [cap * P1][K1]
+    bf16* x1c = nullptr;  // [cap * P1][K1] (with grads)
     bf16* a1 = nullptr;   // [cap * P1][C1]
     bf16* a2 = nullptr;   // [cap * P2][C2]
     bf16* u = nullptr;    // [cap][NU]
@@ -809,7 +866,6 @@ int grow_work(fftdock_proposal* p, int cap, bool grads) {
     const bool gr = grads || w.grads;
     w.release();
     drop_graph(p);
-    PK(dalloc(&w.x1c, (size_t)c * P1 * K1));
     PK(dalloc(&w.a1, (size_t)c * P1 * C1));
     PK(dalloc(&w.a2, (size_t)c * P2 * C2));
     PK(dalloc(&w.u, (size_t)c * NU));
@@ -817,6 +873,7 @@ int grow_work(fftdock_proposal* p, int cap, bool grads) {
     PK(dalloc(&w.sidx, (size_t)c));
     PK(dalloc(&w.y, (size_t)c));
     if (gr) {
+        PK(dalloc(&w.x1c, (size_t)c * P1 * K1));
         PK(dalloc(&w.dy, (size_t)c));
         PK(dalloc(&w.dzf, (size_t)c * HID));
         PK(dalloc(&w.dz3, (size_t)c * P3 * C3));
@@ -840,16 +897,13 @@ cudaError_t gemm_tiled(int M, int N, int K, const OpA& A, const OpB& B, const bf
     return cudaGetLastError();
 }
 
-// Tile of a GEMM: 128 x 16 for the 16-channel outputs of many rows, otherwise 64
-// rows and 32 or 64 columns where that fills the GPU twice over (2 x 152 CTAs),
-// else 32 x 32, which gives four times the CTAs.
+// Tile of a GEMM: 64 rows and 32 or 64 columns where that fills the GPU twice over
+// (2 x 152 CTAs), else 32 x 32, which gives four times the CTAs.
 template <bool AT, bool BT, class OpA, class OpB, class Epi>
 cudaError_t gemm_launch(int M, int N, int K, const OpA& A, const OpB& B, const bf16* any, int kc, int splits, Epi epi,
                         cudaStream_t s) {
     constexpr int kFill = 2 * 152;
     const int m64 = (M + 63) / 64 * splits;
-    if (N <= 16 && m64 / 2 >= kFill)
-        return gemm_tiled<128, 16, 32, 16, AT, BT>(M, N, K, A, B, any, kc, splits, epi, s);
     if (N <= 32 && m64 >= kFill)
         return gemm_tiled<64, 32, 32, 16, AT, BT>(M, N, K, A, B, any, kc, splits, epi, s);
     if (m64 * ((N + 63) / 64) >= kFill)
@@ -874,15 +928,14 @@ cudaError_t gemm(int M, int N, int K, const OpA& A, const OpB& B, const bf16* an
     return cudaGetLastError();
 }
 
-// forward of n samples (n <= work capacity): u, h1 and y in the work buffers
-cudaError_t launch_forward(fftdock_proposal* p, int n, const SampleSrc& src, cudaStream_t s) {
+// forward of n samples (n <= work capacity): u, h1 and y in the work buffers,
+// with rows also conv1's im2col rows
+cudaError_t launch_forward(fftdock_proposal* p, int n, const SampleSrc& src, bool rows, cudaStream_t s) {
     Work& w = p->wk;
     cudaError_t e;
-    prep_kernel<<<n, THREADS, 0, s>>>(ligands(p), src, w.x1c, w.u, w.sidx);
+    prep_kernel<<<n, THREADS, 0, s>>>(ligands(p), src, p->wp + OP1, p->wb + OB1, w.a1, rows ? w.x1c : nullptr, w.u,
+                                      w.sidx);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    if ((e = gemm<false, true>(n * P1, C1, K1, Dense{w.x1c, K1}, Dense{p->wp + OP1, K1}, p->wp,
-                               EpiBiasRelu{w.a1, C1, p->wb + OB1}, 1, nullptr, s)) != cudaSuccess)
-        return e;
     if ((e = gemm<false, true>(n * P2, C2, K2, Im2col<C1, D1>{w.a1}, Dense{p->wp + OP2, K2}, p->wp,
                                EpiBiasRelu{w.a2, C2, p->wb + OB2}, 1, nullptr, s)) != cudaSuccess)
         return e;
@@ -910,7 +963,7 @@ cudaError_t colsum(const bf16* in, int rows, int cols, float* part, float* out, 
 // the batch's forward, loss, backward and weight gradients into p->g (no update)
 cudaError_t launch_gradients(fftdock_proposal* p, int B, const SampleSrc& src, const float* target, cudaStream_t s) {
     Work& w = p->wk;
-    cudaError_t e = launch_forward(p, B, src, s);
+    cudaError_t e = launch_forward(p, B, src, true, s);
     if (e != cudaSuccess) return e;
     float* g = p->g;
     head_kernel<<<(B + 7) / 8, THREADS, 0, s>>>(p->wb, w.h1, B, w.y, target, w.sidx, B, w.dy, w.dzf, p->loss);
@@ -1208,7 +1261,7 @@ int fftdock_proposal_predict_device(fftdock_proposal* p, int32_t lig, int32_t n,
     }
     for (int off = 0; off < n; off += PREDICT_CHUNK) {
         const int nc = std::min(PREDICT_CHUNK, n - off);
-        PK(launch_forward(p, nc, SampleSrc{2, nullptr, d_rot, n, off, lig, nullptr, 0}, s));
+        PK(launch_forward(p, nc, SampleSrc{2, nullptr, d_rot, n, off, lig, nullptr, 0}, false, s));
         head_kernel<<<(nc + 7) / 8, THREADS, 0, s>>>(p->wb, p->wk.h1, nc, d_out + off, nullptr, nullptr, nc, nullptr,
                                                      nullptr, nullptr);
         PK(cudaGetLastError());
