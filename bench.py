@@ -477,27 +477,27 @@ def run_ours(args):
     }
     if tensor:
         # executed tcgen05 work per pencil and 128-rotation group: K * W/8
-        # chunks of 6 MMAs (real and imaginary output x hi*hi, hi*lo, lo*hi)
-        # of 128 x 128 x 16; one of the three split products is the FP32
+        # chunks of 3 MMAs (hi*hi, hi*lo, lo*hi) of 128 rotations x real and
+        # imaginary outputs x 16; one of the three split products is the FP32
         # product being emulated
+        cols = 2 * ((n + 7) // 8 * 8) if n <= 128 else 512
         n_batches = math.ceil(n_rot / batch)
         groups_per_step = sum(math.ceil(min(batch, n_rot - b0) / 128) for b0 in range(0, n_rot, batch))
         nh = n * (n // 2 + 1)
-        flops_per_group = nh * k_terms * (info["window_w"] // 8) * 6 * (2.0 * 128 * 128 * 16)
+        flops_per_group = nh * k_terms * (info["window_w"] // 8) * 3 * (2.0 * 128 * cols * 16)
         flops_per_launch = flops_per_group * groups_per_step / n_batches
         executed = flops_per_launch / (avg_launch_ms / 1000.0) / 1e12
         peak, peak_kind = load_peaks("bf16_tflops_sustained")
         roofline = {"bound": "tensor", "achieved": executed, "peak": peak, "unit": "TFLOP/s",
-                    "frac": executed / peak, "traffic": None, "kernel": "pencil_tc",
+                    "frac": executed / peak, "traffic": None, "kernel": "pencil_tcp" if n <= 128 else "pencil_tc",
                     "peak_source": peak_kind + " sustained bf16 (the kernel runs inside a seconds-long step)",
                     "useful_achieved": executed / 3.0, "useful_frac": executed / 3.0 / peak,
-                    "flops_basis": "executed split-FP16 MMA work: N^2(N/2+1) pencils x K x W/8 chunks x 6 MMAs "
-                                   "of 128x128x16 per 128-rotation group (W = %d); useful = executed / 3 (the "
-                                   "hi*hi, hi*lo, lo*hi products emulate one FP32 product)" % info["window_w"],
-                    "limiter": "the CUDA-core producers of the MMA operands (entry walk, tile conversion "
-                               "and build: shared-memory and LSU traffic and its latency); the tensor pipe "
-                               "is busy about a third of the time, and halving the MMAs' shared-memory "
-                               "operand reads did not change the kernel's time",
+                    "flops_basis": "executed split-FP16 MMA work: N^2(N/2+1) pencils x K x W/8 chunks x 3 MMAs "
+                                   "of 128x%dx16 per 128-rotation group (W = %d); useful = executed / 3 (the "
+                                   "hi*hi, hi*lo, lo*hi products emulate one FP32 product)" % (cols, info["window_w"]),
+                    "limiter": "the SM's shared-memory data path (ncu: 92 % of its cycles busy with MMA operand "
+                               "reads, entry walk, tile conversion and build, and global accesses); the tensor "
+                               "pipe is busy 37 % of the time",
                     "kernel_share": share, "hbm": hbm}
     else:
         roofline = {"bound": "hbm", "achieved": pencil_gbs, "peak": peak_gbs, "unit": "GB/s",

@@ -84,7 +84,9 @@ enum {
  * where it is the faster form (cubic edges <= 128 and box grids with Nx <=
  * 256, FP32 spectra, an unweighted term set with at least 4 terms: at 64^3
  * with the single shape term, and at 144^3, the FFT form is faster), else FFT; a ligand whose window exceeds the tensor stage's shared
- * memory runs the FFT form.  The no-allocation scan always runs the FFT form;
+ * memory runs the FFT form, and so do a scan's last few rotations beside whole
+ * groups of 128, where the results are rescored in FP64 (not for correlation
+ * grids, candidates or queues).  The no-allocation scan always runs the FFT form;
  * fftdock_scan_pairs follows the same rule per grid edge. */
 enum {
     FFTDOCK_PENCIL_AUTO = 0,

@@ -8,17 +8,16 @@
 // spectrum product summed over terms, inverse x transform), plane stage
 // (inverse y transform, real inverse z transform, exact per-plane top 16),
 // finalize (merge, FP64 direct-space rescoring, sort, maxValCorr, unwrap per
-// axis) -- with every transform length a runtime value: one warp per line
-// runs a mixed-radix Stockham FFT (radices 4, 6, 2, 9, 3, 5, 7, 11, 13 in
-// that order of preference) out of shared memory with a twiddle table per
-// axis (even-length plane rows: two lines per warp, 16 lanes each).  The receptor's transforms
-// run the same line FFT in FP64.
+// axis) -- with every transform length a runtime value.  This file holds prep,
+// finalize and the launches; the stages are pencil_tcp.cuh / pencil_tc.cuh (tensor
+// form), pencil_lines.cuh through pencil_box*.cu (FFT form), plane_lines.cuh
+// through plane_box.cu, and receptor_fft.cu for the receptor's transforms.
 //
 // Layout (Hz = Nz/2 + 1, pencil p = ky Hz + kz, PP = Ny Hz rounded up to 32):
 //   spec  [K][Nx][PP]  float2  R^_t(kx, p) / V
 //   rgrid [K][V]       double  real-space receptor terms (FP64 rescoring)
-//   ent   [B][n_ent]   uint32  t << 24 | x << 16 | y << 8 | z, sorted by (t, x)
-//   offs  [B][K Nx+1]  int32   start of bin (t, x)
+//   ent   [B][n_ent]   uint32  t << 24 | x << 16 | y << 8 | z, sorted by (t, x, y mod qc)
+//   offs  [B][K Nx qc+1]  int32  start of bin (t, x, y mod qc)
 //   g2    [B][Nx][PP]  float2  per-x complex (ky, kz) planes
 //   cand  [B][Nx][16]          per-plane FP32 candidate pools
 #include <cuda_runtime.h>
@@ -40,7 +39,7 @@ constexpr int kBoxWarps = 8;  // lines (pencils, columns, rows) per CTA
 
 // ---------------------------------------------------------------------------
 // ligand prep: rotate (the reference's operation order, no FMA), toLogical
-// per axis, bins (t, x), stable sort (one CTA per rotation)
+// per axis, bins (t, x, y mod qc), stable sort (one CTA per rotation)
 // ---------------------------------------------------------------------------
 // ent_t (tensor form): the transposed entries of ligand_prep_kernel
 __global__ void __launch_bounds__(256) box_prep_kernel(const double* __restrict__ rot,

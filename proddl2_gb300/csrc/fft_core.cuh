@@ -1,7 +1,10 @@
 // Shared FFT building blocks for the correlation-scan kernels.
 //
-// Every 1-D transform of length N in this library is a two-pass Stockham
-// decomposition N = R1 * G executed by G warps, one line per lane:
+// In-register DFTs (packed two-lane FP32 arithmetic) for every line pass, and the
+// two-pass Stockham decomposition N = R1 * G of pencil_kernel (unweighted sets of
+// several terms on cubic edges; the other stages' in-place passes are in
+// pencil_lines.cuh, plane_lines.cuh and receptor_fft.cu), G warps, one line per
+// lane:
 //   pass 1: warp w holds the line's elements x = w + G*r (r < R1) in
 //           registers and does one radix-R1 DFT in registers;
 //   exchange through shared memory (one element per (position, lane));

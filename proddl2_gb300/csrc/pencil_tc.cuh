@@ -1,4 +1,6 @@
-// Tensor-core form of the pencil stage (tcgen05, sm_103a).
+// Tensor-core form of the pencil stage (tcgen05, sm_103a), one pencil per CTA: for
+// odd Ny, Nx above 128 and windows that do not fit pencil_tcp.cuh, which runs the
+// others over pencil pairs.
 //
 // For one pencil (ky, kz) and a group of 128 rotations r, the pencil kernel's
 // "forward x-FFT, conj(R^_t) product summed over terms, inverse x-FFT" is a

@@ -7,7 +7,7 @@
 //   rgrid [K][N^3]     double  real-space receptor terms (FP64 rescoring)
 //   ent   [B][n_ent]   uint32  per-rotation ligand entries t<<24|x<<16|y<<8|z,
 //                              sorted by (t, x, y mod qc), atom order inside a bin
-//   offs  [B][K*N+1]   int32   start of bin (t, x) at offs[t*N + x]
+//   offs  [B][K*N*qc+1]  int32  start of bin (t, x, y mod qc)
 //   g2    [B][N][PP]   float2  sum_t conj(R^_t) L^_t inverse-transformed
 //                              along x: one complex (ky, kz) plane per x
 //   cand  [B][N][KC]           per-plane FP32 candidate pools
