@@ -124,7 +124,7 @@ __device__ __forceinline__ int tap_source(int din, int oz, int oy, int ox, int t
 // summed in steps of 16 k in order whatever the tile.  Against one stage of 64 x 64
 // tiles (a step then waits for its loads): of a 256-sample training step, weight
 // gradients of conv3, conv2, conv1 91, 92, 87 -> 11, 13, 11 us, fc1 45 -> 7, conv3 63
-// -> 9; of 4,096 predictions, conv2 120 -> 72 us, conv3 66 -> 26.  gridDim.z > 1 splits K into
+// -> 9; of 4,096 predictions, conv3 66 -> 26 us.  gridDim.z > 1 splits K into
 // equal multiples of 32; each split hands its partial sums to the epilogue with
 // its index.
 // ---------------------------------------------------------------------------
@@ -419,20 +419,29 @@ __device__ void occupancy(const double* __restrict__ xyz, int n, double L, const
 }
 
 // one CTA per sample: occupancy -> x0 (BF16, in shared memory with a border of
-// zeros) -> a1[s * P1 + pos][C1], conv1 with bias and ReLU: each warp multiplies 64
-// positions' taps, gathered from x0 into the fragments, by the weights w1 [C1][K1]
-// (columns 27..31 zero); the sums' order is gemm_kernel's.  The descriptor ->
-// u[s][NA3..].  Training (x1c) also stores conv1's im2col rows x1c[s * P1 +
-// pos][tap] for the weight gradient: column 27 is 1 (the bias gradient comes out
-// there), 28..31 zero.  4,096 predictions: 134 MB of rows no longer written and
-// read, 67 + 93 us (this kernel and a GEMM) -> 64 us.
+// zeros) -> conv1 -> a1 in shared memory -> conv2 -> a2[s * P2 + pos][C2], each with
+// bias and ReLU and the order of sums of gemm_kernel (steps of 16 k; of conv2 a
+// step is a tap).  conv1: each warp multiplies 64 positions' taps, gathered from x0
+// into the fragments, by w1 [C1][K1] (columns 27..31 zero).  conv2: a warp takes 16
+// positions x 16 channels; ldmatrix gathers a tap's rows from a1, whose slots are
+// swizzled by y so that the eight rows of a matrix (x in steps of 2, two y) lie on
+// distinct banks, and the weights' fragments come through L1 (a copy in fragment
+// order: this kernel 103 -> 101 us, but the training step 2 % slower).  The descriptor ->
+// u[s][NA3..].  Training also stores a1 [s * P1 + pos][C1] and conv1's im2col rows
+// x1c[s * P1 + pos][tap] for the weight gradient: column 27 is 1 (the bias gradient
+// comes out there), 28..31 zero.  4,096 predictions, this kernel and what it
+// replaced: 67 (occupancy, rows) + 93 (conv1) + 71 us (conv2) -> 103 us.
 constexpr int GP = G0 + 2;
 __global__ void __launch_bounds__(THREADS) prep_kernel(Ligands lg, SampleSrc src, const bf16* __restrict__ w1,
-                                                       const bf16* __restrict__ b1, bf16* __restrict__ a1,
-                                                       bf16* __restrict__ x1c, bf16* __restrict__ u,
-                                                       int* __restrict__ sidx) {
-    __shared__ float occ[NX0];
-    __shared__ bf16 xp[GP * GP * GP];
+                                                       const bf16* __restrict__ b1, const bf16* __restrict__ w2,
+                                                       const bf16* __restrict__ b2, bf16* __restrict__ a1,
+                                                       bf16* __restrict__ x1c, bf16* __restrict__ a2,
+                                                       bf16* __restrict__ u, int* __restrict__ sidx) {
+    __shared__ __align__(16) float occ[NX0];             // then a1: [C1 / 8][P1] slots of 8 channels
+    __shared__ __align__(16) bf16 xp[GP * GP * GP];      // begins with 18 zeros
+    static_assert(sizeof(occ) == (size_t)P1 * C1 * sizeof(bf16), "a1 takes the occupancy's place");
+    bf16* a1s = reinterpret_cast<bf16*>(occ);
+    auto slot = [](int pos) { return pos ^ ((pos >> 4) & 1); };  // x ^ (y / 2 mod 2)
     __shared__ float rs[11];
     const int b = blockIdx.x;
     int idx, lig;
@@ -502,10 +511,44 @@ __global__ void __launch_bounds__(THREADS) prep_kernel(Ligands lg, SampleSrc src
 #pragma unroll
                 for (int h = 0; h < 2; ++h) {
                     const float v0 = acc[j][2 * h] + bias[j][0], v1 = acc[j][2 * h + 1] + bias[j][1];
-                    *reinterpret_cast<__nv_bfloat162*>(a1 + ((size_t)b * P1 + pos + 8 * h) * C1 + 8 * j + 2 * tig) =
-                        __halves2bfloat162(f2b(v0 > 0.f ? v0 : 0.f), f2b(v1 > 0.f ? v1 : 0.f));
+                    const __nv_bfloat162 v = __halves2bfloat162(f2b(v0 > 0.f ? v0 : 0.f), f2b(v1 > 0.f ? v1 : 0.f));
+                    *reinterpret_cast<__nv_bfloat162*>(a1s + (j * P1 + slot(pos + 8 * h)) * 8 + 2 * tig) = v;
+                    if (a1)
+                        *reinterpret_cast<__nv_bfloat162*>(a1 + ((size_t)b * P1 + pos + 8 * h) * C1 + 8 * j + 2 * tig) = v;
                 }
         }
+    }
+    __syncthreads();
+    {
+        const int w = threadIdx.x >> 5, l = threadIdx.x & 31, gid = l >> 2, tig = l & 3;
+        const int oz = w >> 1, n0 = 16 * (w & 1);  // 16 positions of one oz, 16 channels
+        // this lane's row and channel half of the four matrices
+        const int row = l & 15, hf = l >> 4;
+        const uint32_t base = (uint32_t)__cvta_generic_to_shared(a1s) + (uint32_t)hf * P1 * 16u;
+        const uint32_t zero = (uint32_t)__cvta_generic_to_shared(xp);
+        float acc[2][4] = {};
+#pragma unroll 3
+        for (int t = 0; t < 27; ++t) {
+            const int z = 2 * oz - 1 + t / 9, y = 2 * (row >> 2) - 1 + (t / 3) % 3, x = 2 * (row & 3) - 1 + t % 3;
+            const bool in = z >= 0 && y >= 0 && x >= 0;
+            uint32_t a[4];
+            ldmatrix4<false>(a, in ? base + 16u * (uint32_t)slot((z * D1 + y) * D1 + x) : zero);
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+                const bf16* wr = w2 + (n0 + 8 * j + gid) * K2 + 16 * t + 2 * tig;
+                const uint32_t wf[2] = {*reinterpret_cast<const uint32_t*>(wr), *reinterpret_cast<const uint32_t*>(wr + 8)};
+                mma_bf16(acc[j], a, wf);
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int n = n0 + 8 * j + 2 * tig;
+                const float v0 = acc[j][2 * h] + b2f(b2[n]), v1 = acc[j][2 * h + 1] + b2f(b2[n + 1]);
+                *reinterpret_cast<__nv_bfloat162*>(a2 + ((size_t)b * P2 + 16 * oz + gid + 8 * h) * C2 + n) =
+                    __halves2bfloat162(f2b(v0 > 0.f ? v0 : 0.f), f2b(v1 > 0.f ? v1 : 0.f));
+            }
     }
     if (!x1c) return;
     // rows of 32 taps as 4 groups of 8
@@ -711,7 +754,7 @@ struct Work {
     int cap = 0;
     bool grads = false;  // the backward buffers are allocated
     bf16* x1c = nullptr;  // [cap * P1][K1] (with grads)
-    bf16* a1 = nullptr;   // [cap * P1][C1]
+    bf16* a1 = nullptr;   // [cap * P1][C1] (with grads)
     bf16* a2 = nullptr;   // [cap * P2][C2]
     bf16* u = nullptr;    // [cap][NU]
     bf16* h1 = nullptr;   // [cap][HID]
@@ -868,7 +911,6 @@ int grow_work(fftdock_proposal* p, int cap, bool grads) {
     const bool gr = grads || w.grads;
     w.release();
     drop_graph(p);
-    PK(dalloc(&w.a1, (size_t)c * P1 * C1));
     PK(dalloc(&w.a2, (size_t)c * P2 * C2));
     PK(dalloc(&w.u, (size_t)c * NU));
     PK(dalloc(&w.h1, (size_t)c * HID));
@@ -876,6 +918,7 @@ int grow_work(fftdock_proposal* p, int cap, bool grads) {
     PK(dalloc(&w.y, (size_t)c));
     if (gr) {
         PK(dalloc(&w.x1c, (size_t)c * P1 * K1));
+        PK(dalloc(&w.a1, (size_t)c * P1 * C1));
         PK(dalloc(&w.dy, (size_t)c));
         PK(dalloc(&w.dzf, (size_t)c * HID));
         PK(dalloc(&w.dz3, (size_t)c * P3 * C3));
@@ -899,15 +942,13 @@ cudaError_t gemm_tiled(int M, int N, int K, const OpA& A, const OpB& B, const bf
     return cudaGetLastError();
 }
 
-// Tile of a GEMM: 64 rows and 32 or 64 columns where that fills the GPU twice over
-// (2 x 152 CTAs), else 32 x 32, which gives four times the CTAs.
+// Tile of a GEMM: 64 x 64 where that fills the GPU twice over (2 x 152 CTAs), else
+// 32 x 32, which gives four times the CTAs.
 template <bool AT, bool BT, class OpA, class OpB, class Epi>
 cudaError_t gemm_launch(int M, int N, int K, const OpA& A, const OpB& B, const bf16* any, int kc, int splits, Epi epi,
                         cudaStream_t s) {
     constexpr int kFill = 2 * 152;
     const int m64 = (M + 63) / 64 * splits;
-    if (N <= 32 && m64 >= kFill)
-        return gemm_tiled<64, 32, 32, 16, AT, BT>(M, N, K, A, B, any, kc, splits, epi, s);
     if (m64 * ((N + 63) / 64) >= kFill)
         return gemm_tiled<64, 64, 32, 32, AT, BT>(M, N, K, A, B, any, kc, splits, epi, s);
     return gemm_tiled<32, 32, 16, 16, AT, BT>(M, N, K, A, B, any, kc, splits, epi, s);
@@ -931,16 +972,13 @@ cudaError_t gemm(int M, int N, int K, const OpA& A, const OpB& B, const bf16* an
 }
 
 // forward of n samples (n <= work capacity): u, h1 and y in the work buffers,
-// with rows also conv1's im2col rows
+// with rows also a1 and conv1's im2col rows
 cudaError_t launch_forward(fftdock_proposal* p, int n, const SampleSrc& src, bool rows, cudaStream_t s) {
     Work& w = p->wk;
     cudaError_t e;
-    prep_kernel<<<n, THREADS, 0, s>>>(ligands(p), src, p->wp + OP1, p->wb + OB1, w.a1, rows ? w.x1c : nullptr, w.u,
-                                      w.sidx);
+    prep_kernel<<<n, THREADS, 0, s>>>(ligands(p), src, p->wp + OP1, p->wb + OB1, p->wp + OP2, p->wb + OB2,
+                                      rows ? w.a1 : nullptr, rows ? w.x1c : nullptr, w.a2, w.u, w.sidx);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    if ((e = gemm<false, true>(n * P2, C2, K2, Im2col<C1, D1>{w.a1}, Dense{p->wp + OP2, K2}, p->wp,
-                               EpiBiasRelu{w.a2, C2, p->wb + OB2}, 1, nullptr, s)) != cudaSuccess)
-        return e;
     if ((e = gemm<false, true>(n * P3, C3, K3, Im2col<C2, D2>{w.a2}, Dense{p->wp + OP3, K3}, p->wp,
                                EpiConv3{w.u, p->wb + OB3}, 1, nullptr, s)) != cudaSuccess)
         return e;
