@@ -292,16 +292,11 @@ size_t prep_smem_bytes(int nx, int K, int n_ent, int qc) {
     return ((size_t)K * nx * qc + 1) * sizeof(int32_t) + (size_t)n_ent * sizeof(uint32_t);
 }
 
-cudaError_t set_smem(const void* fn, size_t bytes) {
-    if (bytes <= kDynSmemNoOptIn) return cudaSuccess;
-    return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-}
-
 cudaError_t box_prep(const BatchArgs& a, cudaStream_t s) {
     const int nb = a.n_rot;
     if (nb <= 0) return cudaSuccess;
     const size_t sm = prep_smem_bytes(a.box.n[0], a.K, a.n_ent, a.classes());
-    cudaError_t e = set_smem((const void*)box_prep_kernel, sm);
+    cudaError_t e = allow_smem((const void*)box_prep_kernel, sm);
     if (e != cudaSuccess) return e;
     box_prep_kernel<<<nb, 256, sm, s>>>(a.rot, a.lig_xyz, a.lig_term, a.n_ent, a.K, a.box, a.ent, a.offs, a.status,
                                         a.lig_w32, a.lig_w32 ? a.ent4 : nullptr, a.ent_idx,
@@ -331,12 +326,12 @@ cudaError_t box_middle(const BatchArgs& a, cudaStream_t s) {
         if (a.tc_pair) {
             if ((e = launch_pencil_tcp<0>(a, nx, ny, nz, nullptr, bx, s)) != cudaSuccess) return e;
         } else if (tc_tiles(nx) == 1) {
-            if ((e = set_smem((const void*)pencil_tc_kernel<0, 1>, smt)) != cudaSuccess) return e;
+            if ((e = allow_smem((const void*)pencil_tc_kernel<0, 1>, smt)) != cudaSuccess) return e;
             pencil_tc_kernel<0, 1><<<gridt, TC_THREADS, smt, s>>>(a.circ, a.cscale, a.ent_t, a.tinfo, a.n_tc_terms,
                                                                  nullptr, a.g2t, a.n_pad, nb, a.x0, a.W, tg,
                                                                  a.tc_slots, a.tc_n_slots, bx, a.err);
         } else {
-            if ((e = set_smem((const void*)pencil_tc_kernel<0, 2>, smt)) != cudaSuccess) return e;
+            if ((e = allow_smem((const void*)pencil_tc_kernel<0, 2>, smt)) != cudaSuccess) return e;
             pencil_tc_kernel<0, 2><<<gridt, TC_THREADS, smt, s>>>(a.circ, a.cscale, a.ent_t, a.tinfo, a.n_tc_terms,
                                                                  nullptr, a.g2t, a.n_pad, nb, a.x0, a.W, tg,
                                                                  a.tc_slots, a.tc_n_slots, bx, a.err);

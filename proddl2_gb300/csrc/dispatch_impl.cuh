@@ -28,18 +28,13 @@ template <int N> struct SizeOpsImpl {
                (size_t)n_ent * sizeof(uint32_t);
     }
 
-    static cudaError_t set_smem(const void* fn, size_t bytes) {
-        if (bytes <= kDynSmemNoOptIn) return cudaSuccess;
-        return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-    }
-
     // the tensor pencil stage: one 128-row x tile up to 128, two up to 256
     static constexpr bool kHasTc = N <= 256;
 
 
     template <typename SpecT> static cudaError_t launch_pencil(const BatchArgs& a, int nb, cudaStream_t s) {
         const size_t sm2 = pencil_smem(a.K, a.n_ent);
-        cudaError_t e = set_smem((const void*)pencil_kernel<N, SpecT>, sm2);
+        cudaError_t e = allow_smem((const void*)pencil_kernel<N, SpecT>, sm2);
         if (e != cudaSuccess) return e;
         dim3 grid2(nb, a.PP / 32);
         pencil_kernel<N, SpecT><<<grid2, 32 * G, sm2, s>>>(static_cast<const SpecT*>(a.spec), a.ent, a.offs, a.tw32,
@@ -55,7 +50,7 @@ template <int N> struct SizeOpsImpl {
         const size_t st = pencil_stage_bytes(N, a.K, Q, a.n_ent, PAIRED);
         const int staged = sm + st <= kPencilMaxSmem ? 1 : 0;
         if (staged) sm += st;
-        cudaError_t e = set_smem((const void*)fn, sm);
+        cudaError_t e = allow_smem((const void*)fn, sm);
         if (e != cudaSuccess) return e;
         const dim3 grid(nb, pencil_grid_y(nb, (N / Q * H + 31) / 32));
         fn<<<grid, NT, sm, s>>>(static_cast<const SpecT*>(a.spec), a.ent, a.ent4, a.offs, a.tw32, a.tw32, a.tw32,
@@ -77,7 +72,7 @@ template <int N> struct SizeOpsImpl {
         if (nb <= 0) return cudaSuccess;
         const Geo geo = make_geo(a.h, N, N, N);
         const size_t sm1 = a.offs_stride(N) * sizeof(int32_t) + (size_t)a.n_ent * sizeof(uint32_t);
-        cudaError_t e = set_smem((const void*)ligand_prep_kernel<N>, sm1);
+        cudaError_t e = allow_smem((const void*)ligand_prep_kernel<N>, sm1);
         if (e != cudaSuccess) return e;
         ligand_prep_kernel<N><<<nb, 256, sm1, s>>>(a.rot, a.lig_xyz, a.lig_term, a.n_ent, a.K, geo, a.ent, a.offs,
                                                     a.status, a.lig_w32, a.lig_w32 ? a.ent4 : nullptr, a.ent_idx,
@@ -104,7 +99,7 @@ template <int N> struct SizeOpsImpl {
                     if (e != cudaSuccess) return e;
                 } else {
                     const size_t smt = tc_smem_bytes(N, a.W / 8, a.n_tc_terms);
-                    if ((e = set_smem((const void*)pencil_tc_kernel<N, MT>, smt)) != cudaSuccess) return e;
+                    if ((e = allow_smem((const void*)pencil_tc_kernel<N, MT>, smt)) != cudaSuccess) return e;
                     dim3 gridt(N * H, (nb + TC_ROT - 1) / TC_ROT);
                     const int tg = a.tc_group > 0 ? a.tc_group : FFTDOCK_TC_TERMS_PER_SUM_DEFAULT;
                     pencil_tc_kernel<N, MT><<<gridt, TC_THREADS, smt, s>>>(a.circ, a.cscale, a.ent_t, a.tinfo,

@@ -26,10 +26,6 @@
 
 namespace fftdock {
 
-// dynamic shared memory up to which a launch needs no opt-in: the 48 KB default
-// also holds a kernel's static arrays
-constexpr size_t kDynSmemNoOptIn = 40 * 1024;
-
 // ---------------------------------------------------------------------------
 // complex helpers (float2 / double2)
 // ---------------------------------------------------------------------------

@@ -402,6 +402,21 @@ int check_ready(fftdock_ctx* ctx) {
 
 namespace fftdock {
 
+cudaError_t allow_smem(const void* fn, size_t bytes) {
+    // no opt-in up to here: the default limit also holds a kernel's static arrays
+    constexpr size_t kDefault = 48 * 1024, kNoOptIn = 40 * 1024;
+    if (bytes <= kNoOptIn) return cudaSuccess;
+    static std::mutex m;
+    const std::lock_guard<std::mutex> lock(m);
+    // (the attribute is read, not remembered: 0.2 us, and right after a device
+    // reset too.  A default limit reads as 48 KB whatever the static arrays.)
+    cudaFuncAttributes fa;
+    const cudaError_t e = cudaFuncGetAttributes(&fa, fn);
+    const int want = (int)std::max(bytes, kDefault + 16);
+    if (e != cudaSuccess || fa.maxDynamicSharedSizeBytes >= want) return e;
+    return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, want);
+}
+
 namespace {
 __global__ void fill_u32_kernel(uint32_t* p, uint32_t v, size_t n) {
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;

@@ -303,6 +303,13 @@ inline int whole_groups(int n, int few) {
 // batch are in a.wide.corr; writes a.peaks / a.n_peaks
 cudaError_t wide_select_batch(const BatchArgs& a, int N, cudaStream_t s);
 
+// Lets `fn` be launched with `bytes` of dynamic shared memory on the current
+// device.  The limit belongs to the function on the device, and contexts of other
+// grids launch the same functions from other threads, so it is only ever raised
+// (a limit lowered between another thread's call and its launch refuses that
+// launch).
+cudaError_t allow_smem(const void* fn, size_t bytes);
+
 struct SizeOps {
     int n;
     bool has_tc;

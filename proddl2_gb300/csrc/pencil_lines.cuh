@@ -384,7 +384,7 @@ cudaError_t launch_box_pencil(const BatchArgs& a, const float2* twx, const float
     const size_t st = pencil_stage_bytes(nx, a.K, Q, a.n_ent, PAIRED);
     const int staged = sm + st <= kPencilMaxSmem ? 1 : 0;
     if (staged) sm += st;
-    cudaError_t e = cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    const cudaError_t e = allow_smem((const void*)fn, sm);
     if (e != cudaSuccess) return e;
     const dim3 grid(a.n_rot, pencil_grid_y(a.n_rot, ((ny / Q) * (nz / 2 + 1) + 31) / 32));
     fn<<<grid, NT, sm, s>>>(static_cast<const float2*>(a.spec), a.ent, a.ent4, a.offs, twx, twy, twz, rx, nx, ny, nz,

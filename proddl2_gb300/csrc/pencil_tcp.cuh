@@ -564,8 +564,7 @@ cudaError_t launch_pencil_tcp(const BatchArgs& a, int nx, int ny, int nz, const 
                               cudaStream_t s) {
     const int nc = a.W / 8, zc = N > 0 || tp_smem_box(nx, ny, nz, nc, a.n_tc_terms, 16) <= kTpMaxSmem ? 16 : 8;
     const size_t sm = N > 0 ? tp_smem_cubic(nx, nc, a.n_tc_terms) : tp_smem_box(nx, ny, nz, nc, a.n_tc_terms, zc);
-    cudaError_t e = cudaFuncSetAttribute((const void*)pencil_tcp_kernel<N>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)sm);
+    const cudaError_t e = allow_smem((const void*)pencil_tcp_kernel<N>, sm);
     if (e != cudaSuccess) return e;
     const int tg = a.tc_group > 0 ? a.tc_group : FFTDOCK_TC_TERMS_PER_SUM_DEFAULT;
     const dim3 grid(ny / 2 * (nz / 2 + 1), (a.n_rot + TC_ROT - 1) / TC_ROT);

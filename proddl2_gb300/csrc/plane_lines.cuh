@@ -761,10 +761,8 @@ __global__ void __launch_bounds__(NT, 768 / NT) plane_lines_kernel(
 // launch with the cluster shape of MODE (4 CTAs along x: the planes of a quad)
 template <int MODE, class... P, class... Args>
 cudaError_t launch_planes(void (*fn)(P...), dim3 grid, int threads, size_t sm, cudaStream_t s, Args... args) {
-    if (sm > kDynSmemNoOptIn) {
-        cudaError_t e = cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-        if (e != cudaSuccess) return e;
-    }
+    const cudaError_t e = allow_smem((const void*)fn, sm);
+    if (e != cudaSuccess) return e;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = dim3(threads);

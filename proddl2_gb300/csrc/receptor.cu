@@ -364,7 +364,7 @@ cudaError_t build_receptor_grids(const ReceptorGridArgs& a, cudaStream_t s) {
     if (lj) {
         const FieldReach fr = field_reach(a.geo, a.lj_cut);
         auto run = [&](auto fn, size_t sm) -> cudaError_t {
-            cudaError_t e2 = cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+            cudaError_t e2 = allow_smem((const void*)fn, sm);
             if (e2 != cudaSuccess) return e2;
             fn<<<run_blocks, 32 * kFieldWarps, sm, s>>>(a.xyz, a.lj_c, a.cells, a.bins, a.geo, fr, a.lj_cut * a.lj_cut,
                                                         md * md, a.rgrid);
@@ -387,9 +387,7 @@ cudaError_t build_receptor_grids(const ReceptorGridArgs& a, cudaStream_t s) {
         const FieldReach fr = field_reach(a.geo, a.ace_cut);
         const size_t sm = ((size_t)a.n_types * a.n_types + (size_t)a.n_types * 32 * kFieldWarps) * sizeof(double) +
                           kFieldWarps * field_warp_bytes<1>(fr.max_len);
-        if ((e = cudaFuncSetAttribute((const void*)ace_terms_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)sm)) != cudaSuccess)
-            return e;
+        if ((e = allow_smem((const void*)ace_terms_kernel, sm)) != cudaSuccess) return e;
         ace_terms_kernel<<<run_blocks, 32 * kFieldWarps, sm, s>>>(a.xyz, a.cells, a.bins, a.geo, fr,
                                                                   a.ace_cut * a.ace_cut, md * md, a.ace_b, a.ace_k,
                                                                   a.ace_a, a.flags, a.emat, a.n_types, a.rgrid);

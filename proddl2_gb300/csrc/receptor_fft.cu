@@ -221,10 +221,6 @@ __global__ void circ_exponent_kernel(const int* __restrict__ cmax, int nh, int8_
     cscale[p] = (int8_t)(e < -100 ? -100 : (e > 100 ? 100 : e));
 }
 
-template <class F> cudaError_t rf_set_smem(F* fn, size_t sm) {
-    return cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-}
-
 }  // namespace
 
 size_t receptor_fft_work(const int dims[3], int K) {
@@ -240,10 +236,10 @@ cudaError_t receptor_fft(const ReceptorFftArgs& a, cudaStream_t s) {
     const double2* twz = a.shared_tw ? a.tw64 : twy + ny;
     cudaError_t e;
     const long rows = (long)nx * ny;
-    if ((e = rf_set_smem(&rf_z_kernel, rf_smem(nz))) != cudaSuccess) return e;
+    if ((e = allow_smem((const void*)rf_z_kernel, rf_smem(nz))) != cudaSuccess) return e;
     rf_z_kernel<<<dim3((unsigned)((rows + 63) / 64), a.K), kRfThreads, rf_smem(nz), s>>>(a.rgrid, a.half, twz, pz, rows);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    if ((e = rf_set_smem(&rf_y_kernel, rf_smem(ny))) != cudaSuccess) return e;
+    if ((e = allow_smem((const void*)rf_y_kernel, rf_smem(ny))) != cudaSuccess) return e;
     rf_y_kernel<<<dim3((nx * hz + 31) / 32, a.K), kRfThreads, rf_smem(ny), s>>>(a.half, twy, py, nx, hz);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     // (the z launch left every value doubled)
@@ -251,11 +247,11 @@ cudaError_t receptor_fft(const ReceptorFftArgs& a, cudaStream_t s) {
     if (a.circ && (e = cudaMemsetAsync(a.cmax, 0, (size_t)nh * sizeof(int), s)) != cudaSuccess) return e;
     const dim3 gx((a.pp + 31) / 32, a.K);
     if (a.spec_bf16) {
-        if ((e = rf_set_smem(&rf_x_kernel<__nv_bfloat162>, rf_smem(nx))) != cudaSuccess) return e;
+        if ((e = allow_smem((const void*)rf_x_kernel<__nv_bfloat162>, rf_smem(nx))) != cudaSuccess) return e;
         rf_x_kernel<__nv_bfloat162><<<gx, kRfThreads, rf_smem(nx), s>>>(
             a.half, twx, px, nh, a.pp, ss, cs, static_cast<__nv_bfloat162*>(a.spec), a.circ, a.cmax);
     } else {
-        if ((e = rf_set_smem(&rf_x_kernel<float2>, rf_smem(nx))) != cudaSuccess) return e;
+        if ((e = allow_smem((const void*)rf_x_kernel<float2>, rf_smem(nx))) != cudaSuccess) return e;
         rf_x_kernel<float2><<<gx, kRfThreads, rf_smem(nx), s>>>(a.half, twx, px, nh, a.pp, ss, cs,
                                                                static_cast<float2*>(a.spec), a.circ, a.cmax);
     }

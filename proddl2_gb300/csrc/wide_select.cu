@@ -499,7 +499,7 @@ cudaError_t wide_select_batch(const BatchArgs& a, int N, cudaStream_t s) {
     wide_gather_kernel<<<grid_r, kPassThreads, 0, s>>>(w.corr, V, w.st, w.cand, w.cnt, mv, 1, rchunk);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     const size_t sm = (size_t)kWideMax * sizeof(u64);
-    e = cudaFuncSetAttribute((const void*)wide_finish_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    e = allow_smem((const void*)wide_finish_kernel, sm);
     if (e != cudaSuccess) return e;
     const int max_out = a.k_out < kMaxLeaders ? a.k_out : kMaxLeaders;
     wide_finish_kernel<<<nb, kFinishThreads, sm, s>>>(w.cand, w.cnt, a.ent, a.status, a.rgrid, a.n_ent, N, w.m,
