@@ -16,7 +16,8 @@
 // Layout (Hz = Nz/2 + 1, pencil p = ky Hz + kz, PP = Ny Hz rounded up to 32):
 //   spec  [K][Nx][PP]  float2  R^_t(kx, p) / V
 //   rgrid [K][V]       double  real-space receptor terms (FP64 rescoring)
-//   ent   [B][n_ent]   uint32  t << 24 | x << 16 | y << 8 | z, sorted by (t, x, y mod qc)
+//   ent   [B][n_ent]   uint32  t << 24 | x << 16 | y << 8 | z, sorted by (t, x, y mod qc);
+//                             tensor form: by (t, x), read by the rescoring only
 //   offs  [B][K Nx qc+1]  int32  start of bin (t, x, y mod qc)
 //   g2    [B][Nx][PP]  float2  per-x complex (ky, kz) planes
 //   cand  [B][Nx][16]          per-plane FP32 candidate pools
@@ -126,6 +127,7 @@ __global__ void __launch_bounds__(256) box_prep_kernel(const double* __restrict_
         ent_t[(((size_t)(q >> 7) * (n_pad >> 2) + (tinfo[ka] >> 2) + kk) * 128 + (q & 127)) * 4 + word] = m;
     }
     __syncthreads();
+    if (ka) pair_counts(cnt, nbins);
     if (tid < 32) {
         uint32_t* ent = ent_out + (size_t)q * n_ent;
         for (int base = 0; base < n_ent; base += 32) {
@@ -134,16 +136,14 @@ __global__ void __launch_bounds__(256) box_prep_kernel(const double* __restrict_
             const uint32_t key = act ? keys[i] : 0xffffffffu;
             const int bin = act ? (int)((key >> 24) * nx + ((key >> 16) & 255u)) * qc + (int)((key >> 8) & qm) : -1;
             const unsigned peers = __match_any_sync(0xffffffffu, bin);
-            const int rank = __popc(peers & ((1u << tid) - 1u));
             const int leader = __ffs(peers) - 1;
-            int dst = 0;
-            if (act) dst = cnt[bin] + rank;
+            const EntrySlot at = entry_slot(cnt, bin, peers, ka > 0, tid);
             __syncwarp();
-            if (act) ent[dst] = key;
+            if (act) ent[at.tx] = key;
             // [q / 128][row / 4][q % 128][row % 4], x relative to x0 (cells
             // outside the window at the dummy row W), as in ligand_prep_kernel
             if (act && ent_t) {
-                const size_t row = (size_t)(dst + __ldg(tpad + (key >> 24)));
+                const size_t row = (size_t)(at.bin + __ldg(tpad + (key >> 24)));
                 uint32_t xr = min(((key >> 16) - (uint32_t)x0) & 255u, (uint32_t)W);
                 if (ka) xr = 2 * xr + (xr < (uint32_t)W ? (key >> 8) & 1u : 0u);
                 ent_t[(((size_t)(q >> 7) * (n_pad >> 2) + (row >> 2)) * 128 + (q & 127)) * 4 + (row & 3)] =
@@ -154,9 +154,9 @@ __global__ void __launch_bounds__(256) box_prep_kernel(const double* __restrict_
                 // i + n_ent / 2 the same atom into term 1
                 const int half = n_ent >> 1;
                 if (i < half)
-                    ent4[(size_t)q * half + dst] =
+                    ent4[(size_t)q * half + at.bin] =
                         make_uint4(key, __float_as_uint(w_in[i]), __float_as_uint(w_in[i + half]), 0u);
-                idx_out[(size_t)q * n_ent + dst] = i;
+                idx_out[(size_t)q * n_ent + at.bin] = i;
             }
             if (act && tid == leader) cnt[bin] += __popc(peers);
             __syncwarp();

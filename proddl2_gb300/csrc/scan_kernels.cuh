@@ -7,6 +7,7 @@
 //   rgrid [K][N^3]     double  real-space receptor terms (FP64 rescoring)
 //   ent   [B][n_ent]   uint32  per-rotation ligand entries t<<24|x<<16|y<<8|z,
 //                              sorted by (t, x, y mod qc), atom order inside a bin
+//                              (tensor form: by (t, x), read by the rescoring only)
 //   offs  [B][K*N*qc+1]  int32  start of bin (t, x, y mod qc)
 //   g2    [B][N][PP]   float2  sum_t conj(R^_t) L^_t inverse-transformed
 //                              along x: one complex (ky, kz) plane per x
@@ -159,6 +160,38 @@ __device__ __forceinline__ void merge_lists(const float* sv, const int* si, int 
     }
 }
 
+// Where ligand prep's scatter puts the entry of lane `l` (bin -1: none): its
+// place `bin` among the sorted rows of the pencil stage, and `tx` in the order
+// (term, x), atom order inside, that the FP64 rescoring sums in whatever the
+// pencil form (a rotation's scores do not depend on the form that found its
+// cells).  They differ for pencil pairs only (`pairs`: bins (t, x, y mod 2)), whose
+// odd bins hold start << 16 | entries so far (pair_counts; at most 32768 entries).
+struct EntrySlot {
+    int bin, tx;
+};
+__device__ __forceinline__ EntrySlot entry_slot(const int32_t* cnt, int bin, unsigned peers, bool pairs, int l) {
+    const unsigned below = (1u << l) - 1u;
+    const int rank = __popc(peers & below);
+    const unsigned peers_tx = pairs ? __match_any_sync(0xffffffffu, bin >> 1) : peers;
+    EntrySlot s{0, 0};
+    if (bin >= 0) {
+        if (pairs) {
+            const int even = cnt[bin & ~1];
+            const uint32_t odd = (uint32_t)cnt[bin | 1];
+            const int n_odd = (int)(odd & 0xffffu);
+            s.bin = ((bin & 1) ? (int)(odd >> 16) + n_odd : even) + rank;
+            s.tx = even + n_odd + __popc(peers_tx & below);
+        } else {
+            s.bin = s.tx = cnt[bin] + rank;
+        }
+    }
+    return s;
+}
+__device__ __forceinline__ void pair_counts(int32_t* cnt, int nbins) {
+    for (int i = 2 * threadIdx.x + 1; i < nbins; i += 2 * blockDim.x) cnt[i] = (int32_t)((uint32_t)cnt[i] << 16);
+    __syncthreads();
+}
+
 // ---------------------------------------------------------------------------
 // K1: rotate + bin + stable sort of the ligand entries of one rotation
 // (MolForceRadial::projectLigand, docking_molforce.hpp:351-368, with
@@ -248,6 +281,7 @@ __global__ void __launch_bounds__(256) ligand_prep_kernel(
         ent_t[(((size_t)(q >> 7) * (n_pad >> 2) + (tinfo[ka] >> 2) + kk) * 128 + (q & 127)) * 4 + word] = m;
     }
     __syncthreads();
+    if (ka) pair_counts(cnt, nbins);
     // stable scatter by one warp: ranks within equal keys follow atom order
     if (tid < 32) {
         uint32_t* ent = ent_out + (size_t)q * n_ent;
@@ -257,12 +291,10 @@ __global__ void __launch_bounds__(256) ligand_prep_kernel(
             const uint32_t key = act ? keys[i] : 0xffffffffu;
             const int bin = act ? (int)((key >> 24) * N + ((key >> 16) & 255u)) * qc + (int)((key >> 8) & qm) : -1;
             const unsigned peers = __match_any_sync(0xffffffffu, bin);
-            const int rank = __popc(peers & ((1u << tid) - 1u));
             const int leader = __ffs(peers) - 1;
-            int dst = 0;
-            if (act) dst = cnt[bin] + rank;
+            const EntrySlot at = entry_slot(cnt, bin, peers, ka > 0, tid);
             __syncwarp();
-            if (act) ent[dst] = key;
+            if (act) ent[at.tx] = key;
             // transposed copy for the tensor pencil stage,
             // [q / 128][row / 4][q % 128][row % 4], with each term's rows
             // padded to a multiple of 8; the term is implied by the row and
@@ -271,7 +303,7 @@ __global__ void __launch_bounds__(256) ligand_prep_kernel(
             // | z, so that one multiply by kz << 16 | ky gives the phase; row =
             // x', or 2 x' + y mod 2 for pencil pairs
             if (act && ent_t) {
-                const size_t row = (size_t)(dst + __ldg(tpad + (key >> 24)));
+                const size_t row = (size_t)(at.bin + __ldg(tpad + (key >> 24)));
                 uint32_t xr = min(((key >> 16) - (uint32_t)x0) & 255u, (uint32_t)W);
                 if (ka) xr = 2 * xr + (xr < (uint32_t)W ? (key >> 8) & 1u : 0u);
                 ent_t[(((size_t)(q >> 7) * (n_pad >> 2) + (row >> 2)) * 128 + (q & 127)) * 4 + (row & 3)] =
@@ -282,9 +314,9 @@ __global__ void __launch_bounds__(256) ligand_prep_kernel(
                 // i + n_ent / 2 the same atom into term 1
                 const int half = n_ent >> 1;
                 if (i < half)
-                    ent4[(size_t)q * half + dst] =
+                    ent4[(size_t)q * half + at.bin] =
                         make_uint4(key, __float_as_uint(w_in[i]), __float_as_uint(w_in[i + half]), 0u);
-                idx_out[(size_t)q * n_ent + dst] = i;
+                idx_out[(size_t)q * n_ent + at.bin] = i;
             }
             if (act && tid == leader) cnt[bin] += __popc(peers);
             __syncwarp();
