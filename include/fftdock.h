@@ -84,9 +84,13 @@ enum {
  * where it is the faster form (cubic edges <= 128 and box grids with Nx <=
  * 256, FP32 spectra, an unweighted term set with at least 4 terms: at 64^3
  * with the single shape term, and at 144^3, the FFT form is faster), else FFT; a ligand whose window exceeds the tensor stage's shared
- * memory runs the FFT form, and so do a scan's last few rotations beside whole
- * groups of 128, where the results are rescored in FP64 (not for correlation
- * grids, candidates or queues).  The no-allocation scan always runs the FFT form;
+ * memory runs the FFT form.  So do, under AUTO, a scan's last few rotations beside
+ * whole groups of 128, where at most 8 peaks per rotation are kept (not for
+ * correlation grids, candidates or queues): scores are summed in one order in
+ * both forms, and the 16 cells rescored per rotation leave a margin, so a
+ * rotation's peaks do not depend on the number of rotations beside it unless
+ * more than 8 cells lie within the FP32 values' error of one another.  The
+ * no-allocation scan always runs the FFT form;
  * fftdock_scan_pairs follows the same rule per grid edge. */
 enum {
     FFTDOCK_PENCIL_AUTO = 0,
@@ -259,7 +263,7 @@ typedef struct fftdock_scan_info {
     int32_t n_terms;       /* K correlation terms */
     int32_t pencil_path;   /* FFTDOCK_PENCIL_FFT or FFTDOCK_PENCIL_TENSOR (the form that runs; under
                             * FFTDOCK_PENCIL_AUTO a scan's last few rotations beside whole groups of 128
-                            * run the FFT form, which is faster for them) */
+                            * run the FFT form, which is faster for them, for up to 8 peaks each) */
     int32_t rot_batch;     /* rotations per device batch */
     int32_t n_entries;     /* ligand entries (0 before fftdock_set_ligand) */
     int32_t window_x0;     /* tensor path: first x cell of the ligand window */

@@ -295,9 +295,11 @@ int run_batches(fftdock_ctx* ctx, int n_rot, const double* rot, int first_id, ff
     const int N = ctx->N, stride = ctx->cfg.peaks_per_rot;
     int rc;
     size_t ev = 0;
-    // (not where FP32 correlations are returned or order a queue: those are one
-    // form's for any number of rotations)
-    const bool fp64_only = !dbg && !pool_v && !a.wide.corr;
+    // (not where FP32 correlations are returned, order a queue or decide a peak:
+    // those are one form's for any number of rotations.  The forms' FP32 values
+    // choose the kKC cells rescored in FP64; over 58,000 rotations of five pairs
+    // the best 15 were always the same cells, the 16th differed in 35.)
+    const bool fp64_only = !dbg && !pool_v && !a.wide.corr && a.k_out <= fftdock::kKC / 2;
     const int few = a.use_tc && fp64_only && ctx->cfg.pencil_mode == FFTDOCK_PENCIL_AUTO
                         ? fftdock::few_rotations(ctx->dims)
                         : 0;

@@ -35,6 +35,32 @@ def test_parts_of_a_rotation_set(dims, part):
             assert np.array_equal(r.peaks, whole.peaks[a:a + part]), a
 
 
+# (grid edge, atoms, seed, rotations whose 16th FP32 candidate is a near tie that
+# the two pencil forms settle differently)
+NEAR_TIES = [(48, 700, 150, 2, [8269, 8881, 12454, 17719, 18861, 19352]),
+             (80, 1500, 400, 2, [2212, 2873, 4580, 5960]),
+             (128, 4000, 1500, 13, [726, 981, 986, 1433, 1913, 2290, 2467, 2703])]
+
+
+@pytest.mark.parametrize("edge,n_rec,n_lig,seed,ties", NEAR_TIES)
+@pytest.mark.parametrize("peaks", [8, 9, 16])
+def test_parts_with_many_peaks(edge, n_rec, n_lig, seed, ties, peaks):
+    # up to all 16 candidates of a rotation are kept: above 8 peaks the parts run
+    # the whole set's form
+    from proddl2_gb300 import FFTScan, ScanConfig, synth
+    pair = synth.make_pair(n_rec, n_lig, 20000 if edge == 48 else 9000 if edge == 80 else 4000, seed=seed)
+    rots = np.asarray(pair.rotations).reshape(-1, 9)
+    rots = np.concatenate([rots[ties], rots[:256 - len(ties)]])
+    with FFTScan(ScanConfig(grid_n=edge, term_set="shape_ace", ace_matrix=pair.ace, peaks_per_rot=peaks)) as s:
+        s.set_receptor(pair.receptor.xyz, pair.receptor.ace_type)
+        s.set_ligand(pair.ligand.xyz, pair.ligand.ace_type)
+        whole = s.scan(rots)
+        for a in range(0, len(rots), 16):
+            r = s.scan(rots[a:a + 16], first_rot_id=a)
+            assert np.array_equal(r.n_peaks, whole.n_peaks[a:a + 16])
+            assert np.array_equal(r.peaks, whole.peaks[a:a + 16]), a
+
+
 def test_pair_list_against_single_scans():
     from proddl2_gb300 import FFTScan, ScanConfig, synth
     from proddl2_gb300.pairs import PairInput, scan_pairs
