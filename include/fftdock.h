@@ -90,8 +90,8 @@ enum {
  * both forms, and the 16 cells rescored per rotation leave a margin, so a
  * rotation's peaks do not depend on the number of rotations beside it unless
  * more than 8 cells lie within the FP32 values' error of one another.  The
- * no-allocation scan always runs the FFT form;
- * fftdock_scan_pairs follows the same rule per grid edge. */
+ * no-allocation scan always runs the FFT form.  fftdock_scan_pairs chooses the
+ * form per grid edge by the same rule and keeps it for all rotations of a pair. */
 enum {
     FFTDOCK_PENCIL_AUTO = 0,
     FFTDOCK_PENCIL_FFT = 1,     /* FP32 x-FFTs on the CUDA cores */
