@@ -212,7 +212,9 @@ int fftdock_set_pair_lj(fftdock_ctx* ctx, int32_t n_rec, const double* rec_xyz, 
 /* Receptor atoms in the grid frame (grid centred on the origin).  Builds the
  * K receptor term grids and keeps their spectra on the device
  * (Worker::prepareReceptor, docking_app.hpp:406-415, and
- * FFTCorrelator::preprocessReceptor, docking_fft.hpp:614-618). */
+ * FFTCorrelator::preprocessReceptor, docking_fft.hpp:614-618).  The work memory
+ * of the set-up (half spectra of up to 512 MiB, 4 bytes per cell, the atoms) stays
+ * with the context for the next receptor. */
 int fftdock_set_receptor(fftdock_ctx* ctx, int32_t n, const double* xyz, const int32_t* type);
 
 /* Ligand atoms in the ligand frame (rotations are applied about the origin,

@@ -113,7 +113,7 @@ struct ReceptorFftArgs {
     int dims[3];
     int K;
     const double* rgrid;   // [K][V]
-    double2* half;         // [K][Nx][Ny][Hz] work (receptor_fft_work bytes)
+    double2* half;         // [terms in flight][Nx][Ny][Hz] work (receptor_fft_work bytes)
     const double2* tw64;   // e^{-2 pi i m / n}: [Nx | Ny | Nz], or one table of a cubic edge (shared_tw)
     bool shared_tw;
     void* spec;            // [K][Nx][pp] out, scaled 1 / V
