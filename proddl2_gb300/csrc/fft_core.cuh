@@ -22,6 +22,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <type_traits>
 #include <utility>
 
 namespace fftdock {
@@ -60,6 +61,10 @@ __device__ __forceinline__ float2 operator-(float2 a, float2 b) {
     asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(f2_bits(a)), "l"(f2_bits(b)));
     return bits_f2(r);
 }
+// the same as two scalar instructions, for kernels that schedule better so
+struct alignas(8) scalar2 { float x, y; };
+__device__ __forceinline__ scalar2 operator+(scalar2 a, scalar2 b) { return {a.x + b.x, a.y + b.y}; }
+__device__ __forceinline__ scalar2 operator-(scalar2 a, scalar2 b) { return {a.x - b.x, a.y - b.y}; }
 __device__ __forceinline__ double2 operator+(double2 a, double2 b) { return make_double2(a.x + b.x, a.y + b.y); }
 __device__ __forceinline__ double2 operator-(double2 a, double2 b) { return make_double2(a.x - b.x, a.y - b.y); }
 
@@ -86,7 +91,7 @@ template <typename C, typename S> __device__ __forceinline__ C cscale(C a, S s) 
 }
 // acc + a s for a real s
 template <typename C, typename S> __device__ __forceinline__ C cmadd(C acc, C a, S s) {
-    if constexpr (sizeof(C) == sizeof(float2)) {
+    if constexpr (std::is_same<C, float2>::value) {
         uint64_t r;
         asm("fma.rn.f32x2 %0, %1, %2, %3;"
             : "=l"(r)

@@ -339,6 +339,13 @@ __global__ void __launch_bounds__(256) ligand_prep_kernel(
 __device__ __forceinline__ float2 spec_load(const float2* p) { return __ldg(p); }
 __device__ __forceinline__ float2 spec_load(const __nv_bfloat162* p) { return __bfloat1622float2(*p); }
 
+// Complex type of its arithmetic: packed adds (float2) but for 128 with FP32
+// spectra, whose generated code is slower with them (80 registers either way):
+// pencil stage of 200 rotations of 18 terms, packed | scalar: 128^3 FP32 9.05 | 8.78 ms,
+// 128^3 BF16 8.55 | 8.76, 64^3 0.77 | 0.82, 96^3 4.30 | 4.60.
+template <int N, typename SpecT>
+using PencilC = std::conditional_t<N == 128 && std::is_same<SpecT, float2>::value, scalar2, float2>;
+
 template <int N, typename SpecT>
 __global__ void __launch_bounds__(32 * SizeTraits<N>::G, PencilTraits<N>::MINB) pencil_kernel(
     const SpecT* __restrict__ spec, const uint32_t* __restrict__ ent, const int32_t* __restrict__ offs,
@@ -347,13 +354,14 @@ __global__ void __launch_bounds__(32 * SizeTraits<N>::G, PencilTraits<N>::MINB) 
     constexpr int G = P::G, R1 = P::R1, H = N / 2 + 1;
     constexpr int PP = pencil_pitch(N);
     constexpr int BUFS = PencilTraits<N>::BUFS;
+    using C = PencilC<N, SpecT>;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    float2* xbuf = reinterpret_cast<float2*>(smem_raw);  // [BUFS][N][32]
-    float2* tws = xbuf + BUFS * N * 32;                  // [N]
+    C* xbuf = reinterpret_cast<C*>(smem_raw);  // [BUFS][N][32]
+    C* tws = xbuf + BUFS * N * 32;             // [N]
     // the phase table once per half-warp lane ([phase][16]): a warp's lanes
     // are consecutive pencils, whose phases for one entry step by its z, so
     // a single table would put lanes on the same banks whenever z is even
-    float2* twr = tws + N;                                  // [N][16]
+    float2* twr = reinterpret_cast<float2*>(tws + N);             // [N][16]
     uint32_t* ent_s = reinterpret_cast<uint32_t*>(twr + N * 16);  // [n_ent]
     int32_t* offs_s = reinterpret_cast<int32_t*>(ent_s + n_ent);  // [K*N+1]
 
@@ -368,7 +376,7 @@ __global__ void __launch_bounds__(32 * SizeTraits<N>::G, PencilTraits<N>::MINB) 
     // 144; the z ky term stays below bit 16), one multiply per phase
     const uint32_t kyz = (kz << 16) | ky;
 
-    for (int i = tid; i < N; i += blockDim.x) tws[i] = tw[i];
+    for (int i = tid; i < N; i += blockDim.x) tws[i] = C{tw[i].x, tw[i].y};
     for (int i = tid; i < N * 16; i += blockDim.x) twr[i] = tw[i >> 4];
     const int32_t* offs_g = offs + (size_t)q * (K * N + 1);
     for (int i = tid; i <= K * N; i += blockDim.x) offs_s[i] = offs_g[i];
@@ -379,17 +387,17 @@ __global__ void __launch_bounds__(32 * SizeTraits<N>::G, PencilTraits<N>::MINB) 
     }
     __syncthreads();
 
-    float2 S[R1];
+    C S[R1];
 #pragma unroll
-    for (int i = 0; i < R1; ++i) S[i] = make_float2(0.f, 0.f);
+    for (int i = 0; i < R1; ++i) S[i] = C{0.f, 0.f};
 
     for (int t = 0; t < K; ++t) {
-        float2 v[R1];
+        C v[R1];
 #pragma unroll
         for (int r = 0; r < R1; ++r) {
             const int x = w + G * r;
             const int b = offs_s[t * N + x], e = offs_s[t * N + x + 1];
-            float2 acc = make_float2(0.f, 0.f);
+            C acc{0.f, 0.f};
             for (int j = b; j < e; ++j) {
                 const uint32_t yz = (ent_s[j] * kyz) >> 16;
                 const unsigned ph = (N & (N - 1)) == 0 ? (yz & (unsigned)(N - 1)) : yz % (unsigned)N;
@@ -400,11 +408,11 @@ __global__ void __launch_bounds__(32 * SizeTraits<N>::G, PencilTraits<N>::MINB) 
             v[r] = acc;
         }
         dft<R1, -1>(v);
-        float2* buf = xbuf + (BUFS == 2 ? (t & 1) * N * 32 : 0);
+        C* buf = xbuf + (BUFS == 2 ? (t & 1) * N * 32 : 0);
 #pragma unroll
         for (int r = 0; r < R1; ++r) buf[(w * R1 + r) * 32 + l] = v[r];
         __syncthreads();
-        float2 F[R1];
+        C F[R1];
         line_pass2<P, -1, 1, 32>(buf, w, l, tws, F);
         if constexpr (BUFS == 1) __syncthreads();  // buf is rewritten by the next term
         const SpecT* sp = spec + (size_t)t * N * PP + p;
@@ -414,19 +422,19 @@ __global__ void __launch_bounds__(32 * SizeTraits<N>::G, PencilTraits<N>::MINB) 
             for (int r = 0; r < G; ++r) {
                 const int kx = w + G * i + R1 * r;
                 const float2 rv = spec_load(sp + (size_t)kx * PP);
-                const float2 f = F[i * G + r];
+                const C f = F[i * G + r];
                 S[i * G + r].x += f.x * rv.x + f.y * rv.y;
                 S[i * G + r].y += f.y * rv.x - f.x * rv.y;
             }
     }
-    float2 v[R1];
+    C v[R1];
     pass2_to_pass1_order<P>(S, v);
     dft<R1, +1>(v);
-    float2* buf = xbuf + (BUFS == 2 ? (K & 1) * N * 32 : 0);
+    C* buf = xbuf + (BUFS == 2 ? (K & 1) * N * 32 : 0);
 #pragma unroll
     for (int r = 0; r < R1; ++r) buf[(w * R1 + r) * 32 + l] = v[r];
     __syncthreads();
-    float2 out[R1];
+    C out[R1];
     line_pass2<P, +1, 1, 32>(buf, w, l, tws, out);
     float2* dst = g2 + (size_t)q * N * PP + p;
 #pragma unroll
@@ -434,7 +442,7 @@ __global__ void __launch_bounds__(32 * SizeTraits<N>::G, PencilTraits<N>::MINB) 
 #pragma unroll
         for (int r = 0; r < G; ++r) {
             const int x = w + G * i + R1 * r;
-            dst[(size_t)x * PP] = out[i * G + r];
+            dst[(size_t)x * PP] = make_float2(out[i * G + r].x, out[i * G + r].y);
         }
 }
 
