@@ -4,28 +4,40 @@
 
 namespace fftdock {
 
-constexpr int kThreads = 256;
+// Threads per plane: 256, or 64 on small planes, whose passes have too few
+// butterflies for more.  Plane stage, ms per 1024 rotations, 64 | 256 threads, from
+// planes and (/) from x-quads: 8 x 8 (8 cells along x) 0.26 | 0.42 / 0.15 | 0.30, 32 x 16 x 16
+// 0.46 | 0.91 / 0.29 | 0.66, 60^3 0.81 | 1.24 / 0.99 | 1.33, 72^3 1.49 | 1.73 / 1.58 | 1.66,
+// 80 x 78 x 78 1.94 | 2.02 / 1.99 | 1.86: the line lies between the last two.
+constexpr int kThreads = 256, kSmallThreads = 64;
+constexpr int kSmallPlane = 2700;  // complex values (ny hz)
 
-template <int MODE> static cudaError_t launch(const BatchArgs& a, const float2* twy, const float2* twz, cudaStream_t s) {
+static_assert(kSmallPlane <= 5400, "clusters start on larger planes");
+
+template <int MODE, int NT> static cudaError_t launch(const BatchArgs& a, const float2* twy, const float2* twz, cudaStream_t s) {
     const int nx = a.box.n[0], ny = a.box.n[1], nz = a.box.n[2];
     PlanePlan pl{};
     if (!plane_plan(ny, nz, pl)) return cudaErrorInvalidValue;
     constexpr bool quad = MODE != kPlanePlanes;
     const int nxp = quad ? (nx + 3) / 4 * 4 : nx;
-    return launch_planes<MODE>(&plane_lines_kernel<0, MODE, kThreads>, dim3(MODE == kPlaneQuadCluster ? nxp : nx, a.n_rot),
-                               kThreads, plane_lines_smem(ny, nz), s, (const float2*)(quad ? a.g2t : a.g2), twy, twz, pl,
+    return launch_planes<MODE>(&plane_lines_kernel<0, MODE, NT>, dim3(MODE == kPlaneQuadCluster ? nxp : nx, a.n_rot),
+                               NT, plane_lines_smem(ny, nz), s, (const float2*)(quad ? a.g2t : a.g2), twy, twz, pl,
                                nx, nxp, a.PP, a.cand_v, a.cand_i, a.dbg_corr);
 }
 
 cudaError_t box_plane(const BatchArgs& a, const float2* twy, const float2* twz, bool quad, cudaStream_t s) {
-    if (!quad) return launch<kPlanePlanes>(a, twy, twz, s);
-    return plane_quad_mode(a.box.n[1], a.box.n[2]) == kPlaneQuad ? launch<kPlaneQuad>(a, twy, twz, s)
-                                                                 : launch<kPlaneQuadCluster>(a, twy, twz, s);
+    const int ny = a.box.n[1], nz = a.box.n[2];
+    const bool small = ny * (nz / 2 + 1) <= kSmallPlane;
+    if (!quad)
+        return small ? launch<kPlanePlanes, kSmallThreads>(a, twy, twz, s) : launch<kPlanePlanes, kThreads>(a, twy, twz, s);
+    if (plane_quad_mode(ny, nz) == kPlaneQuadCluster) return launch<kPlaneQuadCluster, kThreads>(a, twy, twz, s);
+    return small ? launch<kPlaneQuad, kSmallThreads>(a, twy, twz, s) : launch<kPlaneQuad, kThreads>(a, twy, twz, s);
 }
 
 cudaError_t box_plane_load() {
     cudaFuncAttributes fa;
-    return cudaFuncGetAttributes(&fa, (const void*)plane_lines_kernel<0, kPlanePlanes, kThreads>);
+    const cudaError_t e = cudaFuncGetAttributes(&fa, (const void*)plane_lines_kernel<0, kPlanePlanes, kThreads>);
+    return e != cudaSuccess ? e : cudaFuncGetAttributes(&fa, (const void*)plane_lines_kernel<0, kPlanePlanes, kSmallThreads>);
 }
 
 }  // namespace fftdock
