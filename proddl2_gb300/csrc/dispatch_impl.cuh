@@ -28,6 +28,8 @@ template <int N> struct SizeOpsImpl {
                (size_t)n_ent * sizeof(uint32_t);
     }
 
+    static constexpr bool kLinesOneTerm = pencil_lines_one_term(N);
+
     // the tensor pencil stage: one 128-row x tile up to 128, two up to 256
     static constexpr bool kHasTc = N <= 256;
 
@@ -114,9 +116,10 @@ template <int N> struct SizeOpsImpl {
             if (a.lig_w32) {
                 if (a.spec_bf16) return cudaErrorNotSupported;  // weighted sets run with FP32 spectra
                 e = launch_pencil_lines<float2, true>(a, nb, s);
-            } else if (a.K == 1) {
-                e = a.spec_bf16 ? launch_pencil_lines<__nv_bfloat162, false>(a, nb, s)
-                                : launch_pencil_lines<float2, false>(a, nb, s);
+            } else if (a.K == 1 && kLinesOneTerm) {
+                if constexpr (kLinesOneTerm)
+                    e = a.spec_bf16 ? launch_pencil_lines<__nv_bfloat162, false>(a, nb, s)
+                                    : launch_pencil_lines<float2, false>(a, nb, s);
             } else {
                 e = a.spec_bf16 ? launch_pencil<__nv_bfloat162>(a, nb, s) : launch_pencil<float2>(a, nb, s);
             }
@@ -165,15 +168,17 @@ template <int N> struct SizeOpsImpl {
     static cudaError_t load_fft_form(int spec_bf16) {
         cudaFuncAttributes fa;
         cudaError_t e = cudaFuncGetAttributes(&fa, (const void*)ligand_prep_kernel<N>);
-        constexpr int C = pencil_ctas(N, false);
+        [[maybe_unused]] constexpr int C = pencil_ctas(N, false);
         if (e == cudaSuccess)
             e = spec_bf16 ? cudaFuncGetAttributes(&fa, (const void*)pencil_kernel<N, __nv_bfloat162>)
                           : cudaFuncGetAttributes(&fa, (const void*)pencil_kernel<N, float2>);
-        if (e == cudaSuccess)
-            e = spec_bf16 ? cudaFuncGetAttributes(
-                                &fa, (const void*)pencil_lines_kernel<N, __nv_bfloat162, false, kPencilQ, kPencilThreads, C>)
-                          : cudaFuncGetAttributes(&fa,
-                                                  (const void*)pencil_lines_kernel<N, float2, false, kPencilQ, kPencilThreads, C>);
+        if constexpr (kLinesOneTerm) {
+            if (e == cudaSuccess)
+                e = spec_bf16 ? cudaFuncGetAttributes(
+                                    &fa, (const void*)pencil_lines_kernel<N, __nv_bfloat162, false, kPencilQ, kPencilThreads, C>)
+                              : cudaFuncGetAttributes(&fa,
+                                                      (const void*)pencil_lines_kernel<N, float2, false, kPencilQ, kPencilThreads, C>);
+        }
         if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, (const void*)plane_lines_kernel<N, kPlanePlanes, plane_threads(N, false)>);
         if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, (const void*)finalize_kernel<N>);
         return e;

@@ -784,7 +784,7 @@ int fftdock_create(const fftdock_config* cfg_in, fftdock_ctx** out) {
     ctx->G = group_size(ctx->B);
     const bool paired = c.term_set == FFTDOCK_TERMS_LJ_COMP;
     ctx->qc = ctx->box ? fftdock::box_pencil_classes(dims, ctx->K, paired)
-                       : fftdock::cubic_pencil_classes(ctx->K, paired);
+                       : fftdock::cubic_pencil_classes(dims[0], ctx->K, paired);
     // centred geometry exactly as UniformCubicGeometry(step, logicalSize)
     const double h = c.grid_step;
     const double s_size = h + h * (double)(N - 1);

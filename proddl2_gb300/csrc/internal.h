@@ -348,8 +348,8 @@ bool tc_pairs_fit(const int dims[3], bool box, int K, int n_ent, int n_chunks, i
 int box_pencil_classes(const int dims[3], int K, bool paired);
 cudaError_t box_pencil(const BatchArgs& a, const float2* twx, const float2* twy, const float2* twz, cudaStream_t s);
 cudaError_t box_pencil_load();
-// the same classes on a cubic edge (K terms; paired: ljComp)
-int cubic_pencil_classes(int K, bool paired);
+// the same classes on the cubic edge n (K terms; paired: ljComp)
+int cubic_pencil_classes(int n, int K, bool paired);
 
 // plane stage of a batch on a box grid (quad: from the tensor stage's x-quads)
 cudaError_t box_plane(const BatchArgs& a, const float2* twy, const float2* twz, bool quad, cudaStream_t s);

@@ -3,7 +3,9 @@
 
 namespace fftdock {
 
-int cubic_pencil_classes(int K, bool paired) { return K == 1 || paired ? kPencilQ : 1; }
+int cubic_pencil_classes(int n, int K, bool paired) {
+    return paired || (K == 1 && pencil_lines_one_term(n)) ? kPencilQ : 1;
+}
 
 const SizeOps* size_ops_small(int n) {
     switch (n) {

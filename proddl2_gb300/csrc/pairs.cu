@@ -207,7 +207,7 @@ int alloc_work(Run& r, Work& w, const SizeData& sd, int B) {
     const int dims[3] = {N, N, N};
     PCK(dalloc(&w.half, fftdock::receptor_fft_work(dims, K) / sizeof(double2)));
     PCK(dalloc(&w.ent, (size_t)B * sd.max_lig));
-    PCK(dalloc(&w.offs, (size_t)B * (K * N * fftdock::cubic_pencil_classes(K, false) + 1)));
+    PCK(dalloc(&w.offs, (size_t)B * (K * N * fftdock::cubic_pencil_classes(N, K, false) + 1)));
     PCK(dalloc(&w.g2, (size_t)B * N * sd.PP));
     PCK(dalloc(&w.cand_v, (size_t)B * N * kKC));
     PCK(dalloc(&w.cand_i, (size_t)B * N * kKC));
@@ -299,7 +299,7 @@ cudaError_t enqueue_pair(Run& r, const fftdock_pair& p, int i, Work& w, const Si
     a.center0 = sd.center0;
     a.ent = w.ent;
     a.offs = w.offs;
-    a.qc = fftdock::cubic_pencil_classes(r.K, false);
+    a.qc = fftdock::cubic_pencil_classes(N, r.K, false);
     a.g2 = w.g2;
     a.cand_v = w.cand_v;
     a.cand_i = w.cand_i;

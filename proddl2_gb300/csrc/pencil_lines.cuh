@@ -73,6 +73,11 @@ template <int N> constexpr LineRadices fixed_pencil_radices() {
     return r;
 }
 
+// One unweighted term on a cubic edge: from 24 on.  16^3 has three tiles of 32 pencils,
+// which leave most of the warps idle: pencil stage of 4000 rotations 0.51 ms, with
+// pencil_kernel 0.45; 24^3 0.58 and 0.63.
+constexpr bool pencil_lines_one_term(int n) { return n > 16; }
+
 // cubic edges: classes y mod Q (four classes leave too few CTAs per SM: shape
 // at 64^3 0.62 against 0.52 ms per 1000 rotations) and resident CTAs
 constexpr int kPencilQ = 2;

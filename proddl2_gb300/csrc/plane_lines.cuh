@@ -651,7 +651,23 @@ __global__ void __launch_bounds__(NT, 768 / NT) plane_lines_kernel(
             if (at < kPlaneCand) { cand_sv[at] = v; cand_si[at] = off; }
         }
     };
-    unsigned qual = __ballot_sync(0xffffffffu, bmin <= bound);
+    // (single-warp CTAs, 16^3: half of the threads qualify, so each offers its own
+    // cells; 4000 rotations 0.77 -> 0.54 ms)
+    if constexpr (NT == 32) {
+        for (int it = tid; bmin <= bound && it < zitems; it += NT) {
+            const int b = div_by(it, nrow, P.m_row);
+            const int line = it - b * nrow;
+            int o0, o1;
+            offs(line, o0, o1);
+            for (int r = 0; r < zl; ++r) {
+                const float2 o = plane[line * lstride + b * zl + r];
+                const int f = (zdigits(b) + r * zstep) * fmul;
+                offer(o.x, o0 + f);
+                if (even || o1 >= 0) offer(o.y, o1 + f);
+            }
+        }
+    }
+    unsigned qual = NT == 32 ? 0u : __ballot_sync(0xffffffffu, bmin <= bound);
     while (qual) {
         const int it0 = w * 32 + __ffs(qual) - 1;
         qual &= qual - 1u;
