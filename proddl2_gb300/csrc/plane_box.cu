@@ -5,13 +5,14 @@
 namespace fftdock {
 
 // Threads per plane: 256, or 64 on small planes, whose passes have too few
-// butterflies for more.  Plane stage, ms per 1024 rotations, 64 | 256 threads, from
-// planes and (/) from x-quads: 8 x 8 (8 cells along x) 0.26 | 0.42 / 0.15 | 0.30, 32 x 16 x 16
-// 0.46 | 0.91 / 0.29 | 0.66, 60^3 0.81 | 1.24 / 0.99 | 1.33, 72^3 1.49 | 1.73 / 1.58 | 1.66,
-// 80 x 78 x 78 1.94 | 2.02 / 1.99 | 1.86: the line lies between the last two.
+// butterflies for more.  Plane stage, ms per 1000 rotations, 64 | 256 threads, from
+// planes and (/) from x-quads: 8^3 0.26 | 0.42 / 0.15 | 0.29, 12 x 13 x 26 0.46 | 0.70 /
+// 0.30 | 0.60, 12 x 24 x 26 0.33 | 0.49 / 0.21 | 0.42.  A lone rotation takes the same
+// time up to about 400 values, then longer the longer the lines: 64 x 8 and 32 x 30
+// 14 | 12 and 16 | 14 us, 169 x 26 51 | 14 us, which loses with 1000 rotations too
+// (1.18 | 0.69 ms).
 constexpr int kThreads = 256, kSmallThreads = 64;
-constexpr int kSmallPlane = 2700;  // complex values (ny hz)
-
+constexpr int kSmallPlane = 400;  // complex values (ny hz)
 static_assert(kSmallPlane <= 5400, "clusters start on larger planes");
 
 template <int MODE, int NT> static cudaError_t launch(const BatchArgs& a, const float2* twy, const float2* twz, cudaStream_t s) {

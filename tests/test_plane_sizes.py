@@ -8,7 +8,8 @@ import pytest
 
 pytestmark = pytest.mark.gpu
 
-DIMS = [(8, 8, 8), (9, 8, 9), (16, 16, 16), (8, 72, 72), (8, 78, 70), (10, 75, 70), (9, 75, 77), (24, 24, 24)]
+DIMS = [(8, 8, 8), (9, 8, 9), (16, 16, 16), (8, 20, 36), (8, 22, 36), (10, 20, 39), (9, 21, 39), (8, 72, 72), (8, 78, 70),
+        (10, 75, 70), (9, 75, 77), (24, 24, 24)]
 
 
 @pytest.mark.parametrize("mode", ["fft", "tensor"])
