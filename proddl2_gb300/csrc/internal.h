@@ -281,10 +281,11 @@ cudaError_t tc_slot_count(int* n_slots);
 // spectra, an unweighted term set with at least kTcMinTerms terms (at 64^3
 // with the single shape term the FFT form measured faster)
 constexpr int kTcMinTerms = 4;
-// Under AUTO with the tensor form selected, up to this many rotations (a call's
-// last rotations after whole groups of 128, or a whole call) run the FFT form:
+// Under AUTO with the tensor form selected and up to 8 peaks per rotation, up to
+// this many rotations (a call's last rotations after whole groups of 128, or a
+// whole call) run the FFT form:
 // the tensor stage costs a whole group's time for any part of one, the FFT form
-// a rotation's time each.  Pencil stage at 19 terms, FFT / tensor, GB300:
+// a rotation's time each.  Pencil stage at 18 terms, FFT / tensor, GB300:
 // 48^3 8 rotations 0.028 / 0.149 ms, 32: 0.065 / 0.149; 96^3 32: 0.60 / 0.93, 48:
 // 0.87 / 0.94; 112^3 16: 0.81 / 1.50, 32: 1.55 / 1.50; 128^3 16: 0.72 / 1.91; box
 // 50x44x36 16: 0.073 / 0.088, 32: 0.107 / 0.088; box 112x120x126 16: 0.92 / 1.96,

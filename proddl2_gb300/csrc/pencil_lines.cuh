@@ -20,9 +20,10 @@
 // the first inverse pass work on the same block of positions without leaving
 // registers, and the last inverse pass writes global memory.
 //
-// Bound: instruction issue (half the slots at 128^3 ljComp: 45 K warp
-// instructions per 64 pencils, about half of them the walk) and the barriers
-// between its phases.  Against one pencil per lane with register-resident x
+// Bound: latency of the phase lookups and transforms with 16 warps per SM.  At
+// 128^3 ljComp they issue in 53 % of the slots (38 K warp instructions per 64 pencils,
+// about half of them the walk), the L1 data path is 59 % busy, the FMA pipe 31 %.
+// Against one pencil per lane with register-resident x
 // transforms (cubic: pencil_kernel) and one warp per pencil with segmented
 // scans (box grids), pencil stage: ljComp 128^3, 1500 atoms 26.9 -> 16.0 ms per
 // 2000 rotations; ljComp 90 x 96 x 100, 800 atoms 47.6 -> 5.4 ms per 1000; shape

@@ -32,9 +32,11 @@
 // Shared memory bounds the window (40 cells at Nx = 128); larger ligands, odd Ny
 // and Nx > 128 run pencil_tc_kernel.  All waits are bounded.
 //
-// Measured (GB300, 19 terms, ms per 1000 rotations, one pencil at a time -> pairs):
-// 32^3 0.55 -> 0.39, 48^3 1.65 -> 1.21, 64^3 3.20 -> 2.44, 96^3 9.3 -> 7.9, 112^3 14.8
-// -> 12.9, 128^3 20.0 -> 17.7.  Bound at 128^3 by shared-memory bandwidth: per term
+// Measured (GB300, 18 terms, ms per 1000 rotations, one pencil at a time -> pairs,
+// with the ligand's atoms and window): 32^3 0.88 -> 0.59 (60, 16), 48^3 2.19 -> 1.59
+// (150, 24), 64^3 3.79 -> 2.73 (300, 24), 80^3 6.59 -> 5.51 (400, 24), 96^3 11.6 -> 9.5
+// (700, 32), 112^3 16.9 -> 14.0 (1000, 32), 128^3 24.9 -> 20.6 (1500, 40), box 112 x
+// 120 x 126 25.9 -> 20.8 (1500, 40).  Bound at 128^3 by shared-memory bandwidth: per term
 // the MMAs read 2,880 wavefronts of operands, walk, conversion and circulant tiles
 // take about 3,900 and global accesses (entries, slots, output) share the same
 // path: 92 % of its cycles busy, tensor pipe 37 %.
@@ -52,8 +54,6 @@ static_assert(256 * TP_MAX_CHUNKS <= 3 * TP_CONV && 4 * ((128 + 8 * TP_MAX_CHUNK
               "conversion tasks and circulant rows per thread");
 
 __host__ __device__ constexpr int tp_groups(int nx8, int n_chunks) { return (nx8 + 8 * n_chunks - 8) / 4; }
-// copies of the box grids' z phase table (lanes of a half-warp; 16: no bank is
-// shared, 8: two lanes share one)
 constexpr size_t tp_smem_core(int nx, int n_chunks, int n_terms) {
     const int nx8 = (nx + 7) / 8 * 8;
     return (size_t)2 * n_chunks * TC_FCHUNK + (size_t)(16 * n_chunks + 1) * 1024 +
@@ -61,6 +61,8 @@ constexpr size_t tp_smem_core(int nx, int n_chunks, int n_terms) {
            (size_t)((2 * n_terms + 1) * 4 + 15) / 16 * 16;
 }
 constexpr size_t tp_smem_cubic(int n, int n_chunks, int n_terms) { return tp_smem_core(n, n_chunks, n_terms) + (size_t)n * 128; }
+// z_copies: copies of the z phase table (lanes of a half-warp; 16: no bank is
+// shared, 8: two lanes share one)
 constexpr size_t tp_smem_box(int nx, int ny, int nz, int n_chunks, int n_terms, int z_copies) {
     return tp_smem_core(nx, n_chunks, n_terms) + (size_t)ny * 128 + (size_t)nz * 8 * z_copies;
 }
@@ -477,8 +479,6 @@ __global__ void __launch_bounds__(TP_THREADS, 1) pencil_tcp_kernel(
                 }
             }
         };
-        // before a group of terms restarts the accumulator: its sum goes to the
-        // slot (every thread orders its tensor-memory loads after its own wait)
         load_c(0);
         for (int k = 0; k < Ka; ++k) {
             load_mask(tid - 32, k);

@@ -34,15 +34,18 @@
 //   distributed shared memory (kPlaneQuad, kPlaneQuadCluster).
 // Odd nz: two rows a, b travel as one complex line a + i b of nz points.
 //
-// Bound: instruction issue and the six shared-memory passes (the plane's
-// bytes move at 2.5 TB/s at 128^3).  Against the kernels it replaced -- on
+// Bound: latency between the barriers of the passes.  At 128^3 24 warps per SM
+// issue in 49 % of the slots from planes and 34 % from x-quads (16 K warp
+// instructions per plane; stalls at barriers, the clusters' among them, and on the
+// first pass's loads), the L1 data path is 66 % and 53 % busy, and the plane's bytes
+// move at 2.4 and 2.2 TB/s.  Against the kernels it replaced -- on
 // cubic edges a two-pass transform with its lines spread over warps (exchange
 // barriers in every pass, (value, offset) minima, one re-read of all cells),
 // on box grids one warp per line through two buffers -- in ms per 1000
 // rotations, planes | x-quads (shape + 18 terms): 48^3 0.46 -> 0.31 | 0.82 ->
 // 0.31, 64^3 0.76 -> 0.51 | 0.99 -> 0.56, 80^3 3.21 -> 1.12 | 3.65 -> 1.01, 96^3
-// 3.47 -> 1.60 | 4.11 -> 1.58, 112^3 7.91 -> 2.35 | 8.57 -> 2.69, 128^3 4.80 ->
-// 3.42 | 5.73 -> 3.87, 144^3 11.6 -> 5.8 | 15.4 -> 6.4; 90 x 96 x 100 14.9 -> 2.9 |,
+// 3.47 -> 1.60 | 4.11 -> 1.58, 112^3 7.91 -> 2.35 | 8.57 -> 2.69, 128^3 4.98 ->
+// 3.53 | 5.70 -> 3.93, 144^3 11.6 -> 5.8 | 15.4 -> 6.4; 90 x 96 x 100 14.9 -> 2.9 |,
 // 112 x 120 x 126 | 20.0 -> 4.5.
 #pragma once
 

@@ -26,7 +26,7 @@ namespace fftdock {
 
 constexpr int KC = 16;  // FP32 candidates kept per plane / per rotation
 
-// Warps per line transform along x (and of the receptor's transforms): G*G | N.
+// Warps per line transform of pencil_kernel: G*G | N.
 template <int N> struct SizeTraits;
 template <> struct SizeTraits<16> { static constexpr int G = 4; };
 template <> struct SizeTraits<24> { static constexpr int G = 2; };
