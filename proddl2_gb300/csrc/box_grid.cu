@@ -128,16 +128,15 @@ __global__ void __launch_bounds__(256) box_prep_kernel(const double* __restrict_
     }
     __syncthreads();
     if (ka) pair_counts(cnt, nbins);
-    if (tid < 32) {
+    auto scatter = [&](auto pairs) {
         uint32_t* ent = ent_out + (size_t)q * n_ent;
         for (int base = 0; base < n_ent; base += 32) {
             const int i = base + tid;
             const bool act = i < n_ent;
             const uint32_t key = act ? keys[i] : 0xffffffffu;
             const int bin = act ? (int)((key >> 24) * nx + ((key >> 16) & 255u)) * qc + (int)((key >> 8) & qm) : -1;
-            const unsigned peers = __match_any_sync(0xffffffffu, bin);
-            const int leader = __ffs(peers) - 1;
-            const EntrySlot at = entry_slot(cnt, bin, peers, ka > 0, tid);
+            const EntrySlot at = entry_slot<decltype(pairs)::value>(cnt, bin, tid);
+            const int leader = __ffs(at.peers) - 1;
             __syncwarp();
             if (act) ent[at.tx] = key;
             // [q / 128][row / 4][q % 128][row % 4], x relative to x0 (cells
@@ -145,7 +144,7 @@ __global__ void __launch_bounds__(256) box_prep_kernel(const double* __restrict_
             if (act && ent_t) {
                 const size_t row = (size_t)(at.bin + __ldg(tpad + (key >> 24)));
                 uint32_t xr = min(((key >> 16) - (uint32_t)x0) & 255u, (uint32_t)W);
-                if (ka) xr = 2 * xr + (xr < (uint32_t)W ? (key >> 8) & 1u : 0u);
+                if (decltype(pairs)::value) xr = 2 * xr + (xr < (uint32_t)W ? (key >> 8) & 1u : 0u);
                 ent_t[(((size_t)(q >> 7) * (n_pad >> 2) + (row >> 2)) * 128 + (q & 127)) * 4 + (row & 3)] =
                     (xr << 24) | (((key >> 8) & 255u) << 16) | (key & 255u);
             }
@@ -158,9 +157,13 @@ __global__ void __launch_bounds__(256) box_prep_kernel(const double* __restrict_
                         make_uint4(key, __float_as_uint(w_in[i]), __float_as_uint(w_in[i + half]), 0u);
                 idx_out[(size_t)q * n_ent + at.bin] = i;
             }
-            if (act && tid == leader) cnt[bin] += __popc(peers);
+            if (act && tid == leader) cnt[bin] += __popc(at.peers);
             __syncwarp();
         }
+    };
+    if (tid < 32) {
+        if (ka) scatter(std::true_type{});
+        else scatter(std::false_type{});
     }
     if (tid == 0) status[q] = bad;
 }

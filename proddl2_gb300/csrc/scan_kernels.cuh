@@ -164,18 +164,24 @@ __device__ __forceinline__ void merge_lists(const float* sv, const int* si, int 
 // place `bin` among the sorted rows of the pencil stage, and `tx` in the order
 // (term, x), atom order inside, that the FP64 rescoring sums in whatever the
 // pencil form (a rotation's scores do not depend on the form that found its
-// cells).  They differ for pencil pairs only (`pairs`: bins (t, x, y mod 2)), whose
+// cells).  They differ for pencil pairs only (PAIRS: bins (t, x, y mod 2)), whose
 // odd bins hold start << 16 | entries so far (pair_counts; at most 32768 entries).
+// peers: the lanes of the same bin.
 struct EntrySlot {
     int bin, tx;
+    unsigned peers;
 };
-__device__ __forceinline__ EntrySlot entry_slot(const int32_t* cnt, int bin, unsigned peers, bool pairs, int l) {
+template <bool PAIRS> __device__ __forceinline__ EntrySlot entry_slot(const int32_t* cnt, int bin, int l) {
     const unsigned below = (1u << l) - 1u;
-    const int rank = __popc(peers & below);
-    const unsigned peers_tx = pairs ? __match_any_sync(0xffffffffu, bin >> 1) : peers;
-    EntrySlot s{0, 0};
+    const unsigned peers_tx = __match_any_sync(0xffffffffu, PAIRS ? bin >> 1 : bin);
+    EntrySlot s{0, 0, peers_tx};
+    if constexpr (PAIRS) {
+        const unsigned odd_lanes = __ballot_sync(0xffffffffu, bin & 1);
+        s.peers &= (bin & 1) ? odd_lanes : ~odd_lanes;
+    }
+    const int rank = __popc(s.peers & below);
     if (bin >= 0) {
-        if (pairs) {
+        if constexpr (PAIRS) {
             const int even = cnt[bin & ~1];
             const uint32_t odd = (uint32_t)cnt[bin | 1];
             const int n_odd = (int)(odd & 0xffffu);
@@ -283,16 +289,15 @@ __global__ void __launch_bounds__(256) ligand_prep_kernel(
     __syncthreads();
     if (ka) pair_counts(cnt, nbins);
     // stable scatter by one warp: ranks within equal keys follow atom order
-    if (tid < 32) {
+    auto scatter = [&](auto pairs) {
         uint32_t* ent = ent_out + (size_t)q * n_ent;
         for (int base = 0; base < n_ent; base += 32) {
             const int i = base + tid;
             const bool act = i < n_ent;
             const uint32_t key = act ? keys[i] : 0xffffffffu;
             const int bin = act ? (int)((key >> 24) * N + ((key >> 16) & 255u)) * qc + (int)((key >> 8) & qm) : -1;
-            const unsigned peers = __match_any_sync(0xffffffffu, bin);
-            const int leader = __ffs(peers) - 1;
-            const EntrySlot at = entry_slot(cnt, bin, peers, ka > 0, tid);
+            const EntrySlot at = entry_slot<decltype(pairs)::value>(cnt, bin, tid);
+            const int leader = __ffs(at.peers) - 1;
             __syncwarp();
             if (act) ent[at.tx] = key;
             // transposed copy for the tensor pencil stage,
@@ -305,7 +310,7 @@ __global__ void __launch_bounds__(256) ligand_prep_kernel(
             if (act && ent_t) {
                 const size_t row = (size_t)(at.bin + __ldg(tpad + (key >> 24)));
                 uint32_t xr = min(((key >> 16) - (uint32_t)x0) & 255u, (uint32_t)W);
-                if (ka) xr = 2 * xr + (xr < (uint32_t)W ? (key >> 8) & 1u : 0u);
+                if (decltype(pairs)::value) xr = 2 * xr + (xr < (uint32_t)W ? (key >> 8) & 1u : 0u);
                 ent_t[(((size_t)(q >> 7) * (n_pad >> 2) + (row >> 2)) * 128 + (q & 127)) * 4 + (row & 3)] =
                     (xr << 24) | (((key >> 8) & 255u) << 16) | (key & 255u);
             }
@@ -318,9 +323,13 @@ __global__ void __launch_bounds__(256) ligand_prep_kernel(
                         make_uint4(key, __float_as_uint(w_in[i]), __float_as_uint(w_in[i + half]), 0u);
                 idx_out[(size_t)q * n_ent + at.bin] = i;
             }
-            if (act && tid == leader) cnt[bin] += __popc(peers);
+            if (act && tid == leader) cnt[bin] += __popc(at.peers);
             __syncwarp();
         }
+    };
+    if (tid < 32) {
+        if (ka) scatter(std::true_type{});
+        else scatter(std::false_type{});
     }
     if (tid == 0) status[q] = bad;
 }
